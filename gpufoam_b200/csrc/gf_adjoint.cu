@@ -202,13 +202,12 @@ __device__ __forceinline__ void stream_gather2(const Grp<G>& g, const Stream& st
 template <int G, class W>
 __device__ void adj_mixture(const Grp<G>& g, const DevMech& M, const W& w, const WsC& wa, const WsLayout& L, const AdjLayout& A,
                             int y_off, double p) {
-    double rhoM, CpM, dCpMdT, alphav;
-    mixture(g, M, w, L, y_off, p, true, &rhoM, &CpM, &dCpMdT, &alphav);
+    const Mix x = mixture<true, true>(g, M, w, L, y_off, p);
     if (g.lane == 0) {
-        wa[A.ms + MS_RHO] = rhoM;
-        wa[A.ms + MS_CPM] = CpM;
-        wa[A.ms + MS_DCPM] = dCpMdT;
-        wa[A.ms + MS_AV] = alphav;
+        wa[A.ms + MS_RHO] = x.rhoM;
+        wa[A.ms + MS_CPM] = x.CpM;
+        wa[A.ms + MS_DCPM] = x.dCpMdT;
+        wa[A.ms + MS_AV] = x.alphav;
     }
     g.sync();
 }
@@ -613,13 +612,11 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
                          const RosCoeffs& C, const OdeParams& o, double p, double h, double* theta_bar) {
     const int m = M.m, ld = L.ld;
     // recompute the attempt (stages kept: k_i, y2, y3; LU factors in L.J)
-    if (g.lane == 0) w[L.scal + S_KCACHE_T] = -1.0;
-    g.sync();
     {
         GF_PH_BEGIN(g)
         // f(y0) keeps its rate constants for the Jacobian at the same state
         derivatives(g, M, w, L, L.y0, p, L.dydx0, true);
-        jacobian(g, M, w, L, L.y0, p, true);
+        jacobian<true>(g, M, w, L, L.y0, p);
         // kept for the Jacobian term: the raw entries (from the Jacobian terms
         // in the staging slots), the converted Jacobian and dfdx
         stream_gather2(g, M.jst[stream_index(G)], w, L.stage, wa, A.raw);
@@ -627,7 +624,7 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
         for (int i = g.lane; i < m; i += G) wa[A.dfc + i] = w[L.dfdx + i];
         g.sync();
         shift_and_factor(g, M, w, L, C, h);
-        ros_attempt<G, W, true>(g, M, w, L, C, o, L.y0, L.yt, p, h, A.y2, A.y3, false, A.f2, A.f3);
+        ros_attempt<G, W, true>(g, M, w, L, C, o, L.y0, L.yt, p, h, A.y2, A.y3, A.f2, A.f3);
         GF_PH_END(g, PH_ADJ_RECOMPUTE)
     }
     // kbar_i = b_i ybar; the ybar of y1 = y0 + sum b_i k_i flows to y0 unchanged

@@ -75,9 +75,14 @@ enum { PH_MIX = 0, PH_NMPOW, PH_OMEGA, PH_GATHER_RHS, PH_JPARAMS, PH_JROWS, PH_T
 
 // ---------------------------------------------------------------- groups
 
-// Cross-warp reduction buffer of a multi-warp group (one group per CTA).
+// Cross-warp reduction buffers of a multi-warp group (one group per CTA): two,
+// used in turn, so that a reduction needs one barrier (a warp writes a buffer
+// again only after the barrier of the reduction in between, which every warp
+// reaches after reading it).
+constexpr int kRedMax = 4;  // values reduced together
+template <int NW>
 __device__ __forceinline__ double* grp_red_buf() {
-    __shared__ double buf[8];
+    __shared__ double buf[2 * NW * kRedMax];
     return buf;
 }
 
@@ -90,6 +95,7 @@ struct Grp {
     static constexpr int W = G > 32 ? G / 32 : 1;  // warps in the group
     int lane;
     unsigned mask;
+    mutable int ph = 0;  // which reduction buffer is next (the same in every thread)
     __device__ __forceinline__ int warp() const { return G > 32 ? lane >> 5 : 0; }  // warp in the group
     __device__ __forceinline__ Grp() {
         const int wl = threadIdx.x & 31;
@@ -109,47 +115,62 @@ struct Grp {
     }
     __device__ __forceinline__ long long bcast_ll(long long v, int src) const {
         if (G == 1) return v;
-        if (G > 32) {
-            long long* b = reinterpret_cast<long long*>(grp_red_buf());
-            __syncthreads();
+        if constexpr (G > 32) {
+            long long* b = reinterpret_cast<long long*>(grp_red_buf<W>()) + (ph ? W * kRedMax : 0);
+            ph ^= 1;
             if (lane == src) b[0] = v;
             __syncthreads();
-            v = b[0];
-            __syncthreads();
-            return v;
+            return b[0];
         }
         return __shfl_sync(mask, v, src, G);
     }
-    __device__ __forceinline__ double sum(double v) const {
+    // N sums (or maxima) over the group at once, the same in every thread:
+    // a shuffle tree inside a warp, then the warps in order (deterministic)
+    template <int N, bool MAX>
+    __device__ __forceinline__ void reduce(double (&v)[N]) const {
+        static_assert(N <= kRedMax, "reduction buffer");
         constexpr int L = G > 32 ? 32 : G;
 #pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o, L);
-        if (G > 32) {
-            double* b = grp_red_buf();
-            if ((threadIdx.x & 31) == 0) b[lane >> 5] = v;
-            __syncthreads();
-            v = b[0];
+        for (int o = L / 2; o > 0; o >>= 1) {
 #pragma unroll
-            for (int k = 1; k < W; ++k) v += b[k];
-            __syncthreads();
+            for (int n = 0; n < N; ++n) {
+                const double x = __shfl_xor_sync(mask, v[n], o, L);
+                v[n] = MAX ? fmax(v[n], x) : v[n] + x;
+            }
         }
-        return v;
+        if constexpr (G > 32) {
+            double* b = grp_red_buf<W>() + (ph ? W * kRedMax : 0);
+            ph ^= 1;
+            if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+                for (int n = 0; n < N; ++n) b[(lane >> 5) * kRedMax + n] = v[n];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                v[n] = b[n];
+#pragma unroll
+                for (int k = 1; k < W; ++k) {
+                    const double x = b[k * kRedMax + n];
+                    v[n] = MAX ? fmax(v[n], x) : v[n] + x;
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ double sum(double v) const {
+        double x[1] = {v};
+        reduce<1, false>(x);
+        return x[0];
+    }
+    template <int N>
+    __device__ __forceinline__ void sums(double (&v)[N]) const {
+        reduce<N, false>(v);
     }
     // max with fmax semantics: a NaN operand is ignored (normaliseError.H:22)
     __device__ __forceinline__ double fmax_(double v) const {
-        constexpr int L = G > 32 ? 32 : G;
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(mask, v, o, L));
-        if (G > 32) {
-            double* b = grp_red_buf();
-            if ((threadIdx.x & 31) == 0) b[lane >> 5] = v;
-            __syncthreads();
-            v = b[0];
-#pragma unroll
-            for (int k = 1; k < W; ++k) v = fmax(v, b[k]);
-            __syncthreads();
-        }
-        return v;
+        double x[1] = {v};
+        reduce<1, true>(x);
+        return x[0];
     }
     __device__ __forceinline__ int any(int p) const {
         if (G == 1) return p;
@@ -260,27 +281,9 @@ __device__ __forceinline__ Poly7 reaction_coeffs_at(const DevMech& M, int r, dou
     return a;
 }
 
-__device__ __forceinline__ Poly7 reaction_coeffs(const DevMech& M, int r, double T) {
-    const int b = coef_branch(T, ldg(M.rTcommon + r));
-    const double* c = M.rcoef + (size_t)b * 7 * M.nR + r;
-    Poly7 a;
-    a.a0 = ldg(c);
-    a.a1 = ldg(c + M.nR);
-    a.a2 = ldg(c + 2 * M.nR);
-    a.a3 = ldg(c + 3 * M.nR);
-    a.a4 = ldg(c + 4 * M.nR);
-    a.a5 = ldg(c + 5 * M.nR);
-    a.a6 = ldg(c + 6 * M.nR);
-    return a;
-}
-
 // gpuThermo.H:177-184 (the perfect-gas Cp term is 0)
 __device__ __forceinline__ double th_Cp(const Poly7& a, double T) {
     return ((((a.a4 * T + a.a3) * T + a.a2) * T + a.a1) * T + a.a0);
-}
-// gpuThermo.H:210-221
-__device__ __forceinline__ double th_Ha(const Poly7& a, double T) {
-    return (((((a.a4 / 5.0 * T + a.a3 / 4.0) * T + a.a2 / 3.0) * T + a.a1 / 2.0) * T + a.a0) * T + a.a5);
 }
 // gpuThermo.H:333-338
 __device__ __forceinline__ double th_dCpdT(const Poly7& a, double T) {
@@ -322,27 +325,6 @@ __device__ __forceinline__ TCache make_tcache(double T) {
     return t;
 }
 
-// ln of the K part of Kc, capped as K() caps it (gpuThermo.H:84-85)
-__device__ __forceinline__ double reaction_lnKc(const DevMech& M, int q, const Rxn& R, const TCache& tc,
-                                                double* Gstd_out, Poly7* a_out) {
-    const Poly7 a = reaction_coeffs_at(M, q, tc.T, R.Tcommon);
-    const double Gstd = th_Gstd(a, tc.T, tc.logT);
-    const double arg = -R.Y * Gstd * tc.invT * (1.0 / kRR);
-    double lnK = arg < 600 ? arg : 0.5 * log(kVGreat);
-    if (!R.nm_small) lnK += R.nm * tc.lx;
-    if (Gstd_out) *Gstd_out = Gstd;
-    if (a_out) *a_out = a;
-    return lnK;
-}
-
-// dKc/dT / Kc (gpuThermo.H:160-166)
-__device__ __forceinline__ double reaction_dKcdTbyKc(const Rxn& R, const TCache& tc, double Gstd, const Poly7& a) {
-    const double S = th_S_pstd(a, tc.T, tc.logT);
-    double ret = (S + Gstd * tc.invT) * R.Y * tc.invT * (1.0 / kRR);
-    if (!R.nm_small) ret = ret - R.nm * tc.invT;
-    return ret;
-}
-
 // gpuSpecieExponent.H:21-36
 __device__ __forceinline__ double integer_pow(double x, int e) {
     if (e == 0) return 1;
@@ -369,19 +351,91 @@ __device__ __forceinline__ double specie_pow_m1(double x, int iexp, double sexp)
     return iexp != kNoIntExp ? integer_pow(x, iexp - 1) : real_pow(x, sexp + (-1.0));
 }
 
-// ln|k| of an Arrhenius factor: k (or the fall-off k0) from the reaction's
-// head, kInf from the fall-off tables; and dln(k)/dT = (beta + Ta/T)/T
-__device__ __forceinline__ double arr_ln0(const Rxn& R, const TCache& tc) {
-    return fma(R.beta0, tc.logT, R.lnA0) - R.Ta0 * tc.invT;
-}
+// ln|kInf| of a fall-off rate and dln(kInf)/dT = (beta + Ta/T)/T
 __device__ __forceinline__ double arr_ln1(const DevMech& M, int q, const TCache& tc) {
     return fma(ldg(M.beta1 + q), tc.logT, ldg(M.lnA1 + q)) - ldg(M.Ta1 + q) * tc.invT;
 }
-__device__ __forceinline__ double arr_dlnkdT0(const Rxn& R, const TCache& tc) {
-    return (R.beta0 + R.Ta0 * tc.invT) * tc.invT;
-}
 __device__ __forceinline__ double arr_dlnkdT1(const DevMech& M, int q, const TCache& tc) {
     return (ldg(M.beta1 + q) + ldg(M.Ta1 + q) * tc.invT) * tc.invT;
+}
+
+// The solve's view of a reaction: its compact record (RxnFast).
+struct RxnF {
+    int meta, slot;
+    unsigned lhs, rhs;
+    double lnA0, beta0, Ta0, nm;
+    __device__ __forceinline__ int type() const { return meta & kRxnType; }
+    __device__ __forceinline__ bool irr() const { return meta & kRxnIrr; }
+    __device__ __forceinline__ int nl() const { return (meta >> kRxnNlShift) & 15; }
+    __device__ __forceinline__ int nr() const { return (meta >> kRxnNrShift) & 15; }
+    __device__ __forceinline__ unsigned side(int sd) const { return sd ? rhs : lhs; }
+    __device__ __forceinline__ bool sq(int sd, int e) const {
+        return (meta >> (kRxnSqShift + kFastSide * sd + e)) & 1;
+    }
+    // sign(A): A = 0 gives k = 0 exactly
+    __device__ __forceinline__ double sign() const {
+        const int b = (meta >> kRxnSignShift) & 3;
+        return b == 0 ? 1.0 : (b == 1 ? -1.0 : 0.0);
+    }
+};
+
+__device__ __forceinline__ RxnF load_fast(const DevMech& M, int q) {
+    const int4* h = reinterpret_cast<const int4*>(M.rxf + q);
+    const int4 h0 = __ldg(h);
+    const double2* hd = reinterpret_cast<const double2*>(h) + 1;
+    const double2 d0 = __ldg(hd), d1 = __ldg(hd + 1);
+    return RxnF{h0.x, h0.y, (unsigned)h0.z, (unsigned)h0.w, d0.x, d0.y, d1.x, d1.y};
+}
+
+// The reaction's third-body concentration (third_body_all), 0 for plain Arrhenius rates.
+template <class W>
+__device__ __forceinline__ double fast_M(const DevMech& M, const W& w, int m_off, const RxnF& R, int q) {
+    int t = (int)((unsigned)R.meta >> kRxnTbShift);
+    if (t == 0) return 0.0;
+    if (t == kRxnTbFar) t = ldg(M.tb_row + q) + 1;
+    return w[m_off + t - 1];
+}
+
+// The seven coefficients of ln K at this temperature's branch (DevMech::lnk).
+struct LnK {
+    double b0, b1, b2, b3, b4, b5, b6;
+};
+__device__ __forceinline__ LnK load_lnK(const DevMech& M, int q, double T) {
+    // one Tcommon for every reaction (the usual case): no load to wait for
+    const double Tc = M.Tc_all == M.Tc_all ? M.Tc_all : ldg(M.rTcommon + q);
+    const double* c = M.lnk + (size_t)coef_branch(T, Tc) * 7 * M.nR + q;
+    LnK a;
+    a.b0 = ldg(c);
+    a.b1 = ldg(c + M.nR);
+    a.b2 = ldg(c + 2 * M.nR);
+    a.b3 = ldg(c + 3 * M.nR);
+    a.b4 = ldg(c + 4 * M.nR);
+    a.b5 = ldg(c + 5 * M.nR);
+    a.b6 = ldg(c + 6 * M.nR);
+    return a;
+}
+// ln Kc with K capped as K() caps it (gpuThermo.H:80-113, 139-169): -Y G / (R T)
+// with Y, R and the polynomial's divisors folded into the coefficients
+__device__ __forceinline__ double fast_lnKc(const RxnF& R, const LnK& a, const TCache& tc) {
+    const double T = tc.T;
+    const double poly = fma(fma(fma(a.b4, T, a.b3), T, a.b2), T, a.b1);
+    double lnK = fma(a.b0, 1.0 - tc.logT, -a.b6);
+    lnK = fma(-poly, T, lnK);
+    lnK = fma(a.b5, tc.invT, lnK);
+    lnK = lnK < 600 ? lnK : 0.5 * log(kVGreat);
+    return fma(R.nm, tc.lx, lnK);
+}
+// d ln Kc / dT (gpuThermo.H:160-166: (S + G/T) Y / (R T) - nm/T). S + G/T is H/T,
+// whose polynomial has no logarithm and no cancellation between the two:
+// -(b0 + 2 b1/2 T + ...) with G's divisors 2, 6, 12, 20 turned into H's 2, 3, 4, 5
+__device__ __forceinline__ double fast_dlnKcdT(const RxnF& R, const LnK& a, const TCache& tc) {
+    const double T = tc.T;
+    double h = fma(4.0 * a.b4, T, 3.0 * a.b3);
+    h = fma(h, T, 2.0 * a.b2);
+    h = fma(h, T, a.b1);
+    h = fma(h, T, a.b0);
+    h = fma(a.b5, tc.invT, h);
+    return -(h + R.nm) * tc.invT;
 }
 
 // Third-body concentrations M_t = sum_i eff_ti c_i of every third-body and
@@ -460,35 +514,100 @@ __device__ __forceinline__ double troe_F(const DevMech& M, int q, const TCache& 
     return exp(x4 * kLn10);
 }
 
-// Forward rate constant kf (operator(), gpuReactionRate.H:164-173); with
-// want_dT also dkf/dT and, for third-body rates, the pure Arrhenius part Ak
-// ("everything", gpuArrheniusReactionRate.H:97-107,
-// gpuThirdBodyArrheniusReactionRate.H:105-121, gpuFallOffReactionRate.H:127-158).
-// Mc: the reaction's third-body concentration (third_body_all), unused for
-// plain Arrhenius rates.
-__device__ __forceinline__ double rate_k(const DevMech& M, int q, const Rxn& R, const TCache& tc, double Mc,
-                                         bool want_dT, double* dT_out, double* Ak_out) {
-    const int type = R.type;
-    if (type == GF_RATE_ARRHENIUS) {
-        const double Ak = R.sA0 * exp(arr_ln0(R, tc));
-        if (want_dT) *dT_out = Ak * arr_dlnkdT0(R, tc);
-        return Ak;
+// Forward rate constant kf (operator(), gpuReactionRate.H:164-173) and, for
+// third-body rates, its pure Arrhenius part Ak: plain and third-body Arrhenius
+// (gpuArrheniusReactionRate.H, gpuThirdBodyArrheniusReactionRate.H), Lindemann
+// and Troe fall-off (gpuFallOffReactionRate.H); the first exponential is one
+// code site for all of them. Mc: the reaction's third-body concentration.
+__device__ __forceinline__ double fast_kf(const DevMech& M, int q, const RxnF& R, const TCache& tc, double Mc,
+                                          double* Ak_out) {
+    const int type = R.type();
+    const double l0 = fma(R.beta0, tc.logT, R.lnA0) - R.Ta0 * tc.invT;
+    const bool falloff = type >= GF_RATE_LINDEMANN_FALLOFF;
+    double l = l0, s = R.sign();
+    if (falloff) {
+        l = arr_ln1(M, q, tc);
+        s = ldg(M.sA1 + q);
     }
-    if (type == GF_RATE_THIRD_BODY_ARRHENIUS) {
-        const double Ak = R.sA0 * exp(arr_ln0(R, tc));
-        if (want_dT) *dT_out = Mc * (Ak * arr_dlnkdT0(R, tc));
-        *Ak_out = Ak;
-        return Mc * Ak;
+    double k = s * exp(l);  // k, or the fall-off kInf
+    *Ak_out = k;
+    if (type == GF_RATE_THIRD_BODY_ARRHENIUS) k *= Mc;
+    if (falloff) {
+        // Pr = k0 / kInf * M, k = kInf Pr / (1 + Pr) F
+        const double Pr = (R.sign() * s) * exp(l0 - l) * Mc;
+        const double F = type == GF_RATE_TROE_FALLOFF ? troe_F(M, q, tc, Pr) : 1.0;
+        k *= (Pr / (1.0 + Pr)) * F;
     }
-    // fall-off: Pr = k0 / kInf * M, k = kInf Pr / (1 + Pr) F
-    const double l0 = arr_ln0(R, tc), l1 = arr_ln1(M, q, tc);
-    const double s0 = R.sA0, s1 = ldg(M.sA1 + q);
-    const double kInf = s1 * exp(l1);
-    const double Pr = (s0 * s1) * exp(l0 - l1) * Mc;
-    const double F = type == GF_RATE_TROE_FALLOFF ? troe_F(M, q, tc, Pr) : 1.0;
-    const double temp = (Pr / (1.0 + Pr)) * F;
-    if (want_dT) *dT_out = (kInf * arr_dlnkdT1(M, q, tc)) * temp;
-    return kInf * temp;
+    return k;
+}
+
+// Concentration products of reactions outside the compact record's terms (a
+// side of more than kFastSide species, an exponent other than 1 and 2), out of
+// line: rare, and their code would sit in the middle of every reaction loop.
+// C = prod c^e in the reference's order (calcCf / calcCr, gpuReaction.H:372-386).
+template <class W>
+__device__ __noinline__ double general_C(const int* idx, const int* iexp, const double* sexp, int n, W w, int c_off) {
+    double C = 1.0;
+    for (int e = 0; e < n; ++e) C *= specie_pow(w[c_off + ldg(idx + e)], ldg(iexp + e), ldg(sexp + e));
+    return C;
+}
+// C, and kmul dC/dc_j to out + j (calcdCfdcj / calcdCrdcj, gpuReaction.H:388-470).
+template <class W>
+__device__ __noinline__ double general_products(const int* idx, const int* iexp, const double* sexp, int n, W w,
+                                                int c_off, double kmul, int out) {
+    double C = 1.0;
+    for (int e = 0; e < n; ++e) C *= specie_pow(w[c_off + ldg(idx + e)], ldg(iexp + e), ldg(sexp + e));
+    for (int j = 0; j < n; ++j) {
+        double d = 1;
+        for (int i = 0; i < n; ++i) {
+            const double x = w[c_off + ldg(idx + i)];
+            const int ie = ldg(iexp + i);
+            const double se = ldg(sexp + i);
+            d *= (i == j) ? se * specie_pow_m1(x, ie, se) : specie_pow(x, ie, se);
+        }
+        w[out + j] = d * kmul;
+    }
+    return C;
+}
+
+// C = prod c^e of one side (0: lhs, 1: rhs): without a branch for the usual
+// reaction (absent species read the 1 kept behind the concentrations).
+template <class W>
+__device__ __forceinline__ double fast_C(const DevMech& M, const W& w, int c_off, const RxnF& R, int q, int sd) {
+    if (R.meta & kRxnGeneral) {
+        const int b = ldg(M.sp_off + q) + (sd ? R.nl() : 0);
+        return general_C(M.sidx + b, M.siexp + b, M.sexp + b, sd ? R.nr() : R.nl(), w, c_off);
+    }
+    double C = 1.0;
+#pragma unroll
+    for (int e = 0; e < kFastSide; ++e) {
+        const double x = w[c_off + ((R.side(sd) >> (10 * e)) & 1023)];
+        C *= R.sq(sd, e) ? x * x : x;
+    }
+    return C;
+}
+// C, and kmul dC/dc_j of the side's species to out + j.
+template <class W>
+__device__ __forceinline__ double fast_products(const DevMech& M, const W& w, int c_off, const RxnF& R, int q, int sd,
+                                                double kmul, int out) {
+    const int n = sd ? R.nr() : R.nl();
+    if (R.meta & kRxnGeneral) {
+        const int b = ldg(M.sp_off + q) + (sd ? R.nl() : 0);
+        return general_products(M.sidx + b, M.siexp + b, M.sexp + b, n, w, c_off, kmul, out);
+    }
+    double pw[kFastSide], dm[kFastSide];
+#pragma unroll
+    for (int e = 0; e < kFastSide; ++e) {
+        const double x = w[c_off + ((R.side(sd) >> (10 * e)) & 1023)];
+        const bool sq = R.sq(sd, e);
+        pw[e] = sq ? x * x : x;
+        dm[e] = sq ? 2.0 * x : 1.0;
+    }
+    static_assert(kFastSide == 3, "the products below");
+    w[out] = dm[0] * pw[1] * pw[2] * kmul;
+    if (n > 1) w[out + 1] = pw[0] * dm[1] * pw[2] * kmul;
+    if (n > 2) w[out + 2] = pw[0] * pw[1] * dm[2] * kmul;
+    return pw[0] * pw[1] * pw[2];
 }
 
 // ------------------------------------------------------------- layout
@@ -522,7 +641,7 @@ __host__ __device__ inline WsLayout make_layout(int nS, int nR, int n_slots, int
     } else {
         L.perm = L.piv;
     }
-    L.c = o; o += nS;
+    L.c = o; o += nS + 1;  // and a 1 for the absent species of a reaction side
     L.Ha = o; o += nS;
     if (sweep) {
         L.Cp = o; o += nS;
@@ -540,52 +659,60 @@ __host__ __device__ inline WsLayout make_layout(int nS, int nR, int n_slots, int
     return L;
 }
 
-// per-call scalars kept in the workspace scal[] block
-enum { S_KCACHE_T = 0 };
-
 // ------------------------------------------------------------ ODE system
+
+// The mixture's scalars: density and its inverse, Cp, dCp/dT, the thermal
+// expansion.
+struct Mix {
+    double rhoM, irho, CpM, dCpMdT, alphav;
+};
 
 // Mixture properties + concentrations (gpuMixture.H:33-121). The sums over
 // species run lane-strided and are combined by a fixed shuffle tree
-// (deterministic; the reference sums sequentially).
-template <int G, class W>
-__device__ __forceinline__ void mixture(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L, int y_off,
-                                        double p, bool jac, double* rhoM_o, double* CpM_o, double* dCpMdT_o,
-                                        double* alphav_o) {
+// (deterministic; the reference sums sequentially), all of them in one
+// reduction. No division per species: 1/rho_i = (R/W_i) T/p, the polynomials'
+// divisors and 1/W_i are in the tables, and the expansion coefficient
+// sum(Y_i / (rho_i T)) rhoM of a perfect gas is 1/T. JAC: also Cp; STORE: also
+// the per-species v and rhoM/W that the adjoint reads.
+template <bool JAC, bool STORE = false, int G, class W>
+__device__ __forceinline__ Mix mixture(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L, int y_off,
+                                       double p) {
     const int nS = M.nS;
     const double T = w[y_off + nS];
-    const double invT = 1.0 / T;
-    double s_rho = 0, s_cp = 0, s_dcp = 0, s_av = 0;
+    const double ToP = T / p;
+    double sm[JAC ? 3 : 2] = {};
     for (int i = g.lane; i < nS; i += G) {
         const double yi = fmax(w[y_off + i], 0.0);
-        const double rhoi = p / (ldg(M.Rsp + i) * T);
-        const Poly7 a = species_coeffs(M, i, T);
-        const double Cpi = th_Cp(a, T);
-        const double Hai = th_Ha(a, T);
-        s_rho += yi / rhoi;
-        s_cp += yi * Cpi;
-        w[L.Ha + i] = Hai;
-        w[L.c + i] = yi / ldg(M.W + i);
-        if (jac) {
-            const double vi = 1.0 / rhoi;
-            s_dcp += yi * th_dCpdT(a, T);
-            s_av += yi * vi * invT;
+        const double vi = ldg(M.Rsp + i) * ToP;
+        const double* a = M.spc + (size_t)coef_branch(T, ldg(M.Tcommon + i)) * 10 * nS + i;
+        const double a0 = ldg(a), a1 = ldg(a + nS), a2 = ldg(a + 2 * nS), a3 = ldg(a + 3 * nS), a4 = ldg(a + 4 * nS);
+        const double h1 = ldg(a + 5 * nS), h2 = ldg(a + 6 * nS), h3 = ldg(a + 7 * nS), h4 = ldg(a + 8 * nS),
+                     a5 = ldg(a + 9 * nS);
+        const double Cpi = (((a4 * T + a3) * T + a2) * T + a1) * T + a0;
+        sm[0] += yi * vi;
+        sm[1] += yi * Cpi;
+        w[L.Ha + i] = ((((h4 * T + h3) * T + h2) * T + h1) * T + a0) * T + a5;
+        w[L.c + i] = yi * ldg(M.invW + i);
+        if (JAC) {
+            sm[JAC ? 2 : 0] += yi * (((4.0 * a4 * T + 3.0 * a3) * T + 2.0 * a2) * T + a1);
             w[L.Cp + i] = Cpi;
-            w[L.vj + i] = vi;
         }
+        if (STORE) w[L.vj + i] = vi;
     }
-    const double rhoM = 1.0 / g.sum(s_rho);
-    *rhoM_o = rhoM;
-    *CpM_o = g.sum(s_cp);
-    if (jac) {
-        *dCpMdT_o = g.sum(s_dcp);
-        *alphav_o = g.sum(s_av) * rhoM;
-    }
+    g.sums(sm);
+    Mix x;
+    x.irho = sm[0];
+    x.rhoM = 1.0 / sm[0];
+    x.CpM = sm[1];
+    x.dCpMdT = JAC ? sm[JAC ? 2 : 0] : 0.0;
+    x.alphav = JAC ? 1.0 / T : 0.0;
     for (int i = g.lane; i < nS; i += G) {
-        w[L.c + i] *= rhoM;
-        if (jac) w[L.rhoMbyW + i] = rhoM / ldg(M.W + i);
+        w[L.c + i] *= x.rhoM;
+        if (STORE) w[L.rhoMbyW + i] = x.rhoM * ldg(M.invW + i);
     }
+    if (g.lane == 0) w[L.c + nS] = 1.0;
     g.sync();
+    return x;
 }
 
 // Net rate omega of every reaction at the clipped temperature (gpuReaction.H:472-488)
@@ -598,25 +725,20 @@ template <int G, class W>
 __device__ __forceinline__ void stage_omega(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
                                             const TCache& tc, bool write_cache) {
     for (int q = g.lane; q < M.nR; q += G) {
-        Rxn R;
-        load_rxn(M, q, R);
-        const int so = R.slot;
-        const double Mc = R.tb_row >= 0 ? w[L.Mtb + R.tb_row] : 0.0;
-        double dummy, Ak = 0.0;
-        const double kf = rate_k(M, q, R, tc, Mc, false, &dummy, &Ak);
-        double kr = 0.0, invKc = 1.0;
-        if (!R.irr) {
-            invKc = exp(-reaction_lnKc(M, q, R, tc, nullptr, nullptr));
-            kr = kf * invKc;
-        }
+        const RxnF R = load_fast(M, q);
+        const LnK a = load_lnK(M, q, tc.T);
+        double Ak;
+        const double kf = fast_kf(M, q, R, tc, fast_M(M, w, L.Mtb, R, q), &Ak);
+        const double invKc = R.irr() ? 1.0 : exp(-fast_lnKc(R, a, tc));
+        const double Cf = fast_C(M, w, L.c, R, q, 0);
+        const double Cr = fast_C(M, w, L.c, R, q, 1);
+        const int so = L.stage + R.slot;
+        w[so] = kf * Cf - (R.irr() ? 0.0 : kf * invKc * Cr);
         if (write_cache) {
-            w[L.stage + so + 1] = kf;
-            w[L.stage + so + 2] = invKc;
-            w[L.stage + so + 3] = Ak;
+            w[so + 1] = kf;
+            w[so + 2] = invKc;
+            w[so + 3] = Ak;
         }
-        const double Cf = side_C(M, w, L.c, R, 0);
-        const double Cr = side_C(M, w, L.c, R, 1);
-        w[L.stage + so] = kf * Cf - kr * Cr;
     }
     g.sync();
 }
@@ -659,18 +781,18 @@ __device__ __forceinline__ void stream_gather(const Grp<G>& g, const Stream& st,
 // 184-189), then dT/dt (:53-63). Writes out[0..m).
 template <int G, class W>
 __device__ __forceinline__ void gather_rhs(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
-                                           int out_off, double rhoM, double CpM) {
+                                           int out_off, const Mix& x) {
     const int nS = M.nS;
     stream_gather(g, M.dst[stream_index(G)], w, L.stage, out_off);
     g.sync();
     double s_h = 0;
     for (int s = g.lane; s < nS; s += G) {
-        const double acc = w[out_off + s] * (ldg(M.W + s) / rhoM);
+        const double acc = w[out_off + s] * (ldg(M.W + s) * x.irho);
         w[out_off + s] = acc;
         s_h += acc * w[L.Ha + s];
     }
     const double sh = g.sum(s_h);
-    if (g.lane == 0) w[out_off + nS] = (-sh) / CpM;
+    if (g.lane == 0) w[out_off + nS] = (-sh) / x.CpM;
     g.sync();
 }
 
@@ -678,156 +800,63 @@ __device__ __forceinline__ void gather_rhs(const Grp<G>& g, const DevMech& M, co
 template <int G, class W>
 __device__ __forceinline__ void derivatives(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
                                             int y_off, double p, int out_off, bool write_cache = false) {
-    double rhoM, CpM, d0, d1;
+    Mix x;
     g.sync();
     {
         GF_PH_BEGIN(g)
-        mixture(g, M, w, L, y_off, p, false, &rhoM, &CpM, &d0, &d1);
+        x = mixture<false>(g, M, w, L, y_off, p);
         GF_PH_END(g, PH_MIX)
     }
     const double T = w[y_off + M.nS];
     const double Tc = fmin(fmax(T, M.Tlow), M.Thigh);
-    const TCache tc = make_tcache(Tc);
-    // the Jacobian evaluates at the unclipped T: the cache serves it only when
-    // the clip left T unchanged
-    const bool cache_requested = write_cache;
-    write_cache = write_cache && (Tc == T);
     {
         GF_PH_BEGIN(g)
         if (M.n_tb > 0) {
             third_body_all(g, M, w, L.c, L.Mtb);
             g.sync();
         }
-        stage_omega(g, M, w, L, tc, write_cache);
+        // The Jacobian takes its rate constants at the unclipped T: where the
+        // clip changes T, a first pass leaves them in the cache.
+        const bool two = write_cache && Tc != T;
+#pragma unroll 1
+        for (int pass = two ? 0 : 1; pass < 2; ++pass)
+            stage_omega(g, M, w, L, make_tcache(pass == 0 ? T : Tc), write_cache && !(two && pass == 1));
         GF_PH_END(g, PH_OMEGA)
     }
-    if (cache_requested && g.lane == 0) w[L.scal + S_KCACHE_T] = write_cache ? T : -1.0;
     {
         GF_PH_BEGIN(g)
-        gather_rhs(g, M, w, L, out_off, rhoM, CpM);
+        gather_rhs(g, M, w, L, out_off, x);
         GF_PH_END(g, PH_GATHER_RHS)
     }
 }
 
-// Product C = prod c^e of one side of a reaction (side 0: lhs, 1: rhs), in
-// the reference's order (calcCf / calcCr, gpuReaction.H:372-386).
-template <class W>
-__device__ __forceinline__ double side_C(const DevMech& M, const W& w, int c_off, const Rxn& R, int side) {
-    const int n = side ? R.nr : R.nl;
-    double C = 1.0;
-    if (n <= kSideInline) {
-#pragma unroll
-        for (int e = 0; e < kSideInline; ++e)
-            if (e < n) C *= specie_pow(w[c_off + R.idx[side][e]], R.iexp[side][e], R.sexp[side][e]);
-        return C;
-    }
-    const int b = R.sp_off + (side ? R.nl : 0);
-    for (int e = 0; e < n; ++e)
-        C *= specie_pow(w[c_off + ldg(M.sidx + b + e)], ldg(M.siexp + b + e), ldg(M.sexp + b + e));
-    return C;
-}
-
-// One side of a reaction: returns C = prod c^e and writes kmul * dC/dc_j to
-// out + j, each the product over i of e_i c_i^(e_i - 1) (i == j) or c_i^e_i
-// (i != j) in the reference's order (calcdCfdcj / calcdCrdcj, :388-470). Up to
-// kSideInline species the powers stay in registers; wider sides recompute
-// them (the same values).
-template <class W>
-__device__ __forceinline__ double side_products(const DevMech& M, const W& w, int c_off, const Rxn& R, int side,
-                                                double kmul, int out) {
-    const int n = side ? R.nr : R.nl;
-    if (n <= kSideInline) {
-        double pw[kSideInline], dm[kSideInline];
-#pragma unroll
-        for (int e = 0; e < kSideInline; ++e) {
-            pw[e] = 1.0;
-            dm[e] = 1.0;
-            if (e < n) {
-                const double x = w[c_off + R.idx[side][e]];
-                pw[e] = specie_pow(x, R.iexp[side][e], R.sexp[side][e]);
-                dm[e] = R.sexp[side][e] * specie_pow_m1(x, R.iexp[side][e], R.sexp[side][e]);
-            }
-        }
-        double C = 1.0;
-#pragma unroll
-        for (int e = 0; e < kSideInline; ++e)
-            if (e < n) C *= pw[e];
-#pragma unroll
-        for (int j = 0; j < kSideInline; ++j) {
-            if (j < n) {
-                double d = 1;
-#pragma unroll
-                for (int i = 0; i < kSideInline; ++i)
-                    if (i < n) d *= (i == j) ? dm[i] : pw[i];
-                w[out + j] = d * kmul;
-            }
-        }
-        return C;
-    }
-    const int b = R.sp_off + (side ? R.nl : 0);
-    double C = 1.0;
-    for (int e = 0; e < n; ++e)
-        C *= specie_pow(w[c_off + ldg(M.sidx + b + e)], ldg(M.siexp + b + e), ldg(M.sexp + b + e));
-    for (int j = 0; j < n; ++j) {
-        double d = 1;
-        for (int i = 0; i < n; ++i) {
-            const double x = w[c_off + ldg(M.sidx + b + i)];
-            const int ie = ldg(M.siexp + b + i);
-            const double se = ldg(M.sexp + b + i);
-            d *= (i == j) ? se * specie_pow_m1(x, ie, se) : specie_pow(x, ie, se);
-        }
-        w[out + j] = d * kmul;
-    }
-    return C;
-}
-
 // Per-reaction Jacobian parameters (computeReactionParameters, gpuReaction.H:650-702)
+// from the rate constants kept by stage_omega.
 template <int G, class W>
 __device__ __forceinline__ void stage_jacobian_params(const Grp<G>& g, const DevMech& M, const W& w,
-                                                      const WsLayout& L, const TCache& tc, bool use_cache) {
+                                                      const WsLayout& L, const TCache& tc) {
     for (int q = g.lane; q < M.nR; q += G) {
-        Rxn R;
-        load_rxn(M, q, R);
-        const int type = R.type;
-        const int nl = R.nl;
-        const int so = R.slot;
-        double ddT = 0.0, Ak = 0.0, kf;
-        double cachedInvKc = 0.0;
-        if (use_cache) {
-            // dk/dT = k dln(k)/dT with the kInf factor for fall-off rates
-            // (gpuFallOffReactionRate.H:140-141)
-            kf = w[L.stage + so + 1];
-            cachedInvKc = w[L.stage + so + 2];
-            Ak = w[L.stage + so + 3];
-            const bool falloff = type == GF_RATE_LINDEMANN_FALLOFF || type == GF_RATE_TROE_FALLOFF;
-            ddT = kf * (falloff ? arr_dlnkdT1(M, q, tc) : arr_dlnkdT0(R, tc));
-        } else {
-            kf = rate_k(M, q, R, tc, R.tb_row >= 0 ? w[L.Mtb + R.tb_row] : 0.0, true, &ddT, &Ak);
-        }
-        const double Cf = side_products(M, w, L.c, R, 0, kf, L.stage + so + 2);
+        const RxnF R = load_fast(M, q);
+        const LnK a = load_lnK(M, q, tc.T);
+        const int so = L.stage + R.slot;
+        const double kf = w[so + 1], invKc = w[so + 2], Ak = w[so + 3];
+        // dk/dT = k dln(k)/dT with the kInf factor for fall-off rates
+        // (gpuFallOffReactionRate.H:140-141)
+        const double ddT = kf * (R.type() >= GF_RATE_LINDEMANN_FALLOFF ? arr_dlnkdT1(M, q, tc)
+                                                                       : fma(R.Ta0, tc.invT, R.beta0) * tc.invT);
+        const double Cf = fast_products(M, w, L.c, R, q, 0, kf, so + 2);
         double dwdT = Cf * ddT;
         double omega = Cf * kf;
-        double Cr = 0.0, invKc = 1.0;
-        if (!R.irr) {
-            double Gstd;
-            Poly7 a;
-            if (use_cache) {
-                a = reaction_coeffs_at(M, q, tc.T, R.Tcommon);
-                Gstd = th_Gstd(a, tc.T, tc.logT);
-                invKc = cachedInvKc;
-            } else {
-                invKc = exp(-reaction_lnKc(M, q, R, tc, &Gstd, &a));
-            }
-            const double dKcdTbyKc = reaction_dKcdTbyKc(R, tc, Gstd, a);
+        double Cr = 0.0;
+        if (!R.irr()) {
             const double kr = kf * invKc;
-            Cr = side_products(M, w, L.c, R, 1, kr, L.stage + so + 2 + nl);
-            const double dkrdT = ddT * invKc - kr * dKcdTbyKc;
-            dwdT -= Cr * dkrdT;
+            Cr = fast_products(M, w, L.c, R, q, 1, kr, so + 2 + R.nl());
+            dwdT -= Cr * (ddT * invKc - kr * fast_dlnKcdT(R, a, tc));
             omega -= Cr * kr;
         }
-        w[L.stage + so] = omega;
-        w[L.stage + so + 1] = dwdT;
-        if (type == GF_RATE_THIRD_BODY_ARRHENIUS) w[L.stage + so + 2 + nl + R.nr] = Ak * (Cf - Cr * invKc);
+        w[so] = omega;
+        w[so + 1] = dwdT;
+        if (R.type() == GF_RATE_THIRD_BODY_ARRHENIUS) w[so + 2 + R.nl() + R.nr()] = Ak * (Cf - Cr * invKc);
     }
     g.sync();
 }
@@ -838,34 +867,30 @@ __device__ __forceinline__ void stage_jacobian_params(const Grp<G>& g, const Dev
 //     third-body terms in the reference's order per entry;
 //   phase 3 (lanes over rows): ddY_dcdY (gpuODESystem.H:65-103);
 //   then the T row (ddT_dtdY, ddT_dtdT, :108-146).
-template <int G, class W>
+// The rate constants are those that derivatives() with write_cache left in the
+// staging slots at the same state. STORE: the mixture's v and rhoM/W are kept
+// too (the adjoint).
+template <bool STORE = false, int G, class W>
 __device__ __forceinline__ void jacobian(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
-                                         int y_off, double p, bool allow_cache = false) {
+                                         int y_off, double p) {
     const int nS = M.nS;
     const int ld = L.ld;
-    double rhoM, CpM, dCpMdT, alphav;
+    Mix x;
     g.sync();
     {
         GF_PH_BEGIN(g)
-        mixture(g, M, w, L, y_off, p, true, &rhoM, &CpM, &dCpMdT, &alphav);
+        x = mixture<true, STORE>(g, M, w, L, y_off, p);
         GF_PH_END(g, PH_MIX)
     }
-    const TCache tc = make_tcache(w[y_off + nS]);
-    const bool use_cache = allow_cache && w[L.scal + S_KCACHE_T] == tc.T;
+    const double alphav = x.alphav, rToP = x.rhoM * (w[y_off + nS] / p);
     {
         GF_PH_BEGIN(g)
-        if (!use_cache && M.n_tb > 0) {
-            third_body_all(g, M, w, L.c, L.Mtb);
-            g.sync();
-        }
-        stage_jacobian_params(g, M, w, L, tc, use_cache);
+        stage_jacobian_params(g, M, w, L, make_tcache(w[y_off + nS]));
         GF_PH_END(g, PH_JPARAMS)
     }
-    // the staging slots that held the cache now hold the Jacobian terms
-    if (allow_cache && g.lane == 0) w[L.scal + S_KCACHE_T] = -1.0;
     {
         GF_PH_BEGIN(g)
-        gather_rhs(g, M, w, L, L.dfdx, rhoM, CpM);
+        gather_rhs(g, M, w, L, L.dfdx, x);
         GF_PH_END(g, PH_GATHER_RHS)
     }
     {
@@ -876,16 +901,17 @@ __device__ __forceinline__ void jacobian(const Grp<G>& g, const DevMech& M, cons
     g.sync();
     // phase 3
     for (int s = g.lane; s < nS; s += G) {
-        const double WiByrhoM = ldg(M.W + s) / rhoM;
+        const double Ws = ldg(M.W + s);
         const double dfs = w[L.dfdx + s];
         const int row = L.J + s * ld;
         double ddN = w[row + nS];
         for (int c = 0; c < nS; ++c) {
             const double raw = w[row + c];
             ddN -= raw * w[L.c + c] * alphav;
-            w[row + c] = WiByrhoM * raw * w[L.rhoMbyW + c] + rhoM * w[L.vj + c] * dfs;
+            // (W_s / rhoM) raw (rhoM / W_c) + rhoM v_c df_s
+            w[row + c] = Ws * ldg(M.invW + c) * raw + rToP * ldg(M.Rsp + c) * dfs;
         }
-        w[row + nS] = WiByrhoM * ddN + alphav * dfs;
+        w[row + nS] = Ws * x.irho * ddN + alphav * dfs;
     }
     g.sync();
     GF_PH_END(g, PH_JROWS)
@@ -897,13 +923,13 @@ __device__ __forceinline__ void jacobian(const Grp<G>& g, const DevMech& M, cons
         double acc = 0.0;
         for (int j = 0; j < nS; ++j) acc -= w[L.J + j * ld + i] * w[L.Ha + j];
         acc -= w[L.Cp + i] * dTdt;
-        w[L.J + nS * ld + i] = acc / CpM;
+        w[L.J + nS * ld + i] = acc / x.CpM;
     }
     // ddT_dtdT (gpuODESystem.H:129-146)
     double s_tt = 0.0;
     for (int i = g.lane; i < nS; i += G) s_tt += w[L.dfdx + i] * w[L.Cp + i] + w[L.J + i * ld + nS] * w[L.Ha + i];
     const double stt = g.sum(s_tt);
-    if (g.lane == 0) w[L.J + nS * ld + nS] = ((-stt) - dTdt * dCpMdT) / CpM;
+    if (g.lane == 0) w[L.J + nS * ld + nS] = ((-stt) - dTdt * x.dCpMdT) / x.CpM;
     g.sync();
     GF_PH_END(g, PH_TROW)
 }
@@ -1709,7 +1735,7 @@ __device__ __forceinline__ void shift_and_factor(const Grp<G>& g, const DevMech&
 template <int G, class W, int NB = 8>
 __device__ __forceinline__ void factor_step(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
                                             const RosCoeffs& C, int y0_off, double p, double dx) {
-    jacobian(g, M, w, L, y0_off, p, true);
+    jacobian(g, M, w, L, y0_off, p);
     shift_and_factor<G, W, NB>(g, M, w, L, C, dx);
 }
 
@@ -1721,13 +1747,15 @@ __device__ __forceinline__ void factor_step(const Grp<G>& g, const DevMech& M, c
 // LU); the stage points are kept at save_y2 / save_y3 and f at them at
 // save_f2 / save_f3.
 // F0 (the solve kernel): the attempt also evaluates the step's f(y0) into
-// dydx0 when first_deriv is set (the first attempt of a step), through the
-// stage loop's derivative call: one call site, a smaller instruction
-// footprint. Otherwise the caller provides dydx0.
+// dydx0, through the stage loop's derivative call: one call site, a smaller
+// instruction footprint. A retried step evaluates it again (the same value),
+// which brings back the rate constants that the Jacobian reads: cheaper than a
+// second copy of the rate code for the few retries (4 % of the attempts).
+// Otherwise the caller provides dydx0.
 template <int G, class W, bool SAVE = false, bool F0 = false, int NB = 8>
 __device__ __forceinline__ double ros_attempt(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L, const RosCoeffs& C,
                               const OdeParams& o, int y0_off, int yt_off, double p, double dx, int save_y2 = -1,
-                              int save_y3 = -1, bool first_deriv = false, int save_f2 = -1, int save_f3 = -1) {
+                              int save_y3 = -1, int save_f2 = -1, int save_f3 = -1) {
     const int m = M.m;
     const int ld = L.ld;
     if constexpr (!F0 && !SAVE) factor_step<G, W, NB>(g, M, w, L, C, y0_off, p, dx);
@@ -1735,10 +1763,10 @@ __device__ __forceinline__ double ros_attempt(const Grp<G>& g, const DevMech& M,
     // f_0 = f(y0), f_i = f(y0 + sum_j a_ij k_j) where the method takes a new
     // derivative (stage 1; stage 2 of Rosenbrock34), else the previous one.
     // One loop, so the solve and the derivative each have a single call site;
-    // with F0, pass st = -1 evaluates f(y0) (first_deriv) and factors the step.
+    // with F0, pass st = -1 evaluates f(y0) and factors the step.
 #pragma unroll 1
     for (int st = F0 ? -1 : 0; st < C.s; ++st) {
-        const bool new_f = st < 0 ? first_deriv : (st == 1 || (st == 2 && C.s == 4));
+        const bool new_f = st < 0 || st == 1 || (st == 2 && C.s == 4);
         int at = y0_off, out = L.dydx0;
         if (st > 0 && new_f) {
             // the stage point (kept at save_y2 / save_y3 when asked: the adjoint sweep)
@@ -1834,12 +1862,13 @@ __device__ __forceinline__ int ode_solve(const Grp<G>& g, const DevMech& M, cons
         double dx = step_dxTry;
         double err = 0.0;
         int rejects = 0;
-        // adaptiveSolve's derivatives call before its retry loop
-        // (gpuAdaptiveSolver.H:96): in the solve kernel, inside the first attempt
-        if constexpr (REC) derivatives(g, M, w, L, *y_off, p, L.dydx0, true);
         do {
             GF_PH_BEGIN(g)
-            err = ros_attempt<G, W, false, !REC, NB>(g, M, w, L, C, o, *y_off, *yt_off, p, dx, -1, -1, rejects == 0);
+            // adaptiveSolve's derivatives call (gpuAdaptiveSolver.H:96), which
+            // also leaves the rate constants for the attempt's Jacobian: in the
+            // solve kernel, inside the attempt
+            if constexpr (REC) derivatives(g, M, w, L, *y_off, p, L.dydx0, true);
+            err = ros_attempt<G, W, false, !REC, NB>(g, M, w, L, C, o, *y_off, *yt_off, p, dx);
             GF_PH_END(g, PH_ATTEMPT)
             ++*attempts;
             if (err > 1) {
@@ -1898,7 +1927,6 @@ __device__ __forceinline__ void process_cell_body(const Grp<G>& g, const DevMech
     const double dT = a.deltaT_cell ? a.deltaT_cell[cell] : a.deltaT;
     double dxTry = a.deltaTChem[cell];
     int status = GF_CELL_OK, accepted = 0, attempts = 0;
-    if (g.lane == 0) w[L.scal + S_KCACHE_T] = -1.0;
     g.sync();
     if (T0 > a.Treact) {
         const RosCoeffs C = ros_coeffs(a.ode.solver);

@@ -12,7 +12,7 @@
 //
 // One warp per cell with the cell's concentrations, third-body sums and
 // per-reaction staging in shared memory: the same device functions as the
-// solve (third_body_all, rate_k, reaction_lnKc, side_C, the dN/dt gather
+// solve (third_body_all, fast_kf, fast_lnKc, fast_C, the dN/dt gather
 // stream). Qdot is one thread per cell with the reference's sequential sum.
 #include <algorithm>
 #include <cfloat>
@@ -35,7 +35,7 @@ __host__ __device__ inline FieldLayout field_layout(const DevMech& M) {
     FieldLayout F{};
     int o = 0;
     F.L.c = o;
-    o += M.nS;
+    o += M.nS + 1;  // and a 1 for the absent species of a reaction side
     F.L.Mtb = o;
     o += M.n_tb > 0 ? M.n_tb : 1;
     F.L.stage = o;
@@ -55,20 +55,19 @@ __device__ __forceinline__ void stage_fields(const Grp<32>& g, const DevMech& M,
                                              const TCache& tc, bool want_tc, double* sumW, double* sumW2) {
     double sW = 0.0, sW2 = 0.0;
     for (int q = g.lane; q < M.nR; q += 32) {
-        Rxn R;
-        load_rxn(M, q, R);
-        const double Mc = R.tb_row >= 0 ? w[L.Mtb + R.tb_row] : 0.0;
-        double dummy, Ak = 0.0;
-        const double kf = rate_k(M, q, R, tc, Mc, false, &dummy, &Ak);
-        double kr = 0.0;
-        if (!R.irr) kr = kf * exp(-reaction_lnKc(M, q, R, tc, nullptr, nullptr));
-        const double omegaf = kf * side_C(M, w, L.c, R, 0);
-        const double omegar = kr * side_C(M, w, L.c, R, 1);
+        const RxnF R = load_fast(M, q);
+        const LnK a = load_lnK(M, q, tc.T);
+        double Ak;
+        const double kf = fast_kf(M, q, R, tc, fast_M(M, w, L.Mtb, R, q), &Ak);
+        const double kr = R.irr() ? 0.0 : kf * exp(-fast_lnKc(R, a, tc));
+        const double omegaf = kf * fast_C(M, w, L.c, R, q, 0);
+        const double omegar = kr * fast_C(M, w, L.c, R, q, 1);
         w[L.stage + R.slot] = omegaf - omegar;
         if (want_tc) {
             double wf = 0.0, wr = 0.0;
-            for (int e = 0; e < R.nr; ++e) wf += ldg(M.sst + R.sp_off + R.nl + e) * omegaf;
-            for (int e = 0; e < R.nl; ++e) wr += ldg(M.sst + R.sp_off + e) * omegar;
+            const double* st = M.sst + ldg(M.sp_off + q);
+            for (int e = 0; e < R.nr(); ++e) wf += ldg(st + R.nl() + e) * omegaf;
+            for (int e = 0; e < R.nl(); ++e) wr += ldg(st + e) * omegar;
             sW += wf + wr;
             sW2 += wf * wf + wr * wr;
         }
@@ -95,6 +94,7 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
             w[F.L.c + i] = ci;
             csum += ci;
         }
+        if (g.lane == 0) w[F.L.c + nS] = 1.0;
         g.sync();
         if (M.n_tb > 0) {
             third_body_all(g, M, w, F.L.c, F.L.Mtb);
@@ -110,23 +110,21 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
             g.sync();
             if (g.lane == 0) {
                 const int q = a.reaction_q;
-                Rxn R;
-                load_rxn(M, q, R);
-                const double Mc = R.tb_row >= 0 ? w[F.L.Mtb + R.tb_row] : 0.0;
-                double dummy, Ak = 0.0;
-                const double kf = rate_k(M, q, R, tcache, Mc, false, &dummy, &Ak);
-                double kr = 0.0;
-                if (!R.irr) kr = kf * exp(-reaction_lnKc(M, q, R, tcache, nullptr, nullptr));
-                const double om = kf * side_C(M, w, F.L.c, R, 0) - kr * side_C(M, w, F.L.c, R, 1);
+                const RxnF R = load_fast(M, q);
+                double Ak;
+                const double kf = fast_kf(M, q, R, tcache, fast_M(M, w, F.L.Mtb, R, q), &Ak);
+                const double kr = R.irr() ? 0.0 : kf * exp(-fast_lnKc(R, load_lnK(M, q, tcache.T), tcache));
+                const double om = kf * fast_C(M, w, F.L.c, R, q, 0) - kr * fast_C(M, w, F.L.c, R, q, 1);
                 if (a.omega) a.omega[cell] = om;
                 if (rr) {
                     // gpuReaction::dNdtByV (gpuReaction.H:490-508): lhs, then rhs
-                    for (int e = 0; e < R.nl; ++e) {
-                        const int b = R.sp_off + e;
+                    const int b0 = ldg(M.sp_off + q);
+                    for (int e = 0; e < R.nl(); ++e) {
+                        const int b = b0 + e;
                         w[F.out + ldg(M.sidx + b)] -= ldg(M.sst + b) * om;
                     }
-                    for (int e = 0; e < R.nr; ++e) {
-                        const int b = R.sp_off + R.nl + e;
+                    for (int e = 0; e < R.nr(); ++e) {
+                        const int b = b0 + R.nl() + e;
                         w[F.out + ldg(M.sidx + b)] += ldg(M.sst + b) * om;
                     }
                 }

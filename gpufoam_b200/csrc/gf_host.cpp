@@ -320,6 +320,16 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
             coef[(size_t)(7 + k) * nS + i] = t.high[k];
         }
     }
+    // species polynomials with the divisions of Ha (gpuThermo.H:210-221) done once
+    std::vector<double> spc((size_t)20 * nS), invW(nS);
+    for (int i = 0; i < nS; ++i) {
+        invW[i] = 1.0 / W[i];
+        for (int b = 0; b < 2; ++b) {
+            const double* a = b ? d->thermos[i].high : d->thermos[i].low;
+            const double v[10] = {a[0], a[1], a[2], a[3], a[4], a[1] / 2.0, a[2] / 3.0, a[3] / 4.0, a[4] / 5.0, a[5]};
+            for (int k = 0; k < 10; ++k) spc[(size_t)(b * 10 + k) * nS + i] = v[k];
+        }
+    }
     const int nRa = std::max(nR, 1);
     // compute order: reactions grouped by rate type (stable within a type)
     std::vector<int> qof(nRa, 0), rof(nRa, 0);  // q -> r and r -> q
@@ -458,6 +468,46 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
                 rxs[((size_t)q * 2 + side) * kSideInline + e] = RxnSpecie{sidx[b + e], siexp[b + e], sexp[b + e]};
         }
     }
+    // the solve's compact records: bit fields, species indices, ln K coefficients
+    std::vector<RxnFast> rxf(nRa);
+    std::vector<double> lnk((size_t)14 * nRa, 0.0);
+    double Tc_all = nR > 0 ? rTc[0] : 0.0;
+    for (int q = 0; q < nR; ++q) {
+        RxnFast& f = rxf[q];
+        if (rTc[q] != Tc_all) Tc_all = NAN;
+        bool general = nl[q] > kFastSide || nr[q] > kFastSide;
+        unsigned side_idx[2] = {0, 0};
+        int sq = 0;
+        for (int side = 0; side < 2; ++side) {
+            const int n = side == 0 ? nl[q] : nr[q];
+            const int b = sp_off[q] + (side == 0 ? 0 : nl[q]);
+            for (int e = 0; e < kFastSide; ++e) {
+                const unsigned i = e < n ? (unsigned)sidx[b + e] : (unsigned)nS;
+                side_idx[side] |= i << (10 * e);
+                if (e < n && siexp[b + e] == 2) sq |= 1 << (kFastSide * side + e);
+            }
+            for (int e = 0; e < n; ++e) general = general || (siexp[b + e] != 1 && siexp[b + e] != 2);
+        }
+        const int sign = sA0[q] > 0 ? 0 : (sA0[q] < 0 ? 1 : 2);
+        const int tb = tb_row[q] + 1 < kRxnTbFar ? tb_row[q] + 1 : kRxnTbFar;
+        f.meta = (int)((unsigned)rtype[q] | (rirr[q] ? kRxnIrr : 0) | (general ? kRxnGeneral : 0) |
+                       ((unsigned)sq << kRxnSqShift) | ((unsigned)sign << kRxnSignShift) |
+                       ((unsigned)nl[q] << kRxnNlShift) | ((unsigned)nr[q] << kRxnNrShift) |
+                       ((unsigned)tb << kRxnTbShift));
+        f.slot = slot[q];
+        f.lhs = side_idx[0];
+        f.rhs = side_idx[1];
+        f.lnA0 = lnA0[q];
+        f.beta0 = beta0[q];
+        f.Ta0 = Ta0[q];
+        f.nm = rnm_small[q] ? 0.0 : rnm[q];
+        // ln K = -Y G / (R T) as (b0 (1 - ln T) - b6) - (b1 + (b2 + (b3 + b4 T) T) T) T + b5 / T
+        const double sc = -rY[q] / kRR;
+        const double div[7] = {1.0, 2.0, 6.0, 12.0, 20.0, 1.0, 1.0};
+        for (int b = 0; b < 2; ++b)
+            for (int k = 0; k < 7; ++k)
+                lnk[(size_t)(b * 7 + k) * nRa + q] = sc * (rcoef[(size_t)(b * 7 + k) * nRa + q] / div[k]);
+    }
     const int ldJ = (nS + 1) | 1;  // the workspace Jacobian row stride (make_layout)
     std::vector<int> dn_pos(nS), je_pos(nE);
     for (int s2 = 0; s2 < nS; ++s2) dn_pos[s2] = s2;
@@ -517,13 +567,14 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
 
     // ---- one device allocation
     DevBuf b;
-    const size_t oW = b.add(W), oR = b.add(Rsp), oTc = b.add(Tc), oCoef = b.add(coef), oHf = b.add(hf);
+    const size_t oW = b.add(W), oR = b.add(Rsp), oTc = b.add(Tc), oCoef = b.add(coef), oHf = b.add(hf),
+                 oSpc = b.add(spc), oInvW = b.add(invW);
     const size_t oRt = b.add(rtype), oRi = b.add(rirr), oNl = b.add(nl), oNr = b.add(nr), oSpo = b.add(sp_off),
                  oSlot = b.add(slot), oRY = b.add(rY), oRnm = b.add(rnm), oRns = b.add(rnm_small), oRTc = b.add(rTc),
                  oRc = b.add(rcoef), oLA0 = b.add(lnA0), oSA0 = b.add(sA0), oB0 = b.add(beta0), oT0 = b.add(Ta0),
                  oLA1 = b.add(lnA1), oSA1 = b.add(sA1), oB1 = b.add(beta1), oT1 = b.add(Ta1), oTroe = b.add(troe),
                  oTb = b.add(tb_row), oEff = b.add(eff), oSi = b.add(sidx), oSie = b.add(siexp), oSst = b.add(sst),
-                 oSe = b.add(sexp), oRxh = b.add(rxh), oRxs = b.add(rxs), oRofq = b.add(qof);
+                 oSe = b.add(sexp), oRxh = b.add(rxh), oRxs = b.add(rxs), oRxf = b.add(rxf), oLnk = b.add(lnk), oRofq = b.add(qof);
     size_t oDst[kNumGroupSizes], oJst[kNumGroupSizes], oCst[kNumGroupSizes];
     for (int k = 0; k < kNumGroupSizes; ++k) {
         oDst[k] = b.add(dst_rec[k]);
@@ -559,6 +610,8 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
     D.Rsp = (const double*)P(oR);
     D.Tcommon = (const double*)P(oTc);
     D.coef = (const double*)P(oCoef);
+    D.spc = (const double*)P(oSpc);
+    D.invW = (const double*)P(oInvW);
     D.hf = (const double*)P(oHf);
     D.rtype = (const int*)P(oRt);
     D.rirr = (const int*)P(oRi);
@@ -585,6 +638,9 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
     D.r_of_q = (const int*)P(oRofq);
     D.rxh = (const RxnHead*)P(oRxh);
     D.rxs = (const RxnSpecie*)P(oRxs);
+    D.rxf = (const RxnFast*)P(oRxf);
+    D.lnk = (const double*)P(oLnk);
+    D.Tc_all = Tc_all;
     D.sidx = (const int*)P(oSi);
     D.siexp = (const int*)P(oSie);
     D.sst = (const double*)P(oSst);

@@ -28,6 +28,22 @@ struct __align__(16) RxnSpecie {
     double exp;
 };
 
+// The solve's per-reaction record (compute order q, 48 bytes, three 16-byte
+// loads): bit fields in meta (below), the first staging slot, up to kFastSide
+// species per side as 10-bit indices (a missing one is nS, where the workspace
+// holds a concentration of 1) and the k (or fall-off k0) factors. Wider sides
+// and exponents other than 1 and 2 (kRxnGeneral) take their products from the
+// stoichiometry tables instead (general_C).
+constexpr int kFastSide = 3;
+constexpr int kRxnType = 3, kRxnIrr = 4, kRxnGeneral = 8, kRxnSqShift = 4, kRxnSignShift = 10, kRxnNlShift = 12,
+              kRxnNrShift = 16, kRxnTbShift = 20;
+constexpr int kRxnTbFar = 4095;  // third-body row + 1, or: read tb_row[q]
+struct __align__(16) RxnFast {
+    int meta, slot;
+    unsigned lhs, rhs;
+    double lnA0, beta0, Ta0, nm;  // nm: 0 where Kc = K (gpuThermo.H:111)
+};
+
 // One record of a gather stream: acc += coef * src[slot] (slot < 0: nothing);
 // pos >= 0 marks the last record of an output entry: dst[pos] = acc, acc = 0.
 struct __align__(16) StreamRec {
@@ -82,6 +98,8 @@ struct DevMech {
     const double* Rsp;         // RR / W
     const double* Tcommon;
     const double* coef;
+    const double* spc;         // [2][10][nS]: Cp a0..a4, then a1/2, a2/3, a3/4, a4/5 and a5 of Ha (b = 0 low, 1 high)
+    const double* invW;        // 1 / W
     const double* hf;          // enthalpy of formation [J/kg] (Qdot)
     // reactions, compute order
     const int* rtype;
@@ -108,6 +126,9 @@ struct DevMech {
     const double* eff;         // [n_tb][nS]
     const int* r_of_q;         // [nR] mechanism index of the reaction in compute position q
     const RxnHead* rxh;        // [nR]
+    const RxnFast* rxf;        // [nR]
+    const double* lnk;         // [2][7][nR]: the coefficients of ln K (b = 0 low, 1 high), see reaction_lnK
+    double Tc_all;             // Tcommon of every reaction, or NaN where they differ
     const RxnSpecie* rxs;      // [nR][2 * kSideInline]: lhs, then rhs (wider sides: sidx/siexp/sexp)
     const int* sidx;
     const int* siexp;          // integer exponent or kNoIntExp

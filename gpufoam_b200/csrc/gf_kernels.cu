@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(32) jacobian_kernel(const DevMech M, const dou
     WsC w{smem};
     for (int i = g.lane; i < M.m; i += 32) w[L.y0 + i] = yi[i];
     const double p = yi[M.nS + 1];
+    derivatives(g, M, w, L, L.y0, p, L.dydx, true);  // leaves the rate constants for the Jacobian
     jacobian(g, M, w, L, L.y0, p);
     double* o = dfdx + (size_t)blockIdx.x * n;
     for (int i = g.lane; i < M.m; i += 32) o[i] = w[L.dfdx + i];
