@@ -1093,203 +1093,233 @@ __device__ __forceinline__ void lu_panel(const Grp<G>& g, const W& w, int A, int
     }
 }
 
-// Panel steps k0 .. k1-1 with the panel held in registers (one full warp):
-// register slot (lane l, r) holds a panel row (initially row k0 + l + 32 r)
-// with its row scaling, and a label: the row position it has in the
-// reference's matrix after the exchanges so far. An exchange of rows k and
-// iMax swaps the two slots' labels instead of moving data; the pivot search,
-// its tie-break ("last max wins" by position), the update condition and the
-// write-back all go by label. The row scaling stays with its data, which is
-// the reference's vv[iMax] = vv[k] (ludecompose.H:71-78); the scaling left at
-// position k is never read again. The pivot search reduces across lanes with
-// three integer warp reductions on order-preserving keys of the non-negative
-// candidates (high word, low word, then the largest position). Same
-// operations, in the same order per entry, as lu_panel. The pivots go to
-// piv[]; the exchanges of the columns outside the panel are left to
-// lu_apply_swaps. Difference: when every candidate of a column is NaN, the
-// reference exchanges row k with row 0 (its iMax starts at 0); here none is.
-template <int RP, int NB, bool EXACT = false, class W>
-__device__ __forceinline__ void lu_panel_reg(const Grp<32>& g, const W& w, int A, int ld, int piv, int vv, int m,
-                                             int k0, int k1) {
-    const int l = g.lane;
-    const int kb = k1 - k0;
-    double a[RP][NB];
-    double sv[RP];
-    int lab[RP];
+// c += a b for one 8 x 8 tile of doubles held by a warp (a: 8 x 4, b: 4 x 8;
+// lane l holds a[l/4][l%4], b[l%4][l/4], c[l/4][2 (l%4) + 0, 1]). The unit
+// accumulates its four products as a chain of FMAs in ascending k (measured on
+// the B200: 262,144 results of random tiles bit for bit), so a tile update is
+// the same as the scalar loop's.
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
+}
+
+constexpr int kPanel = 8;  // columns per panel of lu_decompose_mma: two tile depths
+
+// Panel steps k0 .. k0+kb-1 with the panel held in registers (one full warp):
+// lane l holds the rows at positions k0 + l + 32 r, each with its row scaling
+// and a label, the position that it has in the reference's matrix after the
+// exchanges so far (-1: no row). An exchange of rows k and iMax swaps two
+// labels; pivot search, tie-break ("last max wins" by position) and update go
+// by label, and at the end perm[] takes the labels: perm[position] = the row of
+// the workspace that holds it. Rows never move. The pivot search reduces the
+// high words of the non-negative candidates with one integer warp reduction;
+// only equal high words need the low words and the position. Meanwhile every
+// lane has formed the reciprocal of its own candidate, so the division is off
+// the chain of dependent operations. Difference: when every candidate of a
+// column is NaN, the reference exchanges row k with row 0 (its iMax starts at
+// 0); here none is. The reciprocal pivots go to rd, the pivots to piv.
+template <int RP, bool EXACT, class W>
+__device__ __forceinline__ void lu_panel_reg(const W& w, int A, int ld, int piv, int sc, int rd, int perm, int m,
+                                             int k0, int kb) {
+    const int l = threadIdx.x & 31;
+    double a[RP][kPanel], sv[RP];
+    int lab[RP], row[RP];
 #pragma unroll
     for (int r = 0; r < RP; ++r) {
         const int p = k0 + l + 32 * r;
-        lab[r] = p < m ? p : m;  // slots past the last row never qualify
+        lab[r] = p < m ? p : -1;
+        row[r] = p < m ? w.ip(perm + p) : 0;
+        sv[r] = p < m ? w[sc + row[r]] : 0.0;
 #pragma unroll
-        for (int t = 0; t < NB; ++t) a[r][t] = (p < m && t < kb) ? w[A + p * ld + k0 + t] : 0.0;
-        sv[r] = p < m ? w[vv + p] : 0.0;
+        for (int t = 0; t < kPanel; ++t) a[r][t] = (p < m && t < kb) ? w[A + row[r] * ld + k0 + t] : 0.0;
     }
 #pragma unroll
-    for (int kk = 0; kk < NB; ++kk) {
+    for (int kk = 0; kk < kPanel; ++kk) {
         if (kk >= kb) break;
         const int k = k0 + kk;
-        // pivot search: the last position with the largest vv * |a| (ludecompose.H:57-63)
-        double best = -1.0;
-        int bi = -1;
+        // the lane's candidate: the last position with the largest vv * |a|
+        // (ludecompose.H:57-63); a zero pivot becomes gpuSmall (:81)
+        double best = -1.0, x = 1.0;
+        int bi = -1, ri = 0;
 #pragma unroll
         for (int r = 0; r < RP; ++r) {
-            if (lab[r] >= k && lab[r] < m) {
-                const double t = sv[r] * fabs(a[r][kk]);
-                if (t > best || (t == best && lab[r] > bi)) {
-                    best = t;
-                    bi = lab[r];
-                }
+            const double t = sv[r] * fabs(a[r][kk]);
+            if (lab[r] >= k && (t > best || (t == best && lab[r] > bi))) {
+                best = t;
+                bi = lab[r];
+                ri = r;
+                x = a[r][kk];
             }
         }
+        if (x == 0.0) x = kSmall;
+        double rinv = 1.0 / x;
         const bool has = bi >= 0;
         const unsigned hi = has ? (unsigned)__double2hiint(best) : 0u;
-        const unsigned lo = has ? (unsigned)__double2loint(best) : 0u;
         const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-        const int mr =
-            (int)__reduce_max_sync(0xffffffffu, (has && hi == mh && lo == ml) ? (unsigned)(bi + 1) : 0u) - 1;
-        const int iMax = mr < 0 ? k : mr;
-        // the slot that holds position iMax becomes position k, and the slot
-        // that held position k becomes iMax
-        int ri = -1;
+        unsigned own = __ballot_sync(0xffffffffu, has && hi == mh);
+        if (__popc(own) != 1) {
+            const bool c = has && hi == mh;
+            const unsigned lo = c ? (unsigned)__double2loint(best) : 0u;
+            const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+            const int mr = (int)__reduce_max_sync(0xffffffffu, (c && lo == ml) ? (unsigned)(bi + 1) : 0u) - 1;
+            if (mr < 0) {
+                // no candidate (a column of NaN): row k stays
 #pragma unroll
-        for (int r = 0; r < RP; ++r)
-            if (lab[r] == iMax) ri = r;
-        const unsigned own = __ballot_sync(0xffffffffu, ri >= 0);
-        const int li = __ffs(own) - 1;
-        ri = __shfl_sync(0xffffffffu, ri, li);
-        if (iMax != k) {
-#pragma unroll
-            for (int r = 0; r < RP; ++r) {
-                if (lab[r] == k)
-                    lab[r] = iMax;
-                else if (lab[r] == iMax)
-                    lab[r] = k;
+                for (int r = 0; r < RP; ++r)
+                    if (lab[r] == k) {
+                        bi = k;
+                        ri = r;
+                        x = a[r][kk];
+                        rinv = x;
+                    }
             }
+            own = __ballot_sync(0xffffffffu, bi == (mr < 0 ? k : mr));
         }
-        if (l == 0) w.ip(piv + k) = iMax;
-        // pivot row (now position k), broadcast; a zero pivot becomes gpuSmall (:81)
-        double urow[NB];
+        const int li = __ffs(own) - 1;
+        rinv = __shfl_sync(0xffffffffu, rinv, li);
+        const int iMax = __shfl_sync(0xffffffffu, bi, li);
+        // the pivot row's remaining entries, to every lane
+        double u[kPanel];
 #pragma unroll
-        for (int t = 0; t < NB; ++t) {
-            double x = a[0][t];
+        for (int t = kk + 1; t < kPanel; ++t) {
+            double y = a[0][t];
 #pragma unroll
             for (int r = 1; r < RP; ++r)
-                if (r == ri) x = a[r][t];
-            urow[t] = (t >= kk && t < kb) ? __shfl_sync(0xffffffffu, x, li) : 0.0;
+                if (r == ri) y = a[r][t];
+            u[t] = __shfl_sync(0xffffffffu, y, li);
         }
-        if (urow[kk] == 0.0) {
-            urow[kk] = kSmall;
 #pragma unroll
-            for (int r = 0; r < RP; ++r)
-                if (l == li && r == ri) a[r][kk] = kSmall;
+        for (int r = 0; r < RP; ++r) {
+            if (l == li && r == ri) {
+                lab[r] = k;
+                a[r][kk] = x;
+            } else if (lab[r] == k) {
+                lab[r] = iMax;
+            }
         }
-        if (k != m - 1) {
-            const double rDiag = 1.0 / urow[kk];
+        if (l == 0) {
+            w.ip(piv + k) = iMax;
+            w[rd + k] = rinv;
+        }
 #pragma unroll
-            for (int r = 0; r < RP; ++r) {
-                if (lab[r] > k && lab[r] < m) {
-                    const double lik = a[r][kk] * rDiag;
-                    a[r][kk] = lik;
+        for (int r = 0; r < RP; ++r) {
+            if (lab[r] > k) {
+                const double lik = a[r][kk] * rinv;
+                a[r][kk] = lik;
 #pragma unroll
-                    for (int t = kk + 1; t < NB; ++t)
-                        if (t < kb) a[r][t] = msub<EXACT>(a[r][t], lik, urow[t]);
-                }
+                for (int t = kk + 1; t < kPanel; ++t) a[r][t] = msub<EXACT>(a[r][t], lik, u[t]);
             }
         }
     }
 #pragma unroll
     for (int r = 0; r < RP; ++r) {
-        if (lab[r] < m) {
+        if (lab[r] >= 0) {
 #pragma unroll
-            for (int t = 0; t < NB; ++t)
-                if (t < kb) w[A + lab[r] * ld + k0 + t] = a[r][t];
-            w[vv + lab[r]] = sv[r];
+            for (int t = 0; t < kPanel; ++t)
+                if (t < kb) w[A + row[r] * ld + k0 + t] = a[r][t];
+            w.ip(perm + lab[r]) = row[r];
         }
     }
 }
 
-// The row exchanges of panel steps k0 .. k1-1 (pivots in piv[]) applied in
-// order to one column j outside the panel.
-template <class W>
-__device__ __forceinline__ void lu_apply_swaps(const W& w, int A, int ld, int piv, int k0, int k1, int j) {
-    for (int k = k0; k < k1; ++k) {
-        const int iMax = w.ip(piv + k);
-        if (iMax != k) {
-            const double t = w[A + k * ld + j];
-            w[A + k * ld + j] = w[A + iMax * ld + j];
-            w[A + iMax * ld + j] = t;
-        }
-    }
-}
-
-// Register-panel form of the blocked LU for a full warp or a multi-warp group
-// (m <= 32 RP, RP panel rows per lane): warp 0 factors each panel in registers; every column outside the
-// panel takes the panel's row exchanges, then (columns right of the panel) its
-// U12 rows; then the trailing matrix is updated (lanes over columns, warps over
-// rows). Every entry receives its updates in k order, as in lu_decompose.
-template <int G, int NB, bool EXACT = false, int RP = 2, class W>
-__device__ __forceinline__ void lu_decompose_regpanel(const Grp<G>& g, const W& w, int A, int ld, int piv, int vv,
-                                                      int m) {
-    constexpr int NWp = G > 32 ? G / 32 : 1;
+// Blocked LU for a full warp or a multi-warp group (m <= 32 RP): warp 0 factors
+// panels of 8 columns in registers (lu_panel_reg); the U12 rows take their
+// updates with lanes over columns; the trailing matrix is updated in 8 x 8
+// tiles by the FP64 matrix instruction, the tiles shared out to the warps in
+// runs along a tile row (the run keeps its part of L in registers). Rows are
+// never exchanged: position i of the reference's matrix is row perm[i], and the
+// solves follow perm. Every entry receives its updates in k order, as in
+// lu_decompose, so factors and pivots are the same bit for bit (EXACT: scalar
+// updates with two roundings). sc: the row scalings; rd: out, 1 / U[i][i].
+//
+// Why: the factorisation was 30k of the 108k warp instructions of an attempt
+// (m = 54, 128 threads): rank-4 updates spent eleven instructions on four FMAs,
+// and the exchanges another pass. A tile takes 16 instructions for 512 FMAs.
+// A form with the whole matrix in registers and one barrier per column was
+// slower (rank-1 updates: 62k instructions).
+template <int G, int RP, bool EXACT, class W>
+__device__ __forceinline__ void lu_decompose_mma(const Grp<G>& g, const W& w, int A, int ld, int piv, int sc, int rd,
+                                                 int perm, int m) {
+    constexpr int NW = G / 32;
     const int wid = g.warp();
-    const int l = G > 32 ? (int)(threadIdx.x & 31) : g.lane;
-    for (int k0 = 0; k0 < m; ) {
-        const int kb = min(NB, m - k0);
-        const int k1 = k0 + kb;
+    const int l = threadIdx.x & 31;
+    for (int i = g.lane; i < m; i += G) w.ip(perm + i) = i;
+    g.sync();
+#pragma unroll 1
+    for (int k0 = 0;; k0 += kPanel) {
+        const int k1 = min(k0 + kPanel, m);
         {
             GF_PH_BEGIN(g)
-            if (wid == 0) {
-                Grp<32> g32;
-                lu_panel_reg<RP, NB, EXACT>(g32, w, A, ld, piv, vv, m, k0, k1);
-            }
+            if (wid == 0) lu_panel_reg<RP, EXACT>(w, A, ld, piv, sc, rd, perm, m, k0, k1 - k0);
             g.sync();
             GF_PH_END(g, PH_LU_PANEL)
         }
+        if (k1 >= m) break;
         {
             GF_PH_BEGIN(g)
-            // row exchanges outside the panel, and U12 of the columns right of it
-            for (int j = g.lane; j < m - kb; j += G) {
-                const int jj = j < k0 ? j : j + kb;
-                lu_apply_swaps(w, A, ld, piv, k0, k1, jj);
-                if (jj >= k1) {
-                    double u[NB];
+            // U12: rows k0 .. k1-1 (a full panel), columns k1 .. m-1
+            if (k1 + (g.lane & ~31) < m) {
+                int ro[kPanel];
 #pragma unroll
-                    for (int t = 0; t < NB; ++t) u[t] = t < kb ? w[A + (k0 + t) * ld + jj] : 0.0;
+                for (int t = 0; t < kPanel; ++t) ro[t] = A + w.ip(perm + k0 + t) * ld;
+                for (int j = k1 + g.lane; j < m; j += G) {
+                    double u[kPanel];
 #pragma unroll
-                    for (int t = 1; t < NB; ++t) {
-                        if (t < kb) {
-                            double v = u[t];
+                    for (int t = 0; t < kPanel; ++t) u[t] = w[ro[t] + j];
 #pragma unroll
-                            for (int t2 = 0; t2 < t; ++t2) v = msub<EXACT>(v, w[A + (k0 + t) * ld + k0 + t2], u[t2]);
-                            u[t] = v;
-                            w[A + (k0 + t) * ld + jj] = v;
-                        }
+                    for (int t = 1; t < kPanel; ++t) {
+#pragma unroll
+                        for (int t2 = 0; t2 < t; ++t2) u[t] = msub<EXACT>(u[t], w[ro[t] + k0 + t2], u[t2]);
+                        w[ro[t] + j] = u[t];
                     }
                 }
             }
             g.sync();
             GF_PH_END(g, PH_LU_U12)
         }
-        if (k1 >= m) break;
-        {
-            GF_PH_BEGIN(g)
-            for (int j = k1 + l; j < m; j += 32) {
-                double u[NB];
-#pragma unroll
-                for (int t = 0; t < NB; ++t) u[t] = t < kb ? w[A + (k0 + t) * ld + j] : 0.0;
-                for (int i = k1 + wid; i < m; i += NWp) {
-                    double a = w[A + i * ld + j];
-#pragma unroll
-                    for (int t = 0; t < NB; ++t)
-                        if (t < kb) a = msub<EXACT>(a, w[A + i * ld + k0 + t], u[t]);
-                    w[A + i * ld + j] = a;
+        GF_PH_BEGIN(g)
+        if constexpr (EXACT) {
+            for (int j = k1 + l; j < m; j += 32)
+                for (int i = k1 + wid; i < m; i += NW) {
+                    const int ri = A + w.ip(perm + i) * ld;
+                    double a = w[ri + j];
+                    for (int t = k0; t < k1; ++t) a = msub<true>(a, w[ri + t], w[A + w.ip(perm + t) * ld + j]);
+                    w[ri + j] = a;
                 }
+        } else {
+            const int nt = (m - k1 + 7) >> 3;
+            const int T = nt * nt;
+            int t = wid * T / NW;
+            const int t_end = (wid + 1) * T / NW;
+            int tr = t / nt, tc = t - tr * nt;
+            const int r8 = l >> 2, c4 = l & 3;
+            const int p0 = A + w.ip(perm + k0 + c4) * ld, p1 = A + w.ip(perm + k0 + 4 + c4) * ld;
+            while (t < t_end) {
+                const int i = k1 + 8 * tr + r8;
+                const bool rin = i < m;
+                const int ri = A + (rin ? w.ip(perm + i) : 0) * ld;
+                const double a0 = rin ? -w[ri + k0 + c4] : 0.0, a1 = rin ? -w[ri + k0 + 4 + c4] : 0.0;
+                const int run = min(nt - tc, t_end - t);
+                int col = k1 + 8 * tc;
+                for (int n = 0; n < run; ++n, col += 8) {
+                    const bool bin = col + r8 < m;
+                    const double b0 = bin ? w[p0 + col + r8] : 0.0, b1 = bin ? w[p1 + col + r8] : 0.0;
+                    const int j = col + 2 * c4;
+                    const bool in0 = rin && j < m, in1 = rin && j + 1 < m;
+                    double c0 = in0 ? w[ri + j] : 0.0, c1 = in1 ? w[ri + j + 1] : 0.0;
+                    mma_f64(c0, c1, a0, b0);
+                    mma_f64(c0, c1, a1, b1);
+                    if (in0) w[ri + j] = c0;
+                    if (in1) w[ri + j + 1] = c1;
+                }
+                t += run;
+                ++tr;
+                tc = 0;
             }
-            g.sync();
-            GF_PH_END(g, PH_LU_TRAIL)
         }
-        k0 = k1;
+        g.sync();
+        GF_PH_END(g, PH_LU_TRAIL)
     }
 }
 
@@ -1446,7 +1476,7 @@ constexpr int kRegRows = 160;
 // permutation as a gather list (perm) or follow the pivots step by step (piv).
 template <int G>
 __host__ __device__ constexpr bool solve_uses_perm(int m) {
-    return (G >= 32 && m <= 64) || (G > 32 && m <= 128) || (G >= 16 && G <= 32 && m <= kRegRows);
+    return (G >= 32 && m <= 128) || (G >= 16 && G <= 32 && m <= kRegRows);
 }
 
 // The solve kernels' layout for a group of G threads: the pivot array the
@@ -1515,7 +1545,8 @@ __device__ __forceinline__ void lu_solve_reg(const Grp<G>& g, const W& w, int A,
 }
 
 // Register form for one full warp with R rows per lane (m <= 32 R): lane l
-// holds rows l + 32 u. The steps run in tiles of 32, the step loop unrolled by
+// holds rows l + 32 u (row perm[i] of the factors at position i,
+// lu_decompose_mma). The steps run in tiles of 32, the step loop unrolled by
 // kSolveUnroll (4: measured faster than 8, 16 and full unrolling, whose code
 // costs more in instruction fetch inside the solve kernel than it saves), so
 // the loads of later steps can be issued early (the loop stores nothing).
@@ -1528,13 +1559,16 @@ template <int R, class W>
 __device__ __forceinline__ void lu_solve_warp(const W& w, int A, int ld, int perm, int rdiag, int m, int b) {
     const int lane = threadIdx.x & 31;
     double x[R];
+    int ro[R];  // the row of the factors at position 32 u + lane
     bool in[R];
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < R; ++u) {
         const int i = u * 32 + lane;
         in[u] = i < m;
-        x[u] = in[u] ? w[b + w.ip(perm + i)] : 0.0;
+        const int pi = in[u] ? w.ip(perm + i) : 0;
+        ro[u] = A + pi * ld;
+        x[u] = in[u] ? w[b + pi] : 0.0;
     }
     // forward substitution with the unit lower factor, column by column
 #pragma unroll
@@ -1545,10 +1579,10 @@ __device__ __forceinline__ void lu_solve_warp(const W& w, int A, int ld, int per
             const int j = 32 * t + l;
             if (j >= m - 1) break;
             const double bj = __shfl_sync(0xffffffffu, x[t], l);
-            if (lane > l && in[t]) x[t] -= w[A + (32 * t + lane) * ld + j] * bj;
+            if (lane > l && in[t]) x[t] -= w[ro[t] + j] * bj;
 #pragma unroll
             for (int u = t + 1; u < R; ++u)
-                if (in[u]) x[u] -= w[A + (32 * u + lane) * ld + j] * bj;
+                if (in[u]) x[u] -= w[ro[u] + j] * bj;
         }
     }
     // backward substitution, descending columns, x_j = (...) * (1 / U[j][j])
@@ -1561,9 +1595,9 @@ __device__ __forceinline__ void lu_solve_warp(const W& w, int A, int ld, int per
             if (j >= m) continue;
             const double xj = __shfl_sync(0xffffffffu, x[t], l) * w[rdiag + j];
             if (lane == l) x[t] = xj;
-            if (lane < l) x[t] -= w[A + (32 * t + lane) * ld + j] * xj;
+            if (lane < l) x[t] -= w[ro[t] + j] * xj;
 #pragma unroll
-            for (int u = 0; u < t; ++u) x[u] -= w[A + (32 * u + lane) * ld + j] * xj;
+            for (int u = 0; u < t; ++u) x[u] -= w[ro[u] + j] * xj;
         }
     }
 #pragma unroll
@@ -1587,15 +1621,12 @@ __device__ __forceinline__ void lu_solve_any(const Grp<G>& g, const W& w, int A,
             GF_PH_END(g, PH_SOLVE)
             return;
         }
-        if constexpr (G > 32) {
-            // 64 < m <= 128 (the 100-species mechanism): four rows per lane,
-            // instead of the shared-memory form with a barrier per step
-            if (m <= 128) {
-                g.sync();
-                if (g.lane < 32) lu_solve_warp<4>(w, A, ld, perm, rdiag, m, b);
-                g.sync();
-                return;
-            }
+        // 64 < m <= 128 (the 100-species mechanism): four rows per lane
+        if (m <= 128) {
+            g.sync();
+            if (G == 32 || g.lane < 32) lu_solve_warp<4>(w, A, ld, perm, rdiag, m, b);
+            g.sync();
+            return;
         }
     }
     if constexpr (G >= 16 && G <= 32) {
@@ -1607,29 +1638,34 @@ __device__ __forceinline__ void lu_solve_any(const Grp<G>& g, const W& w, int A,
     lu_solve(g, w, A, ld, piv, m, b);
 }
 
-// The factorisation as the solve kernels run it, after the row scaling vv:
-// the register-panel form for a full warp or a multi-warp group (m <= 64),
-// the blocked form otherwise, both with panels of NB columns; then, for groups of 16 or more threads, the
-// reciprocal pivots 1 / U[i][i] (written over vv, which is no longer needed)
+// The factorisation as the solve kernels run it, after the row scaling sc: by
+// register panels and matrix tiles for 32 or more threads (m <= 128; rows left
+// in place, perm), the blocked form otherwise, with panels of NB columns and
+// rows exchanged; then, for groups of 16 or more threads, the reciprocal pivots
+// 1 / U[i][i] in rd (sc and rd may be the same array for fewer than 32 threads)
 // and the row permutation of the solves (lu_solve_any).
 template <int G, bool EXACT = false, int NB = 8, class W>
-__device__ __forceinline__ void lu_factor(const Grp<G>& g, const W& w, int A, int ld, int piv, int vv, int perm,
-                                          int m) {
+__device__ __forceinline__ void lu_factor(const Grp<G>& g, const W& w, int A, int ld, int piv, int sc, int rd,
+                                          int perm, int m) {
+    if constexpr (G >= 32) {
+        if (m <= 128) {
+            GF_PH_BEGIN(g)
+            if (m <= 64)
+                lu_decompose_mma<G, 2, EXACT>(g, w, A, ld, piv, sc, rd, perm, m);
+            else
+                lu_decompose_mma<G, 4, EXACT>(g, w, A, ld, piv, sc, rd, perm, m);
+            GF_PH_END(g, PH_LU)
+            return;
+        }
+    }
     {
         GF_PH_BEGIN(g)
-        bool done = false;
-        if constexpr (G >= 32) {
-            if (m <= 64) {
-                lu_decompose_regpanel<G, NB, EXACT>(g, w, A, ld, piv, vv, m);
-                done = true;
-            }
-        }
-        if (!done) lu_decompose_blocked<G, NB, EXACT>(g, w, A, ld, piv, vv, m);
+        lu_decompose_blocked<G, NB, EXACT>(g, w, A, ld, piv, sc, m);
         GF_PH_END(g, PH_LU)
     }
     if (G >= 16) {
         GF_PH_BEGIN(g)
-        for (int i = g.lane; i < m; i += G) w[vv + i] = 1.0 / w[A + i * ld + i];
+        for (int i = g.lane; i < m; i += G) w[rd + i] = 1.0 / w[A + i * ld + i];
         lu_perm(g, w, piv, perm, m);
         GF_PH_END(g, PH_LU_PERM)
     }
@@ -1723,12 +1759,13 @@ __device__ __forceinline__ void shift_and_factor(const Grp<G>& g, const DevMech&
                                                  const RosCoeffs& C, double dx) {
     const int m = M.m;
     const int ld = L.ld;
+    const int sc = G >= 32 ? L.k2 : L.vv;  // the row scalings; the stages are not written yet
     {
         GF_PH_BEGIN(g)
-        shift_and_scale(g, w, L.J, ld, L.vv, m, 1.0 / (C.gamma * dx));
+        shift_and_scale(g, w, L.J, ld, sc, m, 1.0 / (C.gamma * dx));
         GF_PH_END(g, PH_SHIFT)
     }
-    lu_factor<G, false, NB>(g, w, L.J, ld, L.piv, L.vv, L.perm, m);
+    lu_factor<G, false, NB>(g, w, L.J, ld, L.piv, sc, L.vv, L.perm, m);
 }
 
 // The Jacobian at y0, then shift_and_factor.

@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(32) lusolve_kernel(int m, const double* LU, co
 
 // The factorisation and the solves exactly as the solve kernels run them
 // (lu_factor, lu_solve_any) with a group of G threads per matrix: after the
-// row scaling of LUDecompose, the register-panel form (G >= 32, m <= 64) or the
-// blocked one, reciprocal pivots for G >= 16; EXACT rounds every update a - l u
+// row scaling of LUDecompose, the register-panel form with matrix tiles
+// (G >= 32, m <= 128) or the blocked one, reciprocal pivots for G >= 16; EXACT rounds every update a - l u
 // twice, as the reference's CPU build does. One matrix per CTA; A [m][m] is
 // replaced by its factors, b [n_rhs][m] by the solutions.
 template <int G, bool EXACT>
@@ -125,21 +125,26 @@ __global__ void __launch_bounds__(G < 32 ? 32 : G) lu_form_kernel(int m, double*
     if (G < 32 && threadIdx.x >= G) return;
     const int ld = m | 1;
     WsC w{smem};
-    const int oA = 0, ovv = m * ld, opiv = ovv + m, operm = opiv + m, ob = operm + m;
+    const int oA = 0, osc = m * ld, ord = osc + m, opiv = ord + m, operm = opiv + m, ob = operm + m;
     double* Ag = A + (size_t)blockIdx.x * m * m;
     for (int e = g.lane; e < m * m; e += G) w[oA + (e / m) * ld + (e % m)] = Ag[e];
     g.sync();
-    row_scale(g, w, oA, ld, ovv, m);
-    lu_factor<G, EXACT>(g, w, oA, ld, opiv, ovv, operm, m);
+    row_scale(g, w, oA, ld, osc, m);
+    lu_factor<G, EXACT>(g, w, oA, ld, opiv, osc, ord, operm, m);
     g.sync();
-    for (int e = g.lane; e < m * m; e += G) Ag[e] = w[oA + (e / m) * ld + (e % m)];
+    // the factors in the reference's row order
+    const bool by_perm = G >= 32 && m <= 128;
+    for (int e = g.lane; e < m * m; e += G) {
+        const int i = by_perm ? w.ip(operm + e / m) : e / m;
+        Ag[e] = w[oA + i * ld + e % m];
+    }
     for (int i = g.lane; i < m; i += G) piv[(size_t)blockIdx.x * m + i] = w.ip(opiv + i);
     for (int r = 0; r < n_rhs; ++r) {
         double* bg = b + ((size_t)blockIdx.x * n_rhs + r) * m;
         g.sync();
         for (int i = g.lane; i < m; i += G) w[ob + i] = bg[i];
         g.sync();
-        lu_solve_any(g, w, oA, ld, opiv, operm, ovv, m, ob);
+        lu_solve_any(g, w, oA, ld, opiv, operm, ord, m, ob);
         g.sync();
         for (int i = g.lane; i < m; i += G) bg[i] = w[ob + i];
     }
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(G < 32 ? 32 : G) lu_form_kernel(int m, double*
 
 template <int G, bool EXACT>
 static int launch_lu_form_g(int n_mats, int m, double* A, int* piv, double* b, int n_rhs, cudaStream_t s) {
-    const size_t smem = ((size_t)m * (m | 1) + 4 * (size_t)m) * sizeof(double);
+    const size_t smem = ((size_t)m * (m | 1) + 5 * (size_t)m) * sizeof(double);
     const void* fn = reinterpret_cast<const void*>(&lu_form_kernel<G, EXACT>);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;

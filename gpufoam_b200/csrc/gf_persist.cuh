@@ -62,7 +62,7 @@ struct PersistShape {
     static constexpr int max_regs(int slim) { return slim ? 128 : (G == 64 ? 200 : 255); }
 };
 
-// NB: columns per LU panel; MS > 0: the matrix size m of every mechanism of
+// NB: columns per LU panel of the blocked form (groups of less than 32 threads, m > 128); MS > 0: the matrix size m of every mechanism of
 // the launch, fixed at compile time (process_cell).
 template <int G, bool SHARED, int SLIM, int NB = 8, int MS = 0>
 __global__ void __maxnreg__(PersistShape<G>::max_regs(SLIM))
