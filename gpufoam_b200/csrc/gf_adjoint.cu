@@ -74,7 +74,7 @@ __host__ __device__ inline AdjLayout make_adj_layout(const WsLayout& L, int nS, 
     A.dfc = o; o += m;                // its dfdx
     A.cb = o; o += nS;
     A.Mb = o; o += (n_tb > 0 ? n_tb : 1);
-    A.gq = o; o += 2 * kSideInline * (nR > 0 ? nR : 1);
+    A.gq = o; o += 2 * kSideInline * (nR > 0 ? nR : 1) + 1;  // and a 0 for the gather's missing records
     A.ms = o; o += MS_N;
     A.vb = o; o += 4 * nS;           // Cp, Ha, rhoM/W, v adjoints
     A.dn = o; o += nS;               // dN/dt adjoints
@@ -172,32 +172,6 @@ __device__ void lu_solve_transposed(const Grp<G>& g, const W& w, const WsC& wa, 
             lu_solve_transposed_warp<10, false>(w, wa, A, ld, perm, m, b, x);
     }
     g.sync();
-}
-
-// stream_gather with the sources in one workspace and the results in another
-template <int G, class WS, class WD>
-__device__ __forceinline__ void stream_gather2(const Grp<G>& g, const Stream& st, const WS& ws, int src, const WD& wd,
-                                               int dst) {
-    constexpr int U = GF_GATHER_BATCH;
-    const int4* r = reinterpret_cast<const int4*>(st.rec) + g.lane;
-    const int len = st.len;
-    double acc = 0.0;
-    for (int k0 = 0; k0 < len; k0 += U) {
-        int4 v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = (k0 + u < len) ? __ldg(r + (size_t)(k0 + u) * G) : make_int4(-1, -1, 0, 0);
-        double x[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) x[u] = v[u].y >= 0 ? ws[src + v[u].y] : 0.0;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (v[u].y >= 0) acc += __hiloint2double(v[u].w, v[u].z) * x[u];
-            if (v[u].x >= 0) {
-                wd[dst + v[u].x] = acc;
-                acc = 0.0;
-            }
-        }
-    }
 }
 
 // Mixture of the state at y (gpuMixture.H:33-121), as mixture() computes it,
@@ -417,7 +391,7 @@ __device__ void adj_reactions(const Grp<G>& g, const DevMech& M, const W& w, con
 // plus the third-body terms c_bar[i] += sum_t Mbar[t] eff[t][i].
 template <int G, class W>
 __device__ void adj_gather_c(const Grp<G>& g, const DevMech& M, const W& w, const WsC& wa, const AdjLayout& A) {
-    stream_gather(g, M.cst[stream_index(G)], wa, A.gq, A.dd);
+    stream_gather(g, M.cst[stream_index(G)], wa, A.gq, wa, A.dd);
     g.sync();
     for (int i = g.lane; i < M.nS; i += G) {
         double acc = wa[A.cb + i] + wa[A.dd + i];
@@ -622,7 +596,7 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
         jacobian<true>(g, M, w, L, L.y0, p);
         // kept for the Jacobian term: the raw entries (from the Jacobian terms
         // in the staging slots), the converted Jacobian and dfdx
-        stream_gather2(g, M.jst[stream_index(G)], w, L.stage, wa, A.raw);
+        stream_gather(g, M.jst[stream_index(G)], w, L.stage, wa, A.raw);
         for (int e = g.lane; e < m * ld; e += G) wa[A.Jc + e] = w[L.J + e];
         for (int i = g.lane; i < m; i += G) wa[A.dfc + i] = w[L.dfdx + i];
         g.sync();
@@ -699,6 +673,10 @@ __global__ void __launch_bounds__(64) adjoint_kernel(const DevMech M, const AdjA
     WsC wa{a.ws + (size_t)blockIdx.x * a.ws_per_cell};
     const RosCoeffs C = ros_coeffs(a.ode.solver);
     const int nS = M.nS, m = M.m;
+    if (g.lane == 0) {
+        w[L.stage + M.n_slots] = 0.0;
+        wa[A.gq + 2 * kSideInline * (M.nR > 0 ? M.nR : 1)] = 0.0;
+    }
     for (;;) {
         long long cell = 0;
         if (g.lane == 0) cell = (long long)atomicAdd(a.queue, 1ull);

@@ -62,17 +62,6 @@ enum { PH_MIX = 0, PH_NMPOW, PH_OMEGA, PH_GATHER_RHS, PH_JPARAMS, PH_JROWS, PH_T
        PH_ADJ_RXN, PH_ATTEMPT, PH_ADJ_RECOMPUTE, PH_ADJ_TSOLVE, PH_ADJ_VJP, PH_ADJ_JTERM, PH_LU_PANEL, PH_LU_U12,
        PH_LU_TRAIL, PH_LU_PERM };
 
-// Unroll depths of two latency-bound loops: third-body rows whose loads are in
-// flight together (third_body_all) and gather-stream records per batch
-// (stream_gather). 4 each: measured faster on the B200 than 8 (more loads in
-// flight, but more code to fetch inside the solve kernel) and than 2.
-#ifndef GF_TB_ROWS
-#define GF_TB_ROWS 4
-#endif
-#ifndef GF_GATHER_BATCH
-#define GF_GATHER_BATCH 4
-#endif
-
 // ---------------------------------------------------------------- groups
 
 // Cross-warp reduction buffers of a multi-warp group (one group per CTA): two,
@@ -186,6 +175,10 @@ struct WsC {
     double* p;
     __device__ __forceinline__ double& operator[](int i) const { return p[i]; }
     __device__ __forceinline__ int& ip(int i) const { return *reinterpret_cast<int*>(p + i); }
+    // the element `bytes` behind element i of a contiguous one
+    __device__ __forceinline__ double at(int i, int bytes) const {
+        return *reinterpret_cast<const double*>(reinterpret_cast<const char*>(p + i) + bytes);
+    }
 };
 // Interleaved workspace: element i of a cell at p[i * s] (p already offset by
 // the cell's slot), so that consecutive threads touch consecutive addresses.
@@ -194,6 +187,7 @@ struct WsS {
     long long s;
     __device__ __forceinline__ double& operator[](int i) const { return p[(long long)i * s]; }
     __device__ __forceinline__ int& ip(int i) const { return *reinterpret_cast<int*>(p + (long long)i * s); }
+    __device__ __forceinline__ double at(int i, int bytes) const { return p[(long long)(i + (bytes >> 3)) * s]; }
 };
 
 template <class T>
@@ -440,59 +434,24 @@ __device__ __forceinline__ double fast_dlnKcdT(const RxnF& R, const LnK& a, cons
 
 // Third-body concentrations M_t = sum_i eff_ti c_i of every third-body and
 // fall-off reaction (gpuThirdBodyEfficiencies.H:28-35), written to Mtb[t]:
-// lanes over species (coalesced rows of eff), warps over reactions, rows in
-// batches of GF_TB_ROWS so that their loads are in flight together; each sum is
-// lane-strided and combined by a fixed shuffle tree (deterministic; the
-// reference sums sequentially, an ulp-level reordering).
+// threads over reactions, the even and the odd species each in order, the
+// efficiencies species by species so that a warp's loads are consecutive. A
+// warp per reaction with a shuffle tree took 4.8k warp instructions for 75
+// reactions of 53 species; this takes 0.6k.
 template <int G, class W>
 __device__ __forceinline__ void third_body_all(const Grp<G>& g, const DevMech& M, const W& w, int c_off, int m_off) {
-    constexpr int LW = G > 32 ? 32 : G;
-    constexpr int NW = G > 32 ? G / 32 : 1;
-    constexpr int RB = GF_TB_ROWS;
-    constexpr int SPL = 3;  // species per lane held at once: nS <= SPL * LW, else looped
-    const int rg = G > 32 ? (g.lane >> 5) : 0;
-    const int rl = G > 32 ? (g.lane & 31) : g.lane;
-    const unsigned mask = G > 32 ? 0xffffffffu : g.mask;
-    const int nS = M.nS;
-    for (int t0 = rg * RB; t0 < M.n_tb; t0 += NW * RB) {
-        double sum[RB];
-        if (nS <= SPL * LW) {
-            double cv[SPL];
-#pragma unroll
-            for (int k = 0; k < SPL; ++k) {
-                const int i = rl + k * LW;
-                cv[k] = i < nS ? w[c_off + i] : 0.0;
-            }
-            double e[RB][SPL];
-#pragma unroll
-            for (int b = 0; b < RB; ++b)
-#pragma unroll
-                for (int k = 0; k < SPL; ++k) {
-                    const int i = rl + k * LW;
-                    e[b][k] = (t0 + b < M.n_tb && i < nS) ? ldg(M.eff + (size_t)(t0 + b) * nS + i) : 0.0;
-                }
-#pragma unroll
-            for (int b = 0; b < RB; ++b) {
-                double acc = 0.0;
-#pragma unroll
-                for (int k = 0; k < SPL; ++k) acc += e[b][k] * cv[k];
-                sum[b] = acc;
-            }
-        } else {
-#pragma unroll
-            for (int b = 0; b < RB; ++b) {
-                double acc = 0.0;
-                if (t0 + b < M.n_tb)
-                    for (int i = rl; i < nS; i += LW) acc += ldg(M.eff + (size_t)(t0 + b) * nS + i) * w[c_off + i];
-                sum[b] = acc;
-            }
+    const int n = M.n_tb;
+    for (int t = g.lane; t < n; t += G) {
+        const double* e = M.effT + t;
+        double s0 = 0.0, s1 = 0.0;
+        int i = 0;
+#pragma unroll 4
+        for (; i + 1 < M.nS; i += 2) {
+            s0 = fma(ldg(e + (size_t)i * n), w[c_off + i], s0);
+            s1 = fma(ldg(e + (size_t)(i + 1) * n), w[c_off + i + 1], s1);
         }
-#pragma unroll
-        for (int b = 0; b < RB; ++b) {
-#pragma unroll
-            for (int o = LW / 2; o > 0; o >>= 1) sum[b] += __shfl_xor_sync(mask, sum[b], o, LW);
-            if (rl == 0 && t0 + b < M.n_tb) w[m_off + t0 + b] = sum[b];
-        }
+        if (i < M.nS) s0 = fma(ldg(e + (size_t)i * n), w[c_off + i], s0);
+        w[m_off + t] = s0 + s1;
     }
 }
 
@@ -652,9 +611,9 @@ __host__ __device__ inline WsLayout make_layout(int nS, int nR, int n_slots, int
         L.vj = L.k3;
         L.rhoMbyW = L.k4;
     }
-    L.stage = o; o += (n_slots > 0 ? n_slots : 1);
+    L.stage = o; o += n_slots + 1;  // and a 0 for the gathers' missing records
+    L.part = L.k3;                  // k3, k4: no stage has written them when f is assembled
     L.Mtb = o; o += (n_tb > 0 ? n_tb : 1);
-    L.scal = o; o += 8;
     L.size = o;
     return L;
 }
@@ -748,33 +707,41 @@ __host__ __device__ constexpr int log2_group(int G) { return G <= 1 ? 0 : 1 + lo
 __host__ __device__ constexpr int stream_index(int G) { return G == 96 ? 9 : log2_group(G); }
 
 // Runs this thread's share of a gather stream (gf_internal.h, Stream):
-// dst[pos] = sum of coef * src[slot] over each entry's records, in order.
-// Every record load is independent of the sums (coalesced 16-byte loads), so
-// they pipeline; one thread owns each output entry (no barriers inside).
-template <int G, class W>
-__device__ __forceinline__ void stream_gather(const Grp<G>& g, const Stream& st, const W& w, int src, int dst) {
-    constexpr int U = GF_GATHER_BATCH;  // records in flight per thread
-    const int4* r = reinterpret_cast<const int4*>(st.rec) + g.lane;
-    const int len = st.len;
+// wd[dst + pos] = sum of coef * ws[src + slot] over each entry's records, in
+// order. The group's loads (48 coalesced bytes and the position) are
+// independent of the sums, so they pipeline; one thread owns each output entry
+// (no barriers inside). Bound by instructions: 20 per four records, where
+// 16-byte records that each carried a position took 12 per record.
+template <int G, class WS, class WD>
+__device__ __forceinline__ void stream_gather(const Grp<G>& g, const Stream& st, const WS& ws, int src, const WD& wd,
+                                              int dst) {
+    const int4* o = reinterpret_cast<const int4*>(st.off) + g.lane;
+    const double2* c = reinterpret_cast<const double2*>(st.coef) + g.lane;
+    const int* p = st.pos + g.lane;
     double acc = 0.0;
-    for (int k0 = 0; k0 < len; k0 += U) {
-        int4 v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = (k0 + u < len) ? __ldg(r + (size_t)(k0 + u) * G) : make_int4(-1, -1, 0, 0);
-        // the sources of the batch are read before any of its results is
-        // stored (the source and destination regions are disjoint)
-        double x[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) x[u] = v[u].y >= 0 ? w[src + v[u].y] : 0.0;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (v[u].y >= 0) acc += __hiloint2double(v[u].w, v[u].z) * x[u];
-            if (v[u].x >= 0) {
-                w[dst + v[u].x] = acc;
-                acc = 0.0;
-            }
+#pragma unroll 2
+    for (int k = 0; k < st.len; ++k) {
+        const int4 v = __ldg(o + (size_t)k * G);
+        const double2 a = __ldg(c + (size_t)k * 2 * G), b = __ldg(c + (size_t)k * 2 * G + G);
+        const int pos = __ldg(p + (size_t)k * G);
+        acc = fma(a.x, ws.at(src, v.x), acc);
+        acc = fma(a.y, ws.at(src, v.y), acc);
+        acc = fma(b.x, ws.at(src, v.z), acc);
+        acc = fma(b.y, ws.at(src, v.w), acc);
+        if (pos >= 0) {
+            wd[dst + pos] = acc;
+            acc = 0.0;
         }
     }
+}
+
+// The sum of a species' parts in the dN/dt gather.
+template <class W>
+__device__ __forceinline__ double part_sum(const W& w, int at, const int* part, int s) {
+    const int e = ldg(part + s + 1);
+    double acc = 0.0;
+    for (int i = ldg(part + s); i < e; ++i) acc += w[at + i];
+    return acc;
 }
 
 // dN_s/dt gathered in the reference's order, scaled to dY/dt (gpuODESystem.H:40-48,
@@ -783,11 +750,12 @@ template <int G, class W>
 __device__ __forceinline__ void gather_rhs(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
                                            int out_off, const Mix& x) {
     const int nS = M.nS;
-    stream_gather(g, M.dst[stream_index(G)], w, L.stage, out_off);
+    stream_gather(g, M.dst[stream_index(G)], w, L.stage, w, L.part);
     g.sync();
+    const int* part = M.dst_part[stream_index(G)];
     double s_h = 0;
     for (int s = g.lane; s < nS; s += G) {
-        const double acc = w[out_off + s] * (ldg(M.W + s) * x.irho);
+        const double acc = part_sum(w, L.part, part, s) * (ldg(M.W + s) * x.irho);
         w[out_off + s] = acc;
         s_h += acc * w[L.Ha + s];
     }
@@ -897,7 +865,7 @@ __device__ __forceinline__ void jacobian(const Grp<G>& g, const DevMech& M, cons
     GF_PH_BEGIN(g)
     // raw dN/dc, T-column and third-body terms of every entry (species rows x
     // species and T columns), one thread per entry, in the reference's order
-    stream_gather(g, M.jst[stream_index(G)], w, L.stage, L.J);
+    stream_gather(g, M.jst[stream_index(G)], w, L.stage, w, L.J);
     g.sync();
     // phase 3
     for (int s = g.lane; s < nS; s += G) {
@@ -1963,6 +1931,7 @@ __device__ __forceinline__ void process_cell_body(const Grp<G>& g, const DevMech
     const double T0 = yin[nS];
     const double dT = a.deltaT_cell ? a.deltaT_cell[cell] : a.deltaT;
     double dxTry = a.deltaTChem[cell];
+    if (g.lane == 0) w[L.stage + M.n_slots] = 0.0;
     int status = GF_CELL_OK, accepted = 0, attempts = 0;
     g.sync();
     if (T0 > a.Treact) {

@@ -39,7 +39,9 @@ __host__ __device__ inline FieldLayout field_layout(const DevMech& M) {
     F.L.Mtb = o;
     o += M.n_tb > 0 ? M.n_tb : 1;
     F.L.stage = o;
-    o += M.n_slots > 0 ? M.n_slots : 1;
+    o += M.n_slots + 1;  // and a 0 for the gather's missing records
+    F.L.part = o;
+    o += 2 * M.m;
     F.out = o;
     o += M.nS;
     F.size = o;
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
     const int warp = threadIdx.x >> 5;
     WsC w{smem + (size_t)warp * F.size};
     const int nS = M.nS;
+    if (g.lane == 0) w[F.L.stage + M.n_slots] = 0.0;
     for (long long cell = (long long)blockIdx.x * per_cta + warp; cell < a.n_cells;
          cell += (long long)gridDim.x * per_cta) {
         const double* y = a.y + cell * a.ld_y;
@@ -139,10 +142,11 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
         stage_fields(g, M, w, F.L, tcache, a.tc != nullptr, &sW, &sW2);
         g.sync();
         if (a.RR) {
-            stream_gather(g, M.dst[stream_index(32)], w, F.L.stage, F.out);
+            stream_gather(g, M.dst[stream_index(32)], w, F.L.stage, w, F.L.part);
             g.sync();
+            const int* part = M.dst_part[stream_index(32)];
             double* rr = a.RR + cell * a.ld_rr;
-            for (int i = g.lane; i < nS; i += 32) rr[i] = w[F.out + i] * ldg(M.W + i);
+            for (int i = g.lane; i < nS; i += 32) rr[i] = part_sum(w, F.L.part, part, i) * ldg(M.W + i);
         }
         if (a.tc) {
             const double sumW = g.sum(sW), sumW2 = g.sum(sW2), ctot = g.sum(csum);

@@ -103,45 +103,81 @@ struct DevBuf {
     }
 };
 
-// Gather streams (gf::Stream): entries with their (slot, coef) records in
-// summation order, split over G threads so that the record counts balance
-// (greedy, largest entry first), each thread's entries in ascending order,
-// interleaved record k of thread t at k * G + t, padded to the longest thread.
-// An entry without records still gets one (it writes zero).
-std::vector<gf::StreamRec> build_stream(const std::vector<std::vector<std::pair<int, double>>>& entries,
-                                        const std::vector<int>& pos, int G, int* len_out) {
+// One entry of a gather: its (slot, coefficient) records in summation order.
+using Records = std::vector<std::pair<int, double>>;
+
+struct StreamTables {
+    std::vector<int> off, pos;
+    std::vector<double> coef;
+    int len = 0;
+};
+
+// Gather streams (gf::Stream): the entries split over G threads so that their
+// groups of four records balance (greedy, largest entry first), each thread's
+// entries in ascending order. An entry without records still gets a group (it
+// writes zero); zero_slot holds 0.
+StreamTables build_stream(const std::vector<Records>& entries, const std::vector<int>& pos, int zero_slot, int G) {
     const int nE = (int)entries.size();
+    auto groups = [&](int e) { return std::max<int>(1, ((int)entries[e].size() + 3) / 4); };
     std::vector<int> order(nE);
     for (int e = 0; e < nE; ++e) order[e] = e;
-    auto cnt = [&](int e) { return std::max<int>(1, (int)entries[e].size()); };
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cnt(a) > cnt(b); });
-    std::vector<long long> load(G, 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return groups(a) > groups(b); });
+    // threads by load, the lowest index first among equals
+    std::vector<std::pair<int, int>> heap(G);
+    for (int t = 0; t < G; ++t) heap[t] = {0, t};
+    auto after = [](const std::pair<int, int>& a, const std::pair<int, int>& b) { return a > b; };
     std::vector<std::vector<int>> owned(G);
+    StreamTables T;
     for (int e : order) {
-        int t = 0;
-        for (int u = 1; u < G; ++u)
-            if (load[u] < load[t]) t = u;
-        load[t] += cnt(e);
-        owned[t].push_back(e);
+        std::pop_heap(heap.begin(), heap.end(), after);
+        auto& h = heap.back();
+        owned[h.second].push_back(e);
+        h.first += groups(e);
+        T.len = std::max(T.len, h.first);
+        std::push_heap(heap.begin(), heap.end(), after);
     }
-    int len = 0;
-    for (int t = 0; t < G; ++t) len = std::max<int>(len, (int)load[t]);
-    std::vector<gf::StreamRec> rec((size_t)std::max(len, 1) * G, gf::StreamRec{-1, -1, 0.0});
+    const size_t n = (size_t)std::max(T.len, 1) * G;
+    T.off.assign(4 * n, zero_slot * (int)sizeof(double));
+    T.coef.assign(4 * n, 0.0);
+    T.pos.assign(n, -1);
     for (int t = 0; t < G; ++t) {
         std::sort(owned[t].begin(), owned[t].end());
-        int k = 0;
+        size_t k = 0;
         for (int e : owned[t]) {
-            const auto& R = entries[e];
-            if (R.empty()) {
-                rec[(size_t)k++ * G + t] = gf::StreamRec{pos[e], -1, 0.0};
-                continue;
+            const Records& R = entries[e];
+            for (int q = 0; q < groups(e); ++q, ++k) {
+                const size_t at = k * G + t;
+                for (size_t i = 0; i < 4 && 4 * (size_t)q + i < R.size(); ++i) {
+                    T.off[4 * at + i] = R[4 * q + i].first * (int)sizeof(double);
+                    T.coef[2 * (2 * k * G + (i / 2) * G + t) + i % 2] = R[4 * q + i].second;
+                }
+                if (q + 1 == groups(e)) T.pos[at] = pos[e];
             }
-            for (size_t i = 0; i < R.size(); ++i)
-                rec[(size_t)k++ * G + t] = gf::StreamRec{i + 1 == R.size() ? pos[e] : -1, R[i].first, R[i].second};
         }
     }
-    *len_out = len;
-    return rec;
+    return T;
+}
+
+// The parts of the dN/dt gather: each entry cut into runs of records, the
+// shortest (a multiple of four) that leave at most `most` parts in all.
+// first[e] .. first[e + 1]: the parts of entry e.
+std::vector<Records> cut_entries(const std::vector<Records>& entries, int most, std::vector<int>* first) {
+    size_t longest = 4;
+    for (const Records& r : entries) longest = std::max(longest, r.size());
+    size_t cap = 4;
+    for (; cap < longest; cap += 4) {
+        size_t n = 0;
+        for (const Records& r : entries) n += std::max<size_t>(1, (r.size() + cap - 1) / cap);
+        if (n <= (size_t)most) break;
+    }
+    std::vector<Records> parts;
+    first->assign(1, 0);
+    for (const Records& r : entries) {
+        for (size_t o = 0; o == 0 || o < r.size(); o += cap)
+            parts.emplace_back(r.begin() + std::min(o, r.size()), r.begin() + std::min(o + cap, r.size()));
+        first->push_back((int)parts.size());
+    }
+    return parts;
 }
 
 }  // namespace
@@ -404,9 +440,9 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
     }
     const int n_slots = slot[nR];
     // per-species terms, built over reactions in mechanism order r
-    std::vector<std::vector<std::pair<int, double>>> dn(nS);
+    std::vector<Records> dn(nS);
     const int nE = nS * (nS + 1);  // raw-Jacobian entries: species rows x (species + T) columns
-    std::vector<std::vector<std::pair<int, double>>> je(nE);
+    std::vector<Records> je(nE);
     for (int r = 0; r < nR; ++r) {
         const gf_reaction& x = d->reactions[r];
         const int so = slot[rof[r]];
@@ -513,7 +549,7 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
     for (int s2 = 0; s2 < nS; ++s2) dn_pos[s2] = s2;
     for (int e = 0; e < nE; ++e) je_pos[e] = (e / (nS + 1)) * ldJ + e % (nS + 1);
     // concentration gathers of the adjoint: species s <- entry slots of its occurrences
-    std::vector<std::vector<std::pair<int, double>>> cg(nS);
+    std::vector<Records> cg(nS);
     int max_side = 0;
     for (int q = 0; q < nR; ++q) {
         max_side = std::max(max_side, std::max(nl[q], nr[q]));
@@ -524,15 +560,26 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
                 cg[sidx[b + e]].push_back({q * 2 * kSideInline + side * kSideInline + e, 1.0});
         }
     }
-    std::vector<std::vector<StreamRec>> dst_rec(kNumGroupSizes), jst_rec(kNumGroupSizes), cst_rec(kNumGroupSizes);
-    int dst_len[kNumGroupSizes], jst_len[kNumGroupSizes], cst_len[kNumGroupSizes];
+    std::vector<StreamTables> dst_t, jst_t, cst_t;
+    std::vector<std::vector<int>> dst_part(kNumGroupSizes);
     for (int k = 0; k < kNumGroupSizes; ++k) {
-        dst_rec[k] = build_stream(dn, dn_pos, group_size_of(k), &dst_len[k]);
-        jst_rec[k] = build_stream(je, je_pos, group_size_of(k), &jst_len[k]);
-        cst_rec[k] = build_stream(cg, dn_pos, group_size_of(k), &cst_len[k]);
+        const int G = group_size_of(k);
+        // as many parts as threads keep the group busy; a workspace has room for 2 m
+        const std::vector<Records> parts = cut_entries(dn, std::max(nS, std::min(G, 2 * (nS + 1))), &dst_part[k]);
+        std::vector<int> part_pos(parts.size());
+        for (size_t i = 0; i < parts.size(); ++i) part_pos[i] = (int)i;
+        dst_t.push_back(build_stream(parts, part_pos, n_slots, G));
+        jst_t.push_back(build_stream(je, je_pos, n_slots, G));
+        cst_t.push_back(build_stream(cg, dn_pos, 2 * kSideInline * nRa, G));
     }
+    std::vector<double> effT(eff.size());
+    for (int t = 0; t < n_tb; ++t)
+        for (int i = 0; i < nS; ++i) effT[(size_t)i * n_tb + t] = eff[(size_t)t * nS + i];
     // keep every array non-empty
-    if (eff.empty()) eff.push_back(0.0);
+    if (eff.empty()) {
+        eff.push_back(0.0);
+        effT.push_back(0.0);
+    }
     if (sidx.empty()) {
         sidx.push_back(0);
         siexp.push_back(0);
@@ -544,15 +591,17 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
     // would send a kernel outside its arrays is refused here, not found on the GPU
     {
         const int m = nS + 1;
-        auto stream_ok = [](const std::vector<StreamRec>& rec, int n_pos, int n_src) {
-            for (const StreamRec& r : rec)
-                if (r.pos >= n_pos || r.slot >= n_src) return false;
+        auto stream_ok = [](const StreamTables& t, int n_pos, int n_src) {
+            for (int p : t.pos)
+                if (p >= n_pos) return false;
+            for (int o : t.off)
+                if (o < 0 || o / (int)sizeof(double) > n_src) return false;  // n_src: the zero
             return true;
         };
         const int n_conc_slots = 2 * kSideInline * nRa;
         for (int k = 0; k < kNumGroupSizes; ++k)
-            if (!stream_ok(dst_rec[k], nS, n_slots) || !stream_ok(jst_rec[k], m * ldJ, n_slots) ||
-                !stream_ok(cst_rec[k], nS, n_conc_slots))
+            if (!stream_ok(dst_t[k], 2 * m, n_slots) || dst_part[k].back() > 2 * m ||
+                !stream_ok(jst_t[k], m * ldJ, n_slots) || !stream_ok(cst_t[k], nS, n_conc_slots))
                 return GF_ERR_UNSUPPORTED;
         for (int q = 0; q < nR; ++q) {
             const int need = std::max(4, 2 + nl[q] + nr[q] + (rtype[q] == GF_RATE_THIRD_BODY_ARRHENIUS ? 1 : 0));
@@ -575,11 +624,18 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
                  oLA1 = b.add(lnA1), oSA1 = b.add(sA1), oB1 = b.add(beta1), oT1 = b.add(Ta1), oTroe = b.add(troe),
                  oTb = b.add(tb_row), oEff = b.add(eff), oSi = b.add(sidx), oSie = b.add(siexp), oSst = b.add(sst),
                  oSe = b.add(sexp), oRxh = b.add(rxh), oRxs = b.add(rxs), oRxf = b.add(rxf), oLnk = b.add(lnk), oRofq = b.add(qof);
-    size_t oDst[kNumGroupSizes], oJst[kNumGroupSizes], oCst[kNumGroupSizes];
+    const size_t oEffT = b.add(effT);
+    struct StreamAt {
+        size_t off, coef, pos;
+    };
+    auto add_stream = [&b](const StreamTables& t) { return StreamAt{b.add(t.off), b.add(t.coef), b.add(t.pos)}; };
+    StreamAt oDst[kNumGroupSizes], oJst[kNumGroupSizes], oCst[kNumGroupSizes];
+    size_t oPart[kNumGroupSizes];
     for (int k = 0; k < kNumGroupSizes; ++k) {
-        oDst[k] = b.add(dst_rec[k]);
-        oJst[k] = b.add(jst_rec[k]);
-        oCst[k] = b.add(cst_rec[k]);
+        oDst[k] = add_stream(dst_t[k]);
+        oJst[k] = add_stream(jst_t[k]);
+        oCst[k] = add_stream(cst_t[k]);
+        oPart[k] = b.add(dst_part[k]);
     }
     gf_mech* m = new (std::nothrow) gf_mech;
     if (!m) return GF_ERR_OUT_OF_MEMORY;
@@ -635,6 +691,7 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
     D.troe = (const double*)P(oTroe);
     D.tb_row = (const int*)P(oTb);
     D.eff = (const double*)P(oEff);
+    D.effT = (const double*)P(oEffT);
     D.r_of_q = (const int*)P(oRofq);
     D.rxh = (const RxnHead*)P(oRxh);
     D.rxs = (const RxnSpecie*)P(oRxs);
@@ -646,9 +703,13 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
     D.sst = (const double*)P(oSst);
     D.sexp = (const double*)P(oSe);
     for (int k = 0; k < kNumGroupSizes; ++k) {
-        D.dst[k] = Stream{(const StreamRec*)P(oDst[k]), dst_len[k]};
-        D.jst[k] = Stream{(const StreamRec*)P(oJst[k]), jst_len[k]};
-        D.cst[k] = Stream{(const StreamRec*)P(oCst[k]), cst_len[k]};
+        auto stream = [&](const StreamAt& a, int len) {
+            return Stream{(const int*)P(a.off), (const double*)P(a.coef), (const int*)P(a.pos), len};
+        };
+        D.dst[k] = stream(oDst[k], dst_t[k].len);
+        D.jst[k] = stream(oJst[k], jst_t[k].len);
+        D.cst[k] = stream(oCst[k], cst_t[k].len);
+        D.dst_part[k] = (const int*)P(oPart[k]);
     }
     D.max_side = max_side;
     m->q_of_r.assign(rof.begin(), rof.begin() + nR);

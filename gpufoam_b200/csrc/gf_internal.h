@@ -44,21 +44,19 @@ struct __align__(16) RxnFast {
     double lnA0, beta0, Ta0, nm;  // nm: 0 where Kc = K (gpuThermo.H:111)
 };
 
-// One record of a gather stream: acc += coef * src[slot] (slot < 0: nothing);
-// pos >= 0 marks the last record of an output entry: dst[pos] = acc, acc = 0.
-struct __align__(16) StreamRec {
-    int pos;
-    int slot;
-    double coef;
-};
-
-// The records of a gather y[pos] = sum coef * x[slot], entry by entry in the
-// reference's summation order, split over G threads (entries balanced by
-// record count) and interleaved: record k of thread t is rec[k * G + t], so
-// a warp's loads are coalesced and every load is independent of the sums.
+// A gather y[pos] = sum coef * x[slot], entry by entry in the reference's
+// summation order, split over G threads (entries balanced by their groups of
+// four records) and interleaved: group k of thread t is off[k * G + t] (the
+// slots' byte offsets; a missing record has coefficient 0 and the offset of a
+// slot that holds 0), coef[2 (k * G) + t] and coef[2 (k * G) + G + t] (two
+// coefficients each) and pos[k * G + t]: >= 0 on the last group of an output
+// entry (dst[pos] = sum), else -1. A warp's loads are coalesced, and every load
+// is independent of the sums.
 struct Stream {
-    const StreamRec* rec;
-    int len;  // records per thread (padded)
+    const int* off;      // int4 per group
+    const double* coef;  // two double2 per group
+    const int* pos;
+    int len;  // groups per thread (padded)
 };
 constexpr int kNumGroupSizes = 10;  // G = 1, 2, 4, ..., 256: stream index log2(G); G = 96: index 9
 constexpr int group_size_of(int k) { return k < 9 ? 1 << k : 96; }
@@ -80,8 +78,11 @@ constexpr int group_size_of(int k) { return k < 9 ? 1 << k : 96; }
 //  * staging slots of reaction q start at slot[q]:
 //      [0] omega, [1] dwdT, [2 .. 2+nl) dCf*kf, [2+nl .. 2+nl+nr) dCr*kr,
 //      third body only: [2+nl+nr] Ak * (Cf - Cr/Kc)
+//    and behind the last reaction's a slot that holds 0
 //  * dst[log2 G]: the gather streams of dN_s/dt: per species s the (omega slot,
-//    signed stoich) terms in mechanism order (gpuReaction.H:490-508)
+//    signed stoich) terms in mechanism order (gpuReaction.H:490-508), cut into
+//    parts so that the species of many reactions do not keep one thread busy
+//    while the others wait; dst_part[log2 G][s] .. [s + 1]: its parts
 //  * jst[log2 G]: the gather streams of the raw Jacobian: entry (row s,
 //    column c < nS or the T column c = nS), position s * ld + c in the
 //    workspace Jacobian, takes its dN/dc, T-column and third-body terms in the
@@ -124,6 +125,7 @@ struct DevMech {
     const double* troe;        // [nR][4]: alpha, 1/Tsss, 1/Ts, Tss
     const int* tb_row;         // [nR] row of eff, -1 for plain Arrhenius
     const double* eff;         // [n_tb][nS]
+    const double* effT;        // [nS][n_tb]
     const int* r_of_q;         // [nR] mechanism index of the reaction in compute position q
     const RxnHead* rxh;        // [nR]
     const RxnFast* rxf;        // [nR]
@@ -135,6 +137,7 @@ struct DevMech {
     const double* sst;
     const double* sexp;
     Stream dst[kNumGroupSizes];
+    const int* dst_part[kNumGroupSizes];
     Stream jst[kNumGroupSizes];
     // the adjoint's concentration gathers: per species s, the per-reaction
     // entry slots q * 2 * kSideInline + e whose species is s
@@ -152,7 +155,8 @@ struct OdeParams {
 // Per-cell workspace layout (in doubles) for a mechanism.
 struct WsLayout {
     int ld;          // Jacobian / LU row stride (odd, bank-conflict free columns)
-    int J, y0, yt, dydx0, dydx, dfdx, k1, k2, k3, k4, c, Cp, Ha, rhoMbyW, vj, vv, piv, perm, stage, Mtb, scal;
+    int J, y0, yt, dydx0, dydx, dfdx, k1, k2, k3, k4, c, Cp, Ha, rhoMbyW, vj, vv, piv, perm, stage, Mtb;
+    int part;        // partial sums of dN/dt, 2 m doubles that are free while f is assembled
     int size;        // total doubles
 };
 

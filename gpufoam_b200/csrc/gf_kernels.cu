@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(32) rates_kernel(const DevMech M, const double
     const double* yi = y + (size_t)blockIdx.x * n;
     WsC w{smem};
     for (int i = g.lane; i < M.m; i += 32) w[L.y0 + i] = yi[i];
+    if (g.lane == 0) w[L.stage + M.n_slots] = 0.0;
     const double p = yi[M.nS + 1];
     derivatives(g, M, w, L, L.y0, p, L.dydx);
     double* o = dydx + (size_t)blockIdx.x * n;
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(32) jacobian_kernel(const DevMech M, const dou
     const double* yi = y + (size_t)blockIdx.x * n;
     WsC w{smem};
     for (int i = g.lane; i < M.m; i += 32) w[L.y0 + i] = yi[i];
+    if (g.lane == 0) w[L.stage + M.n_slots] = 0.0;
     const double p = yi[M.nS + 1];
     derivatives(g, M, w, L, L.y0, p, L.dydx, true);  // leaves the rate constants for the Jacobian
     jacobian(g, M, w, L, L.y0, p);
