@@ -110,9 +110,8 @@ struct AdjArgs {
 // (forward substitution), L^T v = z (backward, unit diagonal), x[perm[i]] =
 // v[i]. One warp, R rows per lane (lane l holds rows l + 32 u), column by
 // column with the pivot value broadcast by a shuffle; the entries used at
-// step j are row j of the factors (contiguous; BY_PERM: at row perm[j] of the
-// workspace, lu_decompose_mma). m <= 32 R.
-template <int R, bool BY_PERM, class W>
+// step j are row j of the factors (contiguous). m <= 32 R.
+template <int R, class W>
 __device__ void lu_solve_transposed_warp(const W& w, const WsC& wa, int A, int ld, int perm, int m, int b, int x) {
     const int lane = threadIdx.x & 31;
     double z[R];
@@ -124,7 +123,7 @@ __device__ void lu_solve_transposed_warp(const W& w, const WsC& wa, int A, int l
     // U^T z = b: z_j = b_j / U[j][j], then b_i -= U[j][i] z_j for i > j
     for (int j = 0; j < m; ++j) {
         const int t = j >> 5, l = j & 31;
-        const int row = A + (BY_PERM ? w.ip(perm + j) : j) * ld;
+        const int row = A + j * ld;
         double zt = z[0];
 #pragma unroll
         for (int u = 1; u < R; ++u)
@@ -140,7 +139,7 @@ __device__ void lu_solve_transposed_warp(const W& w, const WsC& wa, int A, int l
     // L^T v = z: v_j final, then z_i -= L[j][i] v_j for i < j (descending j)
     for (int j = m - 1; j >= 0; --j) {
         const int t = j >> 5, l = j & 31;
-        const int row = A + (BY_PERM ? w.ip(perm + j) : j) * ld;
+        const int row = A + j * ld;
         double zt = z[0];
 #pragma unroll
         for (int u = 1; u < R; ++u)
@@ -165,11 +164,11 @@ __device__ void lu_solve_transposed(const Grp<G>& g, const W& w, const WsC& wa, 
     g.sync();
     if (threadIdx.x < 32) {
         if (m <= 64)
-            lu_solve_transposed_warp<2, true>(w, wa, A, ld, perm, m, b, x);
+            lu_solve_transposed_warp<2>(w, wa, A, ld, perm, m, b, x);
         else if (m <= 128)
-            lu_solve_transposed_warp<4, true>(w, wa, A, ld, perm, m, b, x);
+            lu_solve_transposed_warp<4>(w, wa, A, ld, perm, m, b, x);
         else
-            lu_solve_transposed_warp<10, false>(w, wa, A, ld, perm, m, b, x);
+            lu_solve_transposed_warp<10>(w, wa, A, ld, perm, m, b, x);
     }
     g.sync();
 }

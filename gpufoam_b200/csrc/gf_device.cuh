@@ -1196,8 +1196,8 @@ __device__ __forceinline__ void lu_panel_reg(const W& w, int A, int ld, int piv,
 // updates with lanes over columns; the trailing matrix is updated in 8 x 8
 // tiles by the FP64 matrix instruction, the tiles shared out to the warps in
 // runs along a tile row (the run keeps its part of L in registers). Rows are
-// never exchanged: position i of the reference's matrix is row perm[i], and the
-// solves follow perm. Every entry receives its updates in k order, as in
+// not exchanged meanwhile: position i of the reference's matrix is row perm[i];
+// one pass at the end puts them in order. Every entry receives its updates in k order, as in
 // lu_decompose, so factors and pivots are the same bit for bit (EXACT: scalar
 // updates with two roundings). sc: the row scalings; rd: out, 1 / U[i][i].
 //
@@ -1288,6 +1288,30 @@ __device__ __forceinline__ void lu_decompose_mma(const Grp<G>& g, const W& w, in
         }
         g.sync();
         GF_PH_END(g, PH_LU_TRAIL)
+    }
+    // rows to their positions, a few columns of a warp at a time
+    {
+        GF_PH_BEGIN(g)
+        constexpr int CB = 4;
+        int from[RP];
+#pragma unroll
+        for (int r = 0; r < RP; ++r) from[r] = l + 32 * r < m ? A + w.ip(perm + l + 32 * r) * ld : A;
+        for (int j0 = wid * CB; j0 < m; j0 += NW * CB) {
+            double v[RP][CB];
+#pragma unroll
+            for (int r = 0; r < RP; ++r)
+#pragma unroll
+                for (int c = 0; c < CB; ++c) v[r][c] = j0 + c < m ? w[from[r] + j0 + c] : 0.0;
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < RP; ++r)
+#pragma unroll
+                for (int c = 0; c < CB; ++c)
+                    if (l + 32 * r < m && j0 + c < m) w[A + (l + 32 * r) * ld + j0 + c] = v[r][c];
+            __syncwarp();
+        }
+        g.sync();
+        GF_PH_END(g, PH_LU_PERM)
     }
 }
 
@@ -1512,65 +1536,112 @@ __device__ __forceinline__ void lu_solve_reg(const Grp<G>& g, const W& w, int A,
     GF_PH_END(g, PH_SOLVE)
 }
 
-// Register form for one full warp with R rows per lane (m <= 32 R): lane l
-// holds rows l + 32 u (row perm[i] of the factors at position i,
-// lu_decompose_mma). The steps run in tiles of 32, the step loop unrolled by
-// kSolveUnroll (4: measured faster than 8, 16 and full unrolling, whose code
-// costs more in instruction fetch inside the solve kernel than it saves), so
-// the loads of later steps can be issued early (the loop stores nothing).
-// Same operations and order as lu_solve_reg.
 #ifndef GF_SOLVE_UNROLL
-#define GF_SOLVE_UNROLL 4
+#define GF_SOLVE_UNROLL 2
 #endif
-constexpr int kSolveUnroll = GF_SOLVE_UNROLL;  // substitution steps unrolled together
+constexpr int kSolveUnroll = GF_SOLVE_UNROLL;  // blocks of columns unrolled together
+// Register form for one full warp with R rows per lane (m <= 32 R): lane l
+// holds rows l + 32 u. Columns go in blocks of four: the block's four values
+// are fetched with shuffles that do not wait for one another, every lane
+// eliminates inside the block by itself (the six factors are at one address for
+// all lanes), and then applies the four columns to its rows; columns that fill
+// no block go one by one. Same operations and order per row as column by column
+// (lu_solve_reg). Bound by the chain of dependent operations of one warp, then
+// by its instructions: rows past m read row 0 and are never stored, so that the
+// loops carry no predicate for them.
 template <int R, class W>
 __device__ __forceinline__ void lu_solve_warp(const W& w, int A, int ld, int perm, int rdiag, int m, int b) {
     const int lane = threadIdx.x & 31;
     double x[R];
-    int ro[R];  // the row of the factors at position 32 u + lane
-    bool in[R];
+    int ro[R];
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < R; ++u) {
         const int i = u * 32 + lane;
-        in[u] = i < m;
-        const int pi = in[u] ? w.ip(perm + i) : 0;
-        ro[u] = A + pi * ld;
-        x[u] = in[u] ? w[b + pi] : 0.0;
+        ro[u] = i < m ? A + i * ld : A;
+        x[u] = i < m ? w[b + w.ip(perm + i)] : 0.0;
     }
-    // forward substitution with the unit lower factor, column by column
+    // forward substitution with the unit lower factor: columns 0 .. m-2
 #pragma unroll
     for (int t = 0; t < R; ++t) {
-        if (32 * t >= m - 1) break;
+        const int n = min(32, m - 1 - 32 * t);  // columns of this tile
+        int l0 = 0;
 #pragma unroll kSolveUnroll
-        for (int l = 0; l < 32; ++l) {
-            const int j = 32 * t + l;
-            if (j >= m - 1) break;
-            const double bj = __shfl_sync(0xffffffffu, x[t], l);
-            if (lane > l && in[t]) x[t] -= w[ro[t] + j] * bj;
+        for (; l0 + 4 <= n; l0 += 4) {
+            const int j0 = 32 * t + l0, rb = A + j0 * ld + j0, d = lane - l0;
+            double y[4];
 #pragma unroll
-            for (int u = t + 1; u < R; ++u)
-                if (in[u]) x[u] -= w[ro[u] + j] * bj;
+            for (int i = 0; i < 4; ++i) y[i] = __shfl_sync(0xffffffffu, x[t], l0 + i);
+            const double l10 = w[rb + ld], l20 = w[rb + 2 * ld], l21 = w[rb + 2 * ld + 1], l30 = w[rb + 3 * ld],
+                         l31 = w[rb + 3 * ld + 1], l32 = w[rb + 3 * ld + 2];
+            y[1] -= l10 * y[0];
+            y[2] -= l20 * y[0];
+            y[3] -= l30 * y[0];
+            y[2] -= l21 * y[1];
+            y[3] -= l31 * y[1];
+            y[3] -= l32 * y[2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double f = w[ro[t] + j0 + k];
+                if (d > k) x[t] -= f * y[k];
+#pragma unroll
+                for (int u = t + 1; u < R; ++u) x[u] -= w[ro[u] + j0 + k] * y[k];
+            }
+        }
+#pragma unroll 1
+        for (; l0 < n; ++l0) {
+            const int j = 32 * t + l0;
+            const double bj = __shfl_sync(0xffffffffu, x[t], l0);
+            if (lane > l0) x[t] -= w[ro[t] + j] * bj;
+#pragma unroll
+            for (int u = t + 1; u < R; ++u) x[u] -= w[ro[u] + j] * bj;
         }
     }
     // backward substitution, descending columns, x_j = (...) * (1 / U[j][j])
 #pragma unroll
     for (int t = R - 1; t >= 0; --t) {
-        if (32 * t >= m) continue;
-#pragma unroll kSolveUnroll
-        for (int l = 31; l >= 0; --l) {
-            const int j = 32 * t + l;
-            if (j >= m) continue;
-            const double xj = __shfl_sync(0xffffffffu, x[t], l) * w[rdiag + j];
-            if (lane == l) x[t] = xj;
-            if (lane < l) x[t] -= w[ro[t] + j] * xj;
+        int n = min(32, m - 32 * t);
+#pragma unroll 1
+        for (; n > 0 && (n & 3); --n) {
+            const int l0 = n - 1, j = 32 * t + l0;
+            const double xj = __shfl_sync(0xffffffffu, x[t], l0) * w[rdiag + j];
+            const double f = w[ro[t] + j];
+            if (lane < l0) x[t] -= f * xj;
+            if (lane == l0) x[t] = xj;
 #pragma unroll
             for (int u = 0; u < t; ++u) x[u] -= w[ro[u] + j] * xj;
+        }
+#pragma unroll kSolveUnroll
+        for (int l0 = n - 4; l0 >= 0; l0 -= 4) {
+            const int j0 = 32 * t + l0, rb = A + j0 * ld + j0, d = lane - l0;
+            double y[4];
+#pragma unroll
+            for (int i = 3; i >= 0; --i) y[i] = __shfl_sync(0xffffffffu, x[t], l0 + i);
+            const double u01 = w[rb + 1], u02 = w[rb + 2], u03 = w[rb + 3], u12 = w[rb + ld + 2], u13 = w[rb + ld + 3],
+                         u23 = w[rb + 2 * ld + 3];
+            y[3] *= w[rdiag + j0 + 3];
+            y[2] -= u23 * y[3];
+            y[1] -= u13 * y[3];
+            y[0] -= u03 * y[3];
+            y[2] *= w[rdiag + j0 + 2];
+            y[1] -= u12 * y[2];
+            y[0] -= u02 * y[2];
+            y[1] *= w[rdiag + j0 + 1];
+            y[0] -= u01 * y[1];
+            y[0] *= w[rdiag + j0];
+#pragma unroll
+            for (int k = 3; k >= 0; --k) {
+                const double f = w[ro[t] + j0 + k];
+                if (d < k) x[t] -= f * y[k];
+                if (d == k) x[t] = y[k];
+#pragma unroll
+                for (int u = 0; u < t; ++u) x[u] -= w[ro[u] + j0 + k] * y[k];
+            }
         }
     }
 #pragma unroll
     for (int u = 0; u < R; ++u)
-        if (in[u]) w[b + 32 * u + lane] = x[u];
+        if (u * 32 + lane < m) w[b + 32 * u + lane] = x[u];
     __syncwarp();
 }
 
@@ -1607,8 +1678,7 @@ __device__ __forceinline__ void lu_solve_any(const Grp<G>& g, const W& w, int A,
 }
 
 // The factorisation as the solve kernels run it, after the row scaling sc: by
-// register panels and matrix tiles for 32 or more threads (m <= 128; rows left
-// in place, perm), the blocked form otherwise, with panels of NB columns and
+// register panels and matrix tiles for 32 or more threads (m <= 128), the blocked form otherwise, with panels of NB columns and
 // rows exchanged; then, for groups of 16 or more threads, the reciprocal pivots
 // 1 / U[i][i] in rd (sc and rd may be the same array for fewer than 32 threads)
 // and the row permutation of the solves (lu_solve_any).

@@ -134,12 +134,7 @@ __global__ void __launch_bounds__(G < 32 ? 32 : G) lu_form_kernel(int m, double*
     row_scale(g, w, oA, ld, osc, m);
     lu_factor<G, EXACT>(g, w, oA, ld, opiv, osc, ord, operm, m);
     g.sync();
-    // the factors in the reference's row order
-    const bool by_perm = G >= 32 && m <= 128;
-    for (int e = g.lane; e < m * m; e += G) {
-        const int i = by_perm ? w.ip(operm + e / m) : e / m;
-        Ag[e] = w[oA + i * ld + e % m];
-    }
+    for (int e = g.lane; e < m * m; e += G) Ag[e] = w[oA + (e / m) * ld + (e % m)];
     for (int i = g.lane; i < m; i += G) piv[(size_t)blockIdx.x * m + i] = w.ip(opiv + i);
     for (int r = 0; r < n_rhs; ++r) {
         double* bg = b + ((size_t)blockIdx.x * n_rhs + r) * m;
