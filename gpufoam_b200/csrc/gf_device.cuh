@@ -26,6 +26,7 @@ namespace gf {
 // gpu_utils/common/gpu_constants.H:13-82
 constexpr double kRR = 6.02214e+26 * 1.38065e-23;
 constexpr double kPstd = 1e5;
+constexpr double kLnPstdR = 2.4871731053390858;  // ln(kPstd / kRR)
 constexpr double kVSmall = 2.2250738585072014e-308;  // numeric_limits<double>::min()
 constexpr double kSmall = 2.220446049250313e-16;     // numeric_limits<double>::epsilon()
 constexpr double kVGreat = 1.7976931348623157e+308 / 10.0;
@@ -315,7 +316,7 @@ __device__ __forceinline__ TCache make_tcache(double T) {
     t.T = T;
     t.invT = 1.0 / T;
     t.logT = log(T);
-    t.lx = log(kPstd / (kRR * T));
+    t.lx = kLnPstdR - t.logT;
     return t;
 }
 
@@ -445,12 +446,23 @@ __device__ __forceinline__ void third_body_all(const Grp<G>& g, const DevMech& M
         const double* e = M.effT + t;
         double s0 = 0.0, s1 = 0.0;
         int i = 0;
-#pragma unroll 4
-        for (; i + 1 < M.nS; i += 2) {
-            s0 = fma(ldg(e + (size_t)i * n), w[c_off + i], s0);
-            s1 = fma(ldg(e + (size_t)(i + 1) * n), w[c_off + i + 1], s1);
+        constexpr int U = 16;  // loads in flight
+        for (; i + U <= M.nS; i += U) {
+            double v[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) v[k] = ldg(e + (size_t)(i + k) * n);
+#pragma unroll
+            for (int k = 0; k < U; k += 2) {
+                s0 = fma(v[k], w[c_off + i + k], s0);
+                s1 = fma(v[k + 1], w[c_off + i + k + 1], s1);
+            }
         }
-        if (i < M.nS) s0 = fma(ldg(e + (size_t)i * n), w[c_off + i], s0);
+#pragma unroll 4
+        for (; i < M.nS; ++i) {
+            const double t = s0;
+            s0 = s1;
+            s1 = fma(ldg(e + (size_t)i * n), w[c_off + i], t);
+        }
         w[m_off + t] = s0 + s1;
     }
 }
@@ -709,17 +721,17 @@ __host__ __device__ constexpr int stream_index(int G) { return G == 96 ? 9 : log
 // Runs this thread's share of a gather stream (gf_internal.h, Stream):
 // wd[dst + pos] = sum of coef * ws[src + slot] over each entry's records, in
 // order. The group's loads (48 coalesced bytes and the position) are
-// independent of the sums, so they pipeline; one thread owns each output entry
-// (no barriers inside). Bound by instructions: 20 per four records, where
+// independent of the sums, so they pipeline (U groups at a time); one thread
+// owns each output entry (no barriers inside). Bound by instructions: 20 per four records, where
 // 16-byte records that each carried a position took 12 per record.
-template <int G, class WS, class WD>
+template <int U = 2, int G, class WS, class WD>
 __device__ __forceinline__ void stream_gather(const Grp<G>& g, const Stream& st, const WS& ws, int src, const WD& wd,
                                               int dst) {
     const int4* o = reinterpret_cast<const int4*>(st.off) + g.lane;
     const double2* c = reinterpret_cast<const double2*>(st.coef) + g.lane;
     const int* p = st.pos + g.lane;
     double acc = 0.0;
-#pragma unroll 2
+#pragma unroll U
     for (int k = 0; k < st.len; ++k) {
         const int4 v = __ldg(o + (size_t)k * G);
         const double2 a = __ldg(c + (size_t)k * 2 * G), b = __ldg(c + (size_t)k * 2 * G + G);
@@ -865,21 +877,38 @@ __device__ __forceinline__ void jacobian(const Grp<G>& g, const DevMech& M, cons
     GF_PH_BEGIN(g)
     // raw dN/dc, T-column and third-body terms of every entry (species rows x
     // species and T columns), one thread per entry, in the reference's order
-    stream_gather(g, M.jst[stream_index(G)], w, L.stage, w, L.J);
+    stream_gather<4>(g, M.jst[stream_index(G)], w, L.stage, w, L.J);
     g.sync();
-    // phase 3
-    for (int s = g.lane; s < nS; s += G) {
+    // phase 3: a thread per row and, where the group has more threads than
+    // rows, per part of its columns
+    const int rows = (nS + 31) & ~31, parts = min(2, max(1, G / rows));
+    const int part = G > 32 ? g.lane / rows : 0;
+    const int c0 = part < parts ? part * nS / parts : nS, c1 = part < parts ? (part + 1) * nS / parts : nS;
+    for (int s = G > 32 ? g.lane - part * rows : g.lane; s < nS && c0 < c1; s += parts > 1 ? rows : G) {
         const double Ws = ldg(M.W + s);
         const double dfs = w[L.dfdx + s];
         const int row = L.J + s * ld;
-        double ddN = w[row + nS];
-        for (int c = 0; c < nS; ++c) {
+        double ddN = 0.0;
+#pragma unroll 4
+        for (int c = c0; c < c1; ++c) {
             const double raw = w[row + c];
-            ddN -= raw * w[L.c + c] * alphav;
+            ddN -= raw * w[L.c + c];
             // (W_s / rhoM) raw (rhoM / W_c) + rhoM v_c df_s
             w[row + c] = Ws * ldg(M.invW + c) * raw + rToP * ldg(M.Rsp + c) * dfs;
         }
-        w[row + nS] = Ws * x.irho * ddN + alphav * dfs;
+        if (parts > 1)
+            w[L.part + part * nS + s] = ddN;
+        else
+            w[row + nS] = Ws * x.irho * (w[row + nS] + ddN * alphav) + alphav * dfs;
+    }
+    if (parts > 1) {
+        g.sync();
+        for (int s = g.lane; s < nS; s += G) {
+            double ddN = 0.0;
+            for (int k = 0; k < parts; ++k) ddN += w[L.part + k * nS + s];
+            const int row = L.J + s * ld;
+            w[row + nS] = ldg(M.W + s) * x.irho * (w[row + nS] + ddN * alphav) + alphav * w[L.dfdx + s];
+        }
     }
     g.sync();
     GF_PH_END(g, PH_JROWS)
@@ -1074,19 +1103,60 @@ __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double
 
 constexpr int kPanel = 8;  // columns per panel of lu_decompose_mma: two tile depths
 
+// The pivot of a panel step by the reference's rule where the high words do not
+// decide it: the last position with the largest vv |a| among the candidates
+// (lab >= k; a NaN is never taken), row k where there is none. Returns the lane
+// and register row that hold it. Out of line: reached on ties only.
+template <int RP>
+struct PivotRows {
+    double t[RP];  // vv |a|
+    int lab[RP];
+};
+template <int RP>
+__device__ __noinline__ int pivot_exact(PivotRows<RP> c, int k) {
+    double best = -1.0;
+    int bi = -1, ri = 0;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+        if (c.lab[r] >= k && (c.t[r] > best || (c.t[r] == best && c.lab[r] > bi))) {
+            best = c.t[r];
+            bi = c.lab[r];
+            ri = r;
+        }
+    }
+    const bool has = bi >= 0;
+    const unsigned hi = has ? (unsigned)__double2hiint(best) : 0u;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const bool c1 = has && hi == mh;
+    const unsigned lo = c1 ? (unsigned)__double2loint(best) : 0u;
+    const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+    int mr = (int)__reduce_max_sync(0xffffffffu, (c1 && lo == ml) ? (unsigned)(bi + 1) : 0u) - 1;
+    if (mr < 0) {
+        mr = k;
+#pragma unroll
+        for (int r = 0; r < RP; ++r)
+            if (c.lab[r] == k) {
+                bi = k;
+                ri = r;
+            }
+    }
+    const int li = __ffs(__ballot_sync(0xffffffffu, bi == mr)) - 1;
+    return li | (__shfl_sync(0xffffffffu, ri, li) << 5);
+}
+
 // Panel steps k0 .. k0+kb-1 with the panel held in registers (one full warp):
 // lane l holds the rows at positions k0 + l + 32 r, each with its row scaling
 // and a label, the position that it has in the reference's matrix after the
 // exchanges so far (-1: no row). An exchange of rows k and iMax swaps two
-// labels; pivot search, tie-break ("last max wins" by position) and update go
-// by label, and at the end perm[] takes the labels: perm[position] = the row of
-// the workspace that holds it. Rows never move. The pivot search reduces the
-// high words of the non-negative candidates with one integer warp reduction;
-// only equal high words need the low words and the position. Meanwhile every
-// lane has formed the reciprocal of its own candidate, so the division is off
-// the chain of dependent operations. Difference: when every candidate of a
-// column is NaN, the reference exchanges row k with row 0 (its iMax starts at
-// 0); here none is. The reciprocal pivots go to rd, the pivots to piv.
+// labels, and at the end perm[] takes the labels: perm[position] = the row of
+// the workspace that holds it. Rows do not move. The pivot search (ludecompose.H
+// :57-63) compares the high words of vv |a|: one integer warp reduction; where
+// they tie, are zero or a NaN is the largest, pivot_exact decides. Meanwhile
+// every lane has formed the reciprocal of its own candidate, so the division is
+// off the chain of dependent operations. A zero pivot becomes gpuSmall (:81).
+// Difference: when every candidate of a column is NaN, the reference exchanges
+// row k with row 0 (its iMax starts at 0); here none is. The reciprocal pivots
+// go to rd, the pivots to piv (unless piv < 0).
 template <int RP, bool EXACT, class W>
 __device__ __forceinline__ void lu_panel_reg(const W& w, int A, int ld, int piv, int sc, int rd, int perm, int m,
                                              int k0, int kb) {
@@ -1098,56 +1168,58 @@ __device__ __forceinline__ void lu_panel_reg(const W& w, int A, int ld, int piv,
         const int p = k0 + l + 32 * r;
         lab[r] = p < m ? p : -1;
         row[r] = p < m ? w.ip(perm + p) : 0;
-        sv[r] = p < m ? w[sc + row[r]] : 0.0;
+        sv[r] = w[sc + row[r]];
 #pragma unroll
-        for (int t = 0; t < kPanel; ++t) a[r][t] = (p < m && t < kb) ? w[A + row[r] * ld + k0 + t] : 0.0;
+        for (int t = 0; t < kPanel; ++t) a[r][t] = t < kb ? w[A + row[r] * ld + k0 + t] : 0.0;
     }
 #pragma unroll
     for (int kk = 0; kk < kPanel; ++kk) {
         if (kk >= kb) break;
         const int k = k0 + kk;
-        // the lane's candidate: the last position with the largest vv * |a|
-        // (ludecompose.H:57-63); a zero pivot becomes gpuSmall (:81)
-        double best = -1.0, x = 1.0;
-        int bi = -1, ri = 0;
+        // the lane's candidate by high words (-1: no candidate)
+        PivotRows<RP> c;
+        int key = -1, ri = 0, tie = 0;
+        double x = a[0][kk];
 #pragma unroll
         for (int r = 0; r < RP; ++r) {
-            const double t = sv[r] * fabs(a[r][kk]);
-            if (lab[r] >= k && (t > best || (t == best && lab[r] > bi))) {
-                best = t;
-                bi = lab[r];
-                ri = r;
-                x = a[r][kk];
+            c.t[r] = sv[r] * fabs(a[r][kk]);
+            c.lab[r] = lab[r];
+            const int h = lab[r] >= k ? __double2hiint(c.t[r]) : -1;
+            if (r == 0) {
+                key = h;
+            } else {
+                tie = h == key ? 1 : (h > key ? 0 : tie);
+                if (h > key) {
+                    key = h;
+                    ri = r;
+                    x = a[r][kk];
+                }
             }
         }
-        if (x == 0.0) x = kSmall;
         double rinv = 1.0 / x;
-        const bool has = bi >= 0;
-        const unsigned hi = has ? (unsigned)__double2hiint(best) : 0u;
-        const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-        unsigned own = __ballot_sync(0xffffffffu, has && hi == mh);
-        if (__popc(own) != 1) {
-            const bool c = has && hi == mh;
-            const unsigned lo = c ? (unsigned)__double2loint(best) : 0u;
-            const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
-            const int mr = (int)__reduce_max_sync(0xffffffffu, (c && lo == ml) ? (unsigned)(bi + 1) : 0u) - 1;
-            if (mr < 0) {
-                // no candidate (a column of NaN): row k stays
+        const int mh = __reduce_max_sync(0xffffffffu, key);
+        const unsigned own = __ballot_sync(0xffffffffu, key == mh);
+        const unsigned tied = __ballot_sync(0xffffffffu, key == mh && tie);
+        int li = __ffs(own) - 1;
+        if (tied != 0 || (own & (own - 1)) != 0 || mh <= 0 || mh > 0x7ff00000) {
+            const int v = pivot_exact<RP>(c, k);
+            li = v & 31;
+            if (l == li) {
+                ri = v >> 5;
 #pragma unroll
                 for (int r = 0; r < RP; ++r)
-                    if (lab[r] == k) {
-                        bi = k;
-                        ri = r;
-                        x = a[r][kk];
-                        rinv = x;
-                    }
+                    if (r == ri) x = a[r][kk];
+                if (x == 0.0) x = kSmall;
+                rinv = 1.0 / x;
             }
-            own = __ballot_sync(0xffffffffu, bi == (mr < 0 ? k : mr));
         }
-        const int li = __ffs(own) - 1;
+        // the pivot row's label, reciprocal and remaining entries, to every lane
+        int mine = lab[0];
+#pragma unroll
+        for (int r = 1; r < RP; ++r)
+            if (r == ri) mine = lab[r];
+        const int iMax = __shfl_sync(0xffffffffu, mine, li);
         rinv = __shfl_sync(0xffffffffu, rinv, li);
-        const int iMax = __shfl_sync(0xffffffffu, bi, li);
-        // the pivot row's remaining entries, to every lane
         double u[kPanel];
 #pragma unroll
         for (int t = kk + 1; t < kPanel; ++t) {
@@ -1159,15 +1231,14 @@ __device__ __forceinline__ void lu_panel_reg(const W& w, int A, int ld, int piv,
         }
 #pragma unroll
         for (int r = 0; r < RP; ++r) {
+            if (lab[r] == k) lab[r] = iMax;
             if (l == li && r == ri) {
                 lab[r] = k;
                 a[r][kk] = x;
-            } else if (lab[r] == k) {
-                lab[r] = iMax;
             }
         }
         if (l == 0) {
-            w.ip(piv + k) = iMax;
+            if (piv >= 0) w.ip(piv + k) = iMax;
             w[rd + k] = rinv;
         }
 #pragma unroll
@@ -1270,16 +1341,30 @@ __device__ __forceinline__ void lu_decompose_mma(const Grp<G>& g, const W& w, in
                 const double a0 = rin ? -w[ri + k0 + c4] : 0.0, a1 = rin ? -w[ri + k0 + 4 + c4] : 0.0;
                 const int run = min(nt - tc, t_end - t);
                 int col = k1 + 8 * tc;
-                for (int n = 0; n < run; ++n, col += 8) {
-                    const bool bin = col + r8 < m;
-                    const double b0 = bin ? w[p0 + col + r8] : 0.0, b1 = bin ? w[p1 + col + r8] : 0.0;
-                    const int j = col + 2 * c4;
-                    const bool in0 = rin && j < m, in1 = rin && j + 1 < m;
-                    double c0 = in0 ? w[ri + j] : 0.0, c1 = in1 ? w[ri + j + 1] : 0.0;
-                    mma_f64(c0, c1, a0, b0);
-                    mma_f64(c0, c1, a1, b1);
-                    if (in0) w[ri + j] = c0;
-                    if (in1) w[ri + j + 1] = c1;
+                // two tiles of the run at a time: their loads and updates overlap
+                for (int n = 0; n < run; n += 2, col += 16) {
+                    double b0[2], b1[2], c0[2], c1[2];
+                    bool in0[2], in1[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int cb = col + 8 * h + r8, j = col + 8 * h + 2 * c4;
+                        const bool on = n + h < run;
+                        b0[h] = on && cb < m ? w[p0 + cb] : 0.0;
+                        b1[h] = on && cb < m ? w[p1 + cb] : 0.0;
+                        in0[h] = on && rin && j < m;
+                        in1[h] = on && rin && j + 1 < m;
+                        c0[h] = in0[h] ? w[ri + j] : 0.0;
+                        c1[h] = in1[h] ? w[ri + j + 1] : 0.0;
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) mma_f64(c0[h], c1[h], a0, b0[h]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int j = col + 8 * h + 2 * c4;
+                        mma_f64(c0[h], c1[h], a1, b1[h]);
+                        if (in0[h]) w[ri + j] = c0[h];
+                        if (in1[h]) w[ri + j + 1] = c1[h];
+                    }
                 }
                 t += run;
                 ++tr;
@@ -1537,7 +1622,7 @@ __device__ __forceinline__ void lu_solve_reg(const Grp<G>& g, const W& w, int A,
 }
 
 #ifndef GF_SOLVE_UNROLL
-#define GF_SOLVE_UNROLL 2
+#define GF_SOLVE_UNROLL 1
 #endif
 constexpr int kSolveUnroll = GF_SOLVE_UNROLL;  // blocks of columns unrolled together
 // Register form for one full warp with R rows per lane (m <= 32 R): lane l
@@ -1803,7 +1888,8 @@ __device__ __forceinline__ void shift_and_factor(const Grp<G>& g, const DevMech&
         shift_and_scale(g, w, L.J, ld, sc, m, 1.0 / (C.gamma * dx));
         GF_PH_END(g, PH_SHIFT)
     }
-    lu_factor<G, false, NB>(g, w, L.J, ld, L.piv, sc, L.vv, L.perm, m);
+    // (the solves of 32 or more threads follow perm)
+    lu_factor<G, false, NB>(g, w, L.J, ld, G >= 32 && m <= 128 ? -1 : L.piv, sc, L.vv, L.perm, m);
 }
 
 // The Jacobian at y0, then shift_and_factor.
