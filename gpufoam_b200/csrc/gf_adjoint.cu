@@ -178,7 +178,7 @@ __device__ void lu_solve_transposed(const Grp<G>& g, const W& w, const WsC& wa, 
 template <int G, class W>
 __device__ void adj_mixture(const Grp<G>& g, const DevMech& M, const W& w, const WsC& wa, const WsLayout& L, const AdjLayout& A,
                             int y_off, double p) {
-    const Mix x = mixture<true, true>(g, M, w, L, y_off, p);
+    const Mix x = mixture<true>(g, M, w, L, y_off, p, true);
     if (g.lane == 0) {
         wa[A.ms + MS_RHO] = x.rhoM;
         wa[A.ms + MS_CPM] = x.CpM;
@@ -590,9 +590,9 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
     // recompute the attempt (stages kept: k_i, y2, y3; LU factors in L.J)
     {
         GF_PH_BEGIN(g)
-        // f(y0) keeps its rate constants for the Jacobian at the same state
-        derivatives(g, M, w, L, L.y0, p, L.dydx0, true);
-        jacobian<true>(g, M, w, L, L.y0, p);
+        // f(y0) keeps its rate constants and mixture for the Jacobian at the same state
+        const Mix x = derivatives(g, M, w, L, L.y0, p, L.dydx0, true);
+        jacobian(g, M, w, L, L.y0, p, L.dydx0, x);
         // kept for the Jacobian term: the raw entries (from the Jacobian terms
         // in the staging slots), the converted Jacobian and dfdx
         stream_gather(g, M.jst[stream_index(G)], w, L.stage, wa, A.raw);

@@ -643,15 +643,15 @@ struct Mix {
 // (deterministic; the reference sums sequentially), all of them in one
 // reduction. No division per species: 1/rho_i = (R/W_i) T/p, the polynomials'
 // divisors and 1/W_i are in the tables, and the expansion coefficient
-// sum(Y_i / (rho_i T)) rhoM of a perfect gas is 1/T. JAC: also Cp; STORE: also
+// sum(Y_i / (rho_i T)) rhoM of a perfect gas is 1/T. jac: also Cp; STORE: also
 // the per-species v and rhoM/W that the adjoint reads.
-template <bool JAC, bool STORE = false, int G, class W>
+template <bool STORE = false, int G, class W>
 __device__ __forceinline__ Mix mixture(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L, int y_off,
-                                       double p) {
+                                       double p, bool jac) {
     const int nS = M.nS;
     const double T = w[y_off + nS];
     const double ToP = T / p;
-    double sm[JAC ? 3 : 2] = {};
+    double sm[3] = {};
     for (int i = g.lane; i < nS; i += G) {
         const double yi = fmax(w[y_off + i], 0.0);
         const double vi = ldg(M.Rsp + i) * ToP;
@@ -664,8 +664,8 @@ __device__ __forceinline__ Mix mixture(const Grp<G>& g, const DevMech& M, const 
         sm[1] += yi * Cpi;
         w[L.Ha + i] = ((((h4 * T + h3) * T + h2) * T + h1) * T + a0) * T + a5;
         w[L.c + i] = yi * ldg(M.invW + i);
-        if (JAC) {
-            sm[JAC ? 2 : 0] += yi * (((4.0 * a4 * T + 3.0 * a3) * T + 2.0 * a2) * T + a1);
+        if (jac) {
+            sm[2] += yi * (((4.0 * a4 * T + 3.0 * a3) * T + 2.0 * a2) * T + a1);
             w[L.Cp + i] = Cpi;
         }
         if (STORE) w[L.vj + i] = vi;
@@ -675,8 +675,8 @@ __device__ __forceinline__ Mix mixture(const Grp<G>& g, const DevMech& M, const 
     x.irho = sm[0];
     x.rhoM = 1.0 / sm[0];
     x.CpM = sm[1];
-    x.dCpMdT = JAC ? sm[JAC ? 2 : 0] : 0.0;
-    x.alphav = JAC ? 1.0 / T : 0.0;
+    x.dCpMdT = sm[2];
+    x.alphav = jac ? 1.0 / T : 0.0;
     for (int i = g.lane; i < nS; i += G) {
         w[L.c + i] *= x.rhoM;
         if (STORE) w[L.rhoMbyW + i] = x.rhoM * ldg(M.invW + i);
@@ -777,14 +777,16 @@ __device__ __forceinline__ void gather_rhs(const Grp<G>& g, const DevMech& M, co
 }
 
 // gpuODESystem::derivatives (gpuODESystem.H:164-196): out = f(y), entries 0..nS
+// With write_cache it also leaves what the Jacobian at the same state needs: the
+// rate constants, the species' Cp, and the mixture (returned).
 template <int G, class W>
-__device__ __forceinline__ void derivatives(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
-                                            int y_off, double p, int out_off, bool write_cache = false) {
+__device__ __forceinline__ Mix derivatives(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
+                                           int y_off, double p, int out_off, bool write_cache = false) {
     Mix x;
     g.sync();
     {
         GF_PH_BEGIN(g)
-        x = mixture<false>(g, M, w, L, y_off, p);
+        x = mixture(g, M, w, L, y_off, p, write_cache);
         GF_PH_END(g, PH_MIX)
     }
     const double T = w[y_off + M.nS];
@@ -808,6 +810,7 @@ __device__ __forceinline__ void derivatives(const Grp<G>& g, const DevMech& M, c
         gather_rhs(g, M, w, L, out_off, x);
         GF_PH_END(g, PH_GATHER_RHS)
     }
+    return x;
 }
 
 // Per-reaction Jacobian parameters (computeReactionParameters, gpuReaction.H:650-702)
@@ -847,30 +850,30 @@ __device__ __forceinline__ void stage_jacobian_params(const Grp<G>& g, const Dev
 //     third-body terms in the reference's order per entry;
 //   phase 3 (lanes over rows): ddY_dcdY (gpuODESystem.H:65-103);
 //   then the T row (ddT_dtdY, ddT_dtdT, :108-146).
-// The rate constants are those that derivatives() with write_cache left in the
-// staging slots at the same state. STORE: the mixture's v and rhoM/W are kept
-// too (the adjoint).
-template <bool STORE = false, int G, class W>
+// The rate constants, Cp and the mixture x are those that derivatives() with
+// write_cache left at the same state, and dfdx is the f that it wrote to f_off
+// (the reference evaluates all of them again), except where the reaction
+// temperature limits clipped its rates: the Jacobian's are not clipped.
+template <int G, class W>
 __device__ __forceinline__ void jacobian(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
-                                         int y_off, double p) {
+                                         int y_off, double p, int f_off, const Mix& x) {
     const int nS = M.nS;
     const int ld = L.ld;
-    Mix x;
-    g.sync();
+    const double T = w[y_off + nS];
+    const double alphav = x.alphav, rToP = x.rhoM * (T / p);
     {
         GF_PH_BEGIN(g)
-        x = mixture<true, STORE>(g, M, w, L, y_off, p);
-        GF_PH_END(g, PH_MIX)
-    }
-    const double alphav = x.alphav, rToP = x.rhoM * (w[y_off + nS] / p);
-    {
-        GF_PH_BEGIN(g)
-        stage_jacobian_params(g, M, w, L, make_tcache(w[y_off + nS]));
+        stage_jacobian_params(g, M, w, L, make_tcache(T));
         GF_PH_END(g, PH_JPARAMS)
     }
     {
         GF_PH_BEGIN(g)
-        gather_rhs(g, M, w, L, L.dfdx, x);
+        if (T < M.Tlow || T > M.Thigh) {
+            gather_rhs(g, M, w, L, L.dfdx, x);
+        } else {
+            for (int i = g.lane; i < M.m; i += G) w[L.dfdx + i] = w[f_off + i];
+            g.sync();
+        }
         GF_PH_END(g, PH_GATHER_RHS)
     }
     {
@@ -1892,14 +1895,6 @@ __device__ __forceinline__ void shift_and_factor(const Grp<G>& g, const DevMech&
     lu_factor<G, false, NB>(g, w, L.J, ld, G >= 32 && m <= 128 ? -1 : L.piv, sc, L.vv, L.perm, m);
 }
 
-// The Jacobian at y0, then shift_and_factor.
-template <int G, class W, int NB = 8>
-__device__ __forceinline__ void factor_step(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L,
-                                            const RosCoeffs& C, int y0_off, double p, double dx) {
-    jacobian(g, M, w, L, y0_off, p);
-    shift_and_factor<G, W, NB>(g, M, w, L, C, dx);
-}
-
 // One attempt solve(y0, dydx0, dx, y) of gpuRosenbrock12/23/34 (their
 // solve(y0, dydx0, dx, y, buffer)); returns the normalised error
 // (normaliseError.H:6-29; the p entry contributes 0). y0 is at y0_off, the
@@ -1912,14 +1907,13 @@ __device__ __forceinline__ void factor_step(const Grp<G>& g, const DevMech& M, c
 // instruction footprint. A retried step evaluates it again (the same value),
 // which brings back the rate constants that the Jacobian reads: cheaper than a
 // second copy of the rate code for the few retries (4 % of the attempts).
-// Otherwise the caller provides dydx0.
+// Without F0 (SAVE) the caller provides dydx0 and the factors.
 template <int G, class W, bool SAVE = false, bool F0 = false, int NB = 8>
 __device__ __forceinline__ double ros_attempt(const Grp<G>& g, const DevMech& M, const W& w, const WsLayout& L, const RosCoeffs& C,
                               const OdeParams& o, int y0_off, int yt_off, double p, double dx, int save_y2 = -1,
                               int save_y3 = -1, int save_f2 = -1, int save_f3 = -1) {
     const int m = M.m;
     const int ld = L.ld;
-    if constexpr (!F0 && !SAVE) factor_step<G, W, NB>(g, M, w, L, C, y0_off, p, dx);
     // stages: k_i solves (I/(gamma dx) - J) k_i = f_i + dx d_i dfdx + sum_j c_ij k_j / dx,
     // f_0 = f(y0), f_i = f(y0 + sum_j a_ij k_j) where the method takes a new
     // derivative (stage 1; stage 2 of Rosenbrock34), else the previous one.
@@ -1940,7 +1934,8 @@ __device__ __forceinline__ double ros_attempt(const Grp<G>& g, const DevMech& M,
             at = pt;
             out = L.dydx;
         }
-        if (new_f) derivatives(g, M, w, L, at, p, out, st < 0);
+        Mix x;
+        if (new_f) x = derivatives(g, M, w, L, at, p, out, st < 0);
         if constexpr (SAVE) {
             if (st > 0 && new_f) {
                 const int fs = st == 1 ? save_f2 : save_f3;
@@ -1949,7 +1944,8 @@ __device__ __forceinline__ double ros_attempt(const Grp<G>& g, const DevMech& M,
         }
         if constexpr (F0) {
             if (st < 0) {
-                factor_step<G, W, NB>(g, M, w, L, C, y0_off, p, dx);
+                jacobian(g, M, w, L, y0_off, p, L.dydx0, x);
+                shift_and_factor<G, W, NB>(g, M, w, L, C, dx);
                 continue;
             }
         }
@@ -2013,7 +2009,7 @@ __device__ __forceinline__ int ode_solve(const Grp<G>& g, const DevMech& M, cons
     double step_dxTry = *dxTry;
     bool last = false;
     double x = xStart;
-    const double inc_threshold = pow(o.maxScale / o.safeScale, -1.0 / o.alphaInc);
+    const double inc_threshold = real_pow(o.maxScale / o.safeScale, -1.0 / o.alphaInc);
     for (int nStep = 0; nStep < o.maxSteps; nStep++) {
         const double dxTry0 = step_dxTry;
         if ((x + step_dxTry - xEnd) * (x + step_dxTry - xStart) > 0) {
@@ -2026,14 +2022,12 @@ __device__ __forceinline__ int ode_solve(const Grp<G>& g, const DevMech& M, cons
         do {
             GF_PH_BEGIN(g)
             // adaptiveSolve's derivatives call (gpuAdaptiveSolver.H:96), which
-            // also leaves the rate constants for the attempt's Jacobian: in the
-            // solve kernel, inside the attempt
-            if constexpr (REC) derivatives(g, M, w, L, *y_off, p, L.dydx0, true);
-            err = ros_attempt<G, W, false, !REC, NB>(g, M, w, L, C, o, *y_off, *yt_off, p, dx);
+            // also leaves what the attempt's Jacobian needs, is inside the attempt
+            err = ros_attempt<G, W, false, true, NB>(g, M, w, L, C, o, *y_off, *yt_off, p, dx);
             GF_PH_END(g, PH_ATTEMPT)
             ++*attempts;
             if (err > 1) {
-                const double scale = fmax(o.safeScale * pow(err, -o.alphaDec), o.minScale);
+                const double scale = fmax(o.safeScale * real_pow(err, -o.alphaDec), o.minScale);
                 dx *= scale;
                 // the reference traps here (gpuAdaptiveSolver.H:111-114); the cap
                 // also ends the loop for step controls that never shrink dx
@@ -2052,7 +2046,7 @@ __device__ __forceinline__ int ode_solve(const Grp<G>& g, const DevMech& M, cons
         *y_off = *yt_off;
         *yt_off = t;
         if (err > inc_threshold) {
-            step_dxTry = fmin(fmax(o.safeScale * pow(err, -o.alphaInc), o.minScale), o.maxScale) * dx;
+            step_dxTry = fmin(fmax(o.safeScale * real_pow(err, -o.alphaInc), o.minScale), o.maxScale) * dx;
         } else {
             step_dxTry = o.safeScale * o.maxScale * dx;
         }

@@ -232,6 +232,41 @@ int ensure_ws(gf_solver* s, size_t bytes) {
     return GF_OK;
 }
 
+// The launch form of a solver that none was set for, by the largest matrix
+// size m of its mechanisms: persistent, the workspace in shared memory where it
+// fits, and the kernel compiled for m where there is one (the autotuner refines
+// this on a sample of cells). Measured on the B200, 64 threads per cell (two
+// warps, any m) against the rule:
+//  * m <= 32: a warp per cell, four cells per CTA; a second warp has no rows or
+//    reactions to work on. 65,536 cells of 10 species 148 -> 63 ms;
+//  * m <= 64: 128 threads and 128 registers; four cells per SM by registers,
+//    the other three warps shorten the reaction loops and gathers, and the rest
+//    of the SM's memory is L1 for the tables. 16,384 cells of 53 species
+//    224 -> 153 ms (96 threads: 139 ms there, but 5 % behind on 64k cells);
+//  * m <= 128: 256 threads; shared memory holds one cell per SM, and only its own
+//    threads hide its latency. 701 cells of 100 species 55 -> 31 ms;
+//  * larger ones, and workspaces in HBM: 64 threads.
+gf_launch_config default_launch(const gf_solver* s) {
+    int m = 0;
+    for (const gf::DevMech& d : s->dmechs) m = std::max(m, d.m);
+    const bool shared = (size_t)s->max_ws_doubles * sizeof(double) <= 227 * 1024;
+    // kind, threads, shared, cells / CTA, CTAs / SM, registers, panel, specialize
+    gf_launch_config c{1, 64, shared ? 1 : 0, 1, 0, 0, 0, 0};
+    if (shared && m <= 32) {
+        c.threads_per_cell = 32;
+        c.cells_per_block = 0;
+    } else if (shared && m <= 64) {
+        c.threads_per_cell = 128;
+        c.register_budget = 1;
+    } else if (shared && m <= 128) {
+        c.threads_per_cell = 256;
+    }
+    gf_launch_config sp = c;
+    sp.specialize = 1;
+    if (gf::persistent_form_compiled(sp, gf::specialized_size(s->dmechs.data(), (int)s->dmechs.size()))) c = sp;
+    return c;
+}
+
 int ensure_staging(gf_solver* s, int n) {
     if (n <= s->staged_cells) return GF_OK;
     cudaFree(s->dY);
@@ -752,11 +787,7 @@ int gf_solver_create(const gf_mech* const* mechs, int n_mechs, const gf_ode_inpu
     s->ode = gf::OdeParams{in->solver, in->absTol, in->relTol, in->maxSteps, in->safeScale, in->alphaInc,
                            in->alphaDec, in->minScale, in->maxScale};
     s->Treact = Treact;
-    // default launch: persistent, two warps per cell (one cell per CTA),
-    // workspace in shared memory when it fits (the autotuner refines this per
-    // mechanism)
-    s->cfg = gf_launch_config{1, 64, 1, 1, 0, 0, 0, 0};  // kind, G, shared, cells/CTA, CTAs/SM, registers, panel, specialize
-    if ((size_t)s->max_ws_doubles * sizeof(double) > 227 * 1024) s->cfg.scratch_in_shared = 0;
+    s->cfg = default_launch(s);
     cudaError_t e = cudaMalloc(&s->queue, 8 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost(&s->queue_host, 8 * sizeof(unsigned long long));
     if (e != cudaSuccess) {

@@ -71,8 +71,9 @@ __global__ void __launch_bounds__(32) jacobian_kernel(const DevMech M, const dou
     for (int i = g.lane; i < M.m; i += 32) w[L.y0 + i] = yi[i];
     if (g.lane == 0) w[L.stage + M.n_slots] = 0.0;
     const double p = yi[M.nS + 1];
-    derivatives(g, M, w, L, L.y0, p, L.dydx, true);  // leaves the rate constants for the Jacobian
-    jacobian(g, M, w, L, L.y0, p);
+    // f leaves the rate constants and the mixture for the Jacobian
+    const Mix x = derivatives(g, M, w, L, L.y0, p, L.dydx, true);
+    jacobian(g, M, w, L, L.y0, p, L.dydx, x);
     double* o = dfdx + (size_t)blockIdx.x * n;
     for (int i = g.lane; i < M.m; i += 32) o[i] = w[L.dfdx + i];
     if (g.lane == 0) o[n - 1] = 0.0;
