@@ -4,9 +4,13 @@
 // scatter of the cell-major rates back into per-species fields
 // (computeRRAndChemDeltaT, gpuChemistryModel.C:351-356). Both are transposes
 // through a shared-memory tile of kTileCells cells, so that the field-side
-// accesses (consecutive cells of one field) and the cell-side accesses
-// (consecutive entries of one cell's row) are both coalesced. HBM-bound data
-// movement, no arithmetic.
+// accesses (a warp: 32 consecutive cells of one field) and the cell-side
+// accesses (a warp: one cell's row) are both coalesced. HBM-bound data movement,
+// no arithmetic: what counts is the bytes in flight, so every warp issues all
+// loads of its share of a tile before it stores them. (Tiles of 16 cells with a
+// division per element moved 1.08 GB of 500,000 cells of 53 species in 334 us,
+// heat release included; 32 cells and one warp per field or row: see
+// launch_qdot.)
 #include <algorithm>
 
 #include "gf_internal.h"
@@ -15,8 +19,10 @@ namespace gf {
 
 namespace {
 
-constexpr int kTileCells = 16;
+constexpr int kTileCells = 32;
 constexpr int kTileThreads = 256;
+constexpr int kTileWarps = kTileThreads / 32;
+constexpr int kInFlight = 8;  // loads of a thread in flight
 
 struct FieldPtrs {
     const double* p[GF_MAX_SPECIES];
@@ -28,22 +34,27 @@ struct FieldOutPtrs {
 // y[c * ld + e] = field_e[c], e < nS the species, nS T, nS + 1 p
 __global__ void __launch_bounds__(kTileThreads)
     gather_states_kernel(const FieldPtrs Y, const double* T, const double* p, int n, int nS, double* y, int ld) {
-    extern __shared__ double tile[];  // [kTileCells][ne]
-    const int ne = nS + 2;
+    extern __shared__ double tile[];  // [kTileCells][ne | 1]
+    const int ne = nS + 2, lt = ne | 1;
+    const int wid = threadIdx.x >> 5, l = threadIdx.x & 31;
     for (long long c0 = (long long)blockIdx.x * kTileCells; c0 < n; c0 += (long long)gridDim.x * kTileCells) {
         const int nc = n - c0 < kTileCells ? (int)(n - c0) : kTileCells;
-        for (int t = threadIdx.x; t < ne * kTileCells; t += blockDim.x) {
-            const int e = t / kTileCells, j = t % kTileCells;
-            if (j < nc) {
-                const double* src = e < nS ? Y.p[e] : (e == nS ? T : p);
-                tile[j * ne + e] = src[c0 + j];
+        for (int e0 = wid; e0 < ne; e0 += kTileWarps * kInFlight) {
+            double v[kInFlight];
+#pragma unroll
+            for (int k = 0; k < kInFlight; ++k) {
+                const int e = e0 + k * kTileWarps;
+                if (e < ne && l < nc) v[k] = __ldcs((e < nS ? Y.p[e] : (e == nS ? T : p)) + c0 + l);
+            }
+#pragma unroll
+            for (int k = 0; k < kInFlight; ++k) {
+                const int e = e0 + k * kTileWarps;
+                if (e < ne && l < nc) tile[l * lt + e] = v[k];
             }
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < nc * ne; t += blockDim.x) {
-            const int j = t / ne, e = t % ne;
-            y[(c0 + j) * ld + e] = tile[j * ne + e];
-        }
+        for (int j = wid; j < nc; j += kTileWarps)
+            for (int e = l; e < ne; e += 32) y[(c0 + j) * ld + e] = tile[j * lt + e];
         __syncthreads();
     }
 }
@@ -51,25 +62,39 @@ __global__ void __launch_bounds__(kTileThreads)
 // field_i[c] = RR[c * ld + i], i < nS
 __global__ void __launch_bounds__(kTileThreads)
     scatter_rates_kernel(const double* RR, int ld, int n, int nS, const FieldOutPtrs out) {
-    extern __shared__ double tile[];  // [kTileCells][nS]
+    extern __shared__ double tile[];  // [kTileCells][nS | 1]
+    const int lt = nS | 1;
+    const int wid = threadIdx.x >> 5, l = threadIdx.x & 31;
+    constexpr int R = kTileCells / kTileWarps;  // rows of a warp
     for (long long c0 = (long long)blockIdx.x * kTileCells; c0 < n; c0 += (long long)gridDim.x * kTileCells) {
         const int nc = n - c0 < kTileCells ? (int)(n - c0) : kTileCells;
-        for (int t = threadIdx.x; t < nc * nS; t += blockDim.x) {
-            const int j = t / nS, i = t % nS;
-            tile[j * nS + i] = RR[(c0 + j) * ld + i];
+        for (int i0 = l; i0 < nS; i0 += 64) {
+            double v[R][2];
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int j = wid + k * kTileWarps, i = i0 + 32 * h;
+                    if (j < nc && i < nS) v[k][h] = __ldcs(RR + (c0 + j) * ld + i);
+                }
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int j = wid + k * kTileWarps, i = i0 + 32 * h;
+                    if (j < nc && i < nS) tile[j * lt + i] = v[k][h];
+                }
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < nS * kTileCells; t += blockDim.x) {
-            const int i = t / kTileCells, j = t % kTileCells;
-            if (j < nc) out.p[i][c0 + j] = tile[j * nS + i];
-        }
+        if (l < nc)
+            for (int i = wid; i < nS; i += kTileWarps) out.p[i][c0 + l] = tile[l * lt + i];
         __syncthreads();
     }
 }
 
 long long tile_grid(int n) {
     const long long tiles = (n + kTileCells - 1) / kTileCells;
-    return std::min<long long>(tiles, 16LL * device_sm_count());
+    return std::min<long long>(tiles, 32LL * device_sm_count());
 }
 
 }  // namespace
@@ -79,7 +104,10 @@ int launch_gather_states(int n, int nS, const double* const* Y, const double* T,
     if (n <= 0) return 0;
     FieldPtrs P{};
     for (int i = 0; i < nS; ++i) P.p[i] = Y[i];
-    const size_t smem = (size_t)kTileCells * (nS + 2) * sizeof(double);
+    const size_t smem = (size_t)kTileCells * ((nS + 2) | 1) * sizeof(double);
+    const cudaError_t e = cudaFuncSetAttribute(gather_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if (e != cudaSuccess) return (int)e;
     gather_states_kernel<<<(unsigned)tile_grid(n), kTileThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         P, T, p, n, nS, y, ld);
     return (int)cudaGetLastError();
@@ -89,7 +117,10 @@ int launch_scatter_rates(int n, int nS, const double* RR, int ld, double* const*
     if (n <= 0) return 0;
     FieldOutPtrs P{};
     for (int i = 0; i < nS; ++i) P.p[i] = out[i];
-    const size_t smem = (size_t)kTileCells * nS * sizeof(double);
+    const size_t smem = (size_t)kTileCells * (nS | 1) * sizeof(double);
+    const cudaError_t e = cudaFuncSetAttribute(scatter_rates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if (e != cudaSuccess) return (int)e;
     scatter_rates_kernel<<<(unsigned)tile_grid(n), kTileThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         RR, ld, n, nS, P);
     return (int)cudaGetLastError();

@@ -10,7 +10,8 @@
 // (:163-166), the rates as gpuReaction::omega computes them
 // (gpuReaction.H:472-488: kf Cf - kr Cr at the clipped temperature).
 //
-// One warp per cell with the cell's concentrations, third-body sums and
+// calculate() and tc(): a lane per cell (cell_lanes_kernel). One reaction, few
+// cells: one warp per cell with the cell's concentrations, third-body sums and
 // per-reaction staging in shared memory: the same device functions as the
 // solve (third_body_all, fast_kf, fast_lnKc, fast_C, the dN/dt gather
 // stream). Qdot is one thread per cell with the reference's sequential sum.
@@ -23,7 +24,8 @@ namespace gf {
 
 namespace {
 
-constexpr int kFieldCellsMax = 4;  // cells (warps) per CTA
+constexpr int kFieldCellsMax = 4;  // cells (warps) per CTA of the warp-per-cell form
+constexpr int kLaneCells = 8192;   // cells from which the lane-per-cell form is the faster one
 
 struct FieldLayout {
     WsLayout L;  // only c, Mtb and stage are used
@@ -156,15 +158,138 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
     }
 }
 
+// calculate() and tc() with a lane per cell: a CTA takes 32 cells, its warps
+// share out the reactions, and every lane evaluates a reaction for its own cell,
+// so the reaction's data is one broadcast load for 32 cells, no warp mixes rate
+// types, and there is no gather. Concentrations and each warp's own dN/dt live in
+// shared memory, species by species over the lanes (stride 33: the transposes in
+// and out are free of bank conflicts too). Per species the order of the
+// reference's sum inside a warp's reactions, then the warps in order. Bound by
+// instructions issued: some 220 per reaction and 32 cells, where a warp per cell
+// took 415 per 32 reactions of one cell and the gather besides.
+constexpr int kLaneStride = 33;
+
+// A value per species of one lane's cell.
+struct WsLane {
+    double* p;
+    __device__ __forceinline__ double& operator[](int i) const { return p[i * kLaneStride]; }
+};
+
+__global__ void __launch_bounds__(128, 4) cell_lanes_kernel(const DevMech M, const FieldArgs a) {
+    extern __shared__ double smem[];
+    const int nS = M.nS, NW = blockDim.x >> 5;
+    const int wid = threadIdx.x >> 5, l = threadIdx.x & 31;
+    double* cs = smem;                                              // [nS + 1][33]
+    double* dN = smem + (size_t)(nS + 1) * kLaneStride;             // [NW][nS][33]
+    double* red = dN + (size_t)NW * nS * kLaneStride;               // [NW][2][32]
+    const WsLane c{cs + l}, d{dN + (size_t)wid * nS * kLaneStride + l};
+    for (long long c0 = (long long)blockIdx.x * 32; c0 < a.n_cells; c0 += (long long)gridDim.x * 32) {
+        const int nc = a.n_cells - c0 < 32 ? (int)(a.n_cells - c0) : 32;
+        for (int j = wid; j < 32; j += NW) {
+            // lanes past the last cell work on a copy of it
+            const long long cell = c0 + min(j, nc - 1);
+            const double rho = a.rho[cell];
+            const double* y = a.y + cell * a.ld_y;
+            for (int i = l; i < nS; i += 32) cs[i * kLaneStride + j] = rho * y[i] / ldg(M.W + i);
+        }
+        if (wid == 0) c[nS] = 1.0;
+        for (int i = 0; i < nS; ++i) d[i] = 0.0;
+        const double T = a.y[(c0 + min(l, nc - 1)) * a.ld_y + nS];
+        const TCache tc = make_tcache(fmin(fmax(T, M.Tlow), M.Thigh));
+        __syncthreads();
+        double sW = 0.0, sW2 = 0.0;
+        for (int q = wid; q < M.nR; q += NW) {
+            const RxnF R = load_fast(M, q);
+            const LnK lk = load_lnK(M, q, tc.T);
+            double Mc = 0.0;
+            int t = (int)((unsigned)R.meta >> kRxnTbShift);
+            if (t != 0) {
+                if (t == kRxnTbFar) t = ldg(M.tb_row + q) + 1;
+                const double* eff = M.eff + (size_t)(t - 1) * nS;
+#pragma unroll 8
+                for (int i = 0; i < nS; ++i) Mc = fma(ldg(eff + i), c[i], Mc);
+            }
+            double Ak;
+            const double kf = fast_kf(M, q, R, tc, Mc, &Ak);
+            const double kr = R.irr() ? 0.0 : kf * exp(-fast_lnKc(R, lk, tc));
+            const double of = kf * fast_C(M, c, 0, R, q, 0), orv = kr * fast_C(M, c, 0, R, q, 1);
+            const double om = of - orv;
+            // dN/dt (gpuReaction.H:490-508): lhs, then rhs
+            const int nl = R.nl(), nr = R.nr(), b = ldg(M.sp_off + q);
+            double wf = 0.0, wr = 0.0;
+            for (int e = 0; e < nl; ++e) {
+                const int sp = ldg(M.sidx + b + e);
+                const double st = ldg(M.sst + b + e);
+                d[sp] = fma(-st, om, d[sp]);
+                wr = fma(st, orv, wr);
+            }
+            for (int e = nl; e < nl + nr; ++e) {
+                const int sp = ldg(M.sidx + b + e);
+                const double st = ldg(M.sst + b + e);
+                d[sp] = fma(st, om, d[sp]);
+                wf = fma(st, of, wf);
+            }
+            // tc()'s two sums over reactions
+            sW += wf + wr;
+            sW2 += wf * wf + wr * wr;
+        }
+        red[wid * 64 + l] = sW;
+        red[wid * 64 + 32 + l] = sW2;
+        __syncthreads();
+        if (a.RR)
+            for (int j = wid; j < nc; j += NW)
+                for (int i = l; i < nS; i += 32) {
+                    double v = 0.0;
+                    for (int k = 0; k < NW; ++k) v += dN[((size_t)k * nS + i) * kLaneStride + j];
+                    a.RR[(c0 + j) * a.ld_rr + i] = v * ldg(M.W + i);
+                }
+        if (a.tc && wid == 0 && l < nc) {
+            double w1 = 0.0, w2 = 0.0, ctot = 0.0;
+            for (int k = 0; k < NW; ++k) {
+                w1 += red[k * 64 + l];
+                w2 += red[k * 64 + 32 + l];
+            }
+            for (int i = 0; i < nS; ++i) ctot += c[i];
+            a.tc[c0 + l] = w2 == 0.0 ? DBL_MAX / 10.0 : w1 / w2 * ctot;
+        }
+        __syncthreads();
+    }
+}
+
 // Qdot = 0 - hf_0 RR_0 - hf_1 RR_1 - ... in species order, each product
-// rounded before the subtraction (no contraction), as the reference's loop.
-__global__ void qdot_kernel(const DevMech M, int n, const double* RR, int ld_rr, double* qdot) {
-    for (long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x; cell < n;
-         cell += (long long)gridDim.x * blockDim.x) {
-        const double* r = RR + cell * ld_rr;
-        double q = 0.0;
-        for (int i = 0; i < M.nS; ++i) q = __dsub_rn(q, __dmul_rn(ldg(M.hf + i), r[i]));
-        qdot[cell] = q;
+// rounded before the subtraction (no contraction), as the reference's loop: a
+// thread per cell, after the warp has brought the rows of its 32 cells to
+// shared memory with coalesced loads, kQdotRows rows in flight. Bound by HBM.
+constexpr int kQdotRows = 8;
+__global__ void __launch_bounds__(128) qdot_kernel(const DevMech M, int n, const double* RR, int ld_rr, double* qdot) {
+    extern __shared__ double smem[];
+    const int nS = M.nS, lt = nS | 1, l = threadIdx.x & 31;
+    const int warps = blockDim.x >> 5;
+    double* tile = smem + (size_t)(threadIdx.x >> 5) * 32 * lt;
+    for (long long c0 = ((long long)blockIdx.x * warps + (threadIdx.x >> 5)) * 32; c0 < n;
+         c0 += (long long)gridDim.x * warps * 32) {
+        const int nc = n - c0 < 32 ? (int)(n - c0) : 32;
+        for (int j0 = 0; j0 < nc; j0 += kQdotRows)
+            for (int i0 = l; i0 < nS; i0 += 64) {
+                double v[kQdotRows][2];
+#pragma unroll
+                for (int k = 0; k < kQdotRows; ++k)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (j0 + k < nc && i0 + 32 * h < nS) v[k][h] = __ldcs(RR + (c0 + j0 + k) * ld_rr + i0 + 32 * h);
+#pragma unroll
+                for (int k = 0; k < kQdotRows; ++k)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (j0 + k < nc && i0 + 32 * h < nS) tile[(j0 + k) * lt + i0 + 32 * h] = v[k][h];
+            }
+        __syncwarp();
+        if (l < nc) {
+            double q = 0.0;
+            for (int i = 0; i < nS; ++i) q = __dsub_rn(q, __dmul_rn(ldg(M.hf + i), tile[l * lt + i]));
+            qdot[c0 + l] = q;
+        }
+        __syncwarp();
     }
 }
 
@@ -172,6 +297,29 @@ __global__ void qdot_kernel(const DevMech M, int n, const double* RR, int ld_rr,
 
 int launch_cell_fields(const DevMech& M, const FieldArgs& a, void* stream) {
     if (a.n_cells <= 0) return 0;
+    // all reactions: a lane per cell, with as many warps as leave room for two
+    // CTAs per SM, while the cells fill the machine; a warp per cell for one
+    // reaction, for few cells and for mechanisms whose sums do not fit
+    if (a.reaction < 0 && a.n_cells >= kLaneCells) {
+        int warps = 4;
+        auto bytes = [&](int w) {
+            return ((size_t)(M.nS + 1) * kLaneStride + (size_t)w * (M.nS * kLaneStride + 64)) * sizeof(double);
+        };
+        while (warps > 1 && bytes(warps) > 113 * 1024) --warps;
+        if (bytes(warps) <= 227 * 1024) {
+            const size_t smem = bytes(warps);
+            const void* fn = reinterpret_cast<const void*>(&cell_lanes_kernel);
+            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return (int)e;
+            int per_sm = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cell_lanes_kernel, 32 * warps, smem);
+            if (e != cudaSuccess) return (int)e;
+            const long long grid =
+                std::min<long long>((a.n_cells + 31) / 32, (long long)std::max(per_sm, 1) * device_sm_count());
+            cell_lanes_kernel<<<(unsigned)grid, 32 * warps, smem, reinterpret_cast<cudaStream_t>(stream)>>>(M, a);
+            return (int)cudaGetLastError();
+        }
+    }
     const FieldLayout F = field_layout(M);
     const size_t per_cell = (size_t)F.size * sizeof(double);
     int dev = 0, max_smem = 0;
@@ -195,9 +343,16 @@ int launch_cell_fields(const DevMech& M, const FieldArgs& a, void* stream) {
 
 int launch_qdot(const DevMech& M, int n, const double* RR, int ld_rr, double* qdot, void* stream) {
     if (n <= 0) return 0;
-    const int threads = 128;
-    const long long grid = std::min<long long>((n + threads - 1) / threads, 8LL * device_sm_count());
-    qdot_kernel<<<(unsigned)grid, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(M, n, RR, ld_rr, qdot);
+    // a tile per warp: four warps, or as many as fit
+    const size_t per_warp = (size_t)32 * (M.nS | 1) * sizeof(double);
+    int warps = 4;
+    while (warps > 1 && per_warp * warps > 100 * 1024) --warps;
+    const size_t smem = per_warp * warps;
+    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&qdot_kernel),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    const long long grid = std::min<long long>((n + 32LL * warps - 1) / (32LL * warps), 8LL * device_sm_count());
+    qdot_kernel<<<(unsigned)grid, 32 * warps, smem, reinterpret_cast<cudaStream_t>(stream)>>>(M, n, RR, ld_rr, qdot);
     return (int)cudaGetLastError();
 }
 

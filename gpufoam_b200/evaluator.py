@@ -560,7 +560,8 @@ def gather_states(Y_fields, T, p, ld: Optional[int] = None):
     for f in list(Y_fields) + [T, p]:
         if f.dtype != torch.float64 or not f.is_cuda or not f.is_contiguous() or f.numel() < n:
             raise ValueError("fields must be contiguous float64 cuda tensors of at least n cells")
-    y = torch.zeros((n, ld), dtype=torch.float64, device="cuda")
+    # the kernel writes every state; only columns behind it are zero
+    y = (torch.zeros if ld > nS + 2 else torch.empty)((n, ld), dtype=torch.float64, device="cuda")
     ptrs = (C.c_void_p * max(nS, 1))(*[f.data_ptr() for f in Y_fields])
     lib = N.load()
     N.check(lib.gf_gather_states(n, nS, ptrs, _ptr(T), _ptr(p), _ptr(y), ld, _stream_ptr()), "gf_gather_states")
