@@ -107,48 +107,89 @@ struct AdjArgs {
 // ------------------------------------------------------------------ pieces
 
 // W^T x = b with the factors of W (rows permuted: P W = L U): U^T z = b
-// (forward substitution), L^T v = z (backward, unit diagonal), x[perm[i]] =
-// v[i]. One warp, R rows per lane (lane l holds rows l + 32 u), column by
-// column with the pivot value broadcast by a shuffle; the entries used at
-// step j are row j of the factors (contiguous). m <= 32 R.
+// (forward substitution, reciprocal pivots rd), L^T v = z (backward, unit
+// diagonal), x[perm[i]] = v[i]. One warp, R rows per lane (lane l holds rows l +
+// 32 u), in blocks of four columns as lu_solve_warp; the entries used at step j
+// are row j of the factors (contiguous). m <= 32 R. Column by column with a
+// division in the chain a step took some 250 cycles.
 template <int R, class W>
-__device__ void lu_solve_transposed_warp(const W& w, const WsC& wa, int A, int ld, int perm, int m, int b, int x) {
+__device__ void lu_solve_transposed_warp(const W& w, const WsC& wa, int A, int ld, int perm, int rd, int m, int b,
+                                         int x) {
     const int lane = threadIdx.x & 31;
     double z[R];
+    int col[R];  // the lane's rows are columns of the factors; past m: column 0, never stored
 #pragma unroll
     for (int u = 0; u < R; ++u) {
         const int i = 32 * u + lane;
+        col[u] = i < m ? A + i : A;
         z[u] = i < m ? wa[b + i] : 0.0;
     }
     // U^T z = b: z_j = b_j / U[j][j], then b_i -= U[j][i] z_j for i > j
-    for (int j = 0; j < m; ++j) {
-        const int t = j >> 5, l = j & 31;
-        const int row = A + j * ld;
-        double zt = z[0];
 #pragma unroll
-        for (int u = 1; u < R; ++u)
-            if (u == t) zt = z[u];
-        const double zj = __shfl_sync(0xffffffffu, zt, l) / w[row + j];
+    for (int t = 0; t < R; ++t) {
+        const int n = min(32, m - 32 * t);
+        int l0 = 0;
+#pragma unroll 1
+        for (; l0 + 4 <= n; l0 += 4) {
+            const int j0 = 32 * t + l0, rb = A + j0 * ld + j0, d = lane - l0;
+            double y[4];
 #pragma unroll
-        for (int u = 0; u < R; ++u) {
-            const int i = 32 * u + lane;
-            if (i == j) z[u] = zj;
-            if (i > j && i < m) z[u] -= w[row + i] * zj;
+            for (int i = 0; i < 4; ++i) y[i] = __shfl_sync(0xffffffffu, z[t], l0 + i);
+            const double u01 = w[rb + 1], u02 = w[rb + 2], u03 = w[rb + 3], u12 = w[rb + ld + 2], u13 = w[rb + ld + 3],
+                         u23 = w[rb + 2 * ld + 3];
+            y[0] *= w[rd + j0];
+            y[1] = (y[1] - u01 * y[0]) * w[rd + j0 + 1];
+            y[2] = ((y[2] - u02 * y[0]) - u12 * y[1]) * w[rd + j0 + 2];
+            y[3] = (((y[3] - u03 * y[0]) - u13 * y[1]) - u23 * y[2]) * w[rd + j0 + 3];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double f = w[col[t] + (j0 + k) * ld];
+                if (d > k) z[t] -= f * y[k];
+                if (d == k) z[t] = y[k];
+#pragma unroll
+                for (int u = t + 1; u < R; ++u) z[u] -= w[col[u] + (j0 + k) * ld] * y[k];
+            }
+        }
+#pragma unroll 1
+        for (; l0 < n; ++l0) {
+            const int j = 32 * t + l0;
+            const double zj = __shfl_sync(0xffffffffu, z[t], l0) * w[rd + j];
+            if (lane > l0) z[t] -= w[col[t] + j * ld] * zj;
+            if (lane == l0) z[t] = zj;
+#pragma unroll
+            for (int u = t + 1; u < R; ++u) z[u] -= w[col[u] + j * ld] * zj;
         }
     }
     // L^T v = z: v_j final, then z_i -= L[j][i] v_j for i < j (descending j)
-    for (int j = m - 1; j >= 0; --j) {
-        const int t = j >> 5, l = j & 31;
-        const int row = A + j * ld;
-        double zt = z[0];
 #pragma unroll
-        for (int u = 1; u < R; ++u)
-            if (u == t) zt = z[u];
-        const double vj = __shfl_sync(0xffffffffu, zt, l);
+    for (int t = R - 1; t >= 0; --t) {
+        int n = min(32, m - 32 * t);
+#pragma unroll 1
+        for (; n > 0 && (n & 3); --n) {
+            const int l0 = n - 1, j = 32 * t + l0;
+            const double vj = __shfl_sync(0xffffffffu, z[t], l0);
+            if (lane < l0) z[t] -= w[col[t] + j * ld] * vj;
 #pragma unroll
-        for (int u = 0; u < R; ++u) {
-            const int i = 32 * u + lane;
-            if (i < j) z[u] -= w[row + i] * vj;
+            for (int u = 0; u < t; ++u) z[u] -= w[col[u] + j * ld] * vj;
+        }
+#pragma unroll 1
+        for (int l0 = n - 4; l0 >= 0; l0 -= 4) {
+            const int j0 = 32 * t + l0, rb = A + j0 * ld + j0, d = lane - l0;
+            double y[4];
+#pragma unroll
+            for (int i = 3; i >= 0; --i) y[i] = __shfl_sync(0xffffffffu, z[t], l0 + i);
+            const double l10 = w[rb + ld], l20 = w[rb + 2 * ld], l21 = w[rb + 2 * ld + 1], l30 = w[rb + 3 * ld],
+                         l31 = w[rb + 3 * ld + 1], l32 = w[rb + 3 * ld + 2];
+            y[2] -= l32 * y[3];
+            y[1] = (y[1] - l31 * y[3]) - l21 * y[2];
+            y[0] = ((y[0] - l30 * y[3]) - l20 * y[2]) - l10 * y[1];
+#pragma unroll
+            for (int k = 3; k >= 0; --k) {
+                const double f = w[col[t] + (j0 + k) * ld];
+                if (d < k) z[t] -= f * y[k];
+#pragma unroll
+                for (int u = 0; u < t; ++u) z[u] -= w[col[u] + (j0 + k) * ld] * y[k];
+            }
         }
     }
 #pragma unroll
@@ -159,16 +200,16 @@ __device__ void lu_solve_transposed_warp(const W& w, const WsC& wa, int A, int l
 }
 
 template <int G, class W>
-__device__ void lu_solve_transposed(const Grp<G>& g, const W& w, const WsC& wa, int A, int ld, int perm, int m, int b,
-                                    int x) {
+__device__ void lu_solve_transposed(const Grp<G>& g, const W& w, const WsC& wa, int A, int ld, int perm, int rd, int m,
+                                    int b, int x) {
     g.sync();
     if (threadIdx.x < 32) {
         if (m <= 64)
-            lu_solve_transposed_warp<2>(w, wa, A, ld, perm, m, b, x);
+            lu_solve_transposed_warp<2>(w, wa, A, ld, perm, rd, m, b, x);
         else if (m <= 128)
-            lu_solve_transposed_warp<4>(w, wa, A, ld, perm, m, b, x);
+            lu_solve_transposed_warp<4>(w, wa, A, ld, perm, rd, m, b, x);
         else
-            lu_solve_transposed_warp<10>(w, wa, A, ld, perm, m, b, x);
+            lu_solve_transposed_warp<10>(w, wa, A, ld, perm, rd, m, b, x);
     }
     g.sync();
 }
@@ -616,7 +657,7 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
         const int rb = A.rb + st * m;
         {
             GF_PH_BEGIN(g)
-            lu_solve_transposed(g, w, wa, L.J, ld, L.perm, m, A.kb + st * m, rb);
+            lu_solve_transposed(g, w, wa, L.J, ld, L.perm, L.vv, m, A.kb + st * m, rb);
             GF_PH_END(g, PH_ADJ_TSOLVE)
         }
         const int fsrc = st == 0 ? A.fb0 : (st == 1 || C.s == 3 ? A.fb2 : A.fb3);
@@ -662,8 +703,15 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
     }
 }
 
-__global__ void __launch_bounds__(64) adjoint_kernel(const DevMech M, const AdjArgs a) {
+// MS > 0: the matrix size fixed at compile time, as in process_cell.
+template <int MS>
+__global__ void __launch_bounds__(64) adjoint_kernel(const DevMech Mp, const AdjArgs a) {
     extern __shared__ double smem[];
+    DevMech M = Mp;
+    if constexpr (MS > 0) {
+        M.m = MS;
+        M.nS = MS - 1;
+    }
     Grp<64> g;
     const WsLayout L = make_layout(M.nS, M.nR, M.n_slots, M.n_tb, true);
     int fwd = 0;
@@ -715,6 +763,7 @@ __global__ void __launch_bounds__(64) adjoint_kernel(const DevMech M, const AdjA
 // The recording solve (gf_solve_record): the persistent form with one cell
 // per 128-thread CTA, workspace in shared memory, at most 128 registers, and
 // each accepted step recorded for the sweep.
+template <int MS>
 __global__ void __launch_bounds__(128, 4) record_kernel(const DevMech M, const LaunchArgs a) {
     extern __shared__ double smem[];
     Grp<128> g;
@@ -723,23 +772,34 @@ __global__ void __launch_bounds__(128, 4) record_kernel(const DevMech M, const L
         if (g.lane == 0) cell = (long long)atomicAdd(a.queue, 1ull);
         cell = g.bcast_ll(cell, 0);
         if (cell >= a.n_cells) break;
-        process_cell<128, WsC, true>(g, M, WsC{smem}, a, (int)cell);
+        process_cell<128, WsC, true, 8, MS>(g, M, WsC{smem}, a, (int)cell);
     }
 }
 
 __global__ void adj_reset(unsigned long long* q) { q[0] = 0; }
 
+// The kernels compiled for the 53-species and the 10-species mechanisms, else
+// the general ones (64-thread sweep of 600 cells of 53 species, before / after:
+// see launch_adjoint_cells).
+using RecordFn = void (*)(const DevMech, const LaunchArgs);
+using AdjointFn = void (*)(const DevMech, const AdjArgs);
+static RecordFn record_fn(int m) { return m == 54 ? record_kernel<54> : (m == 11 ? record_kernel<11> : record_kernel<0>); }
+static AdjointFn adjoint_fn(int m) {
+    return m == 54 ? adjoint_kernel<54> : (m == 11 ? adjoint_kernel<11> : adjoint_kernel<0>);
+}
+
 int launch_record(const DevMech& M, const LaunchArgs& a, void* stream) {
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int smem = make_layout(M.nS, M.nR, M.n_slots, M.n_tb).size * (int)sizeof(double);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
-    cudaFuncSetAttribute(record_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const RecordFn fn = record_fn(M.m);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, record_kernel, 128, smem);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, smem);
     if (e != cudaSuccess) return (int)e;
     if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
     launch_epilogue_reset(a.queue, stream);
-    if (a.n_cells > 0) record_kernel<<<per_sm * device_sm_count(), 128, smem, s>>>(M, a);
+    if (a.n_cells > 0) fn<<<per_sm * device_sm_count(), 128, smem, s>>>(M, a);
     return (int)cudaGetLastError();
 }
 
@@ -759,9 +819,10 @@ static int adjoint_smem_bytes(const DevMech& M) {
 int adjoint_blocks_per_sm(const DevMech& M) {
     const int smem = adjoint_smem_bytes(M);
     if (smem > 227 * 1024) return 0;
-    cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const AdjointFn fn = adjoint_fn(M.m);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_kernel, 64, smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 64, smem) != cudaSuccess) return 0;
     return per_sm;
 }
 
@@ -790,7 +851,7 @@ int launch_adjoint_cells(const DevMech& M, int n_cells, const double* traj, int 
     a.queue = queue;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     adj_reset<<<1, 1, 0, s>>>(queue);
-    if (n_cells > 0) adjoint_kernel<<<n_blocks, 64, adjoint_smem_bytes(M), s>>>(M, a);
+    if (n_cells > 0) adjoint_fn(M.m)<<<n_blocks, 64, adjoint_smem_bytes(M), s>>>(M, a);
     return (int)cudaGetLastError();
 }
 
