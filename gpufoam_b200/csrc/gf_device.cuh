@@ -1293,7 +1293,13 @@ __device__ __forceinline__ void lu_decompose_mma(const Grp<G>& g, const W& w, in
         const int k1 = min(k0 + kPanel, m);
         {
             GF_PH_BEGIN(g)
-            if (wid == 0) lu_panel_reg<RP, EXACT>(w, A, ld, piv, sc, rd, perm, m, k0, k1 - k0);
+            // the last panels have one row per lane: 70 instead of 110 instructions a step
+            if (wid == 0) {
+                if (RP == 1 || m - k0 <= 32)
+                    lu_panel_reg<1, EXACT>(w, A, ld, piv, sc, rd, perm, m, k0, k1 - k0);
+                else
+                    lu_panel_reg<RP, EXACT>(w, A, ld, piv, sc, rd, perm, m, k0, k1 - k0);
+            }
             g.sync();
             GF_PH_END(g, PH_LU_PANEL)
         }
@@ -1743,7 +1749,12 @@ __device__ __forceinline__ void lu_solve_any(const Grp<G>& g, const W& w, int A,
         if (m <= 64) {
             g.sync();
             GF_PH_BEGIN(g)
-            if (G == 32 || g.lane < 32) lu_solve_warp<2>(w, A, ld, perm, rdiag, m, b);
+            if (G == 32 || g.lane < 32) {
+                if (m <= 32)
+                    lu_solve_warp<1>(w, A, ld, perm, rdiag, m, b);
+                else
+                    lu_solve_warp<2>(w, A, ld, perm, rdiag, m, b);
+            }
             g.sync();
             GF_PH_END(g, PH_SOLVE)
             return;
@@ -1776,7 +1787,9 @@ __device__ __forceinline__ void lu_factor(const Grp<G>& g, const W& w, int A, in
     if constexpr (G >= 32) {
         if (m <= 128) {
             GF_PH_BEGIN(g)
-            if (m <= 64)
+            if (m <= 32)
+                lu_decompose_mma<G, 1, EXACT>(g, w, A, ld, piv, sc, rd, perm, m);
+            else if (m <= 64)
                 lu_decompose_mma<G, 2, EXACT>(g, w, A, ld, piv, sc, rd, perm, m);
             else
                 lu_decompose_mma<G, 4, EXACT>(g, w, A, ld, piv, sc, rd, perm, m);
@@ -2009,7 +2022,7 @@ __device__ __forceinline__ int ode_solve(const Grp<G>& g, const DevMech& M, cons
     double step_dxTry = *dxTry;
     bool last = false;
     double x = xStart;
-    const double inc_threshold = real_pow(o.maxScale / o.safeScale, -1.0 / o.alphaInc);
+    const double inc_threshold = pow(o.maxScale / o.safeScale, -1.0 / o.alphaInc);
     for (int nStep = 0; nStep < o.maxSteps; nStep++) {
         const double dxTry0 = step_dxTry;
         if ((x + step_dxTry - xEnd) * (x + step_dxTry - xStart) > 0) {
@@ -2027,7 +2040,7 @@ __device__ __forceinline__ int ode_solve(const Grp<G>& g, const DevMech& M, cons
             GF_PH_END(g, PH_ATTEMPT)
             ++*attempts;
             if (err > 1) {
-                const double scale = fmax(o.safeScale * real_pow(err, -o.alphaDec), o.minScale);
+                const double scale = fmax(o.safeScale * pow(err, -o.alphaDec), o.minScale);
                 dx *= scale;
                 // the reference traps here (gpuAdaptiveSolver.H:111-114); the cap
                 // also ends the loop for step controls that never shrink dx
@@ -2046,7 +2059,7 @@ __device__ __forceinline__ int ode_solve(const Grp<G>& g, const DevMech& M, cons
         *y_off = *yt_off;
         *yt_off = t;
         if (err > inc_threshold) {
-            step_dxTry = fmin(fmax(o.safeScale * real_pow(err, -o.alphaInc), o.minScale), o.maxScale) * dx;
+            step_dxTry = fmin(fmax(o.safeScale * pow(err, -o.alphaInc), o.minScale), o.maxScale) * dx;
         } else {
             step_dxTry = o.safeScale * o.maxScale * dx;
         }
