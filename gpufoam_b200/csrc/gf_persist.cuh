@@ -84,7 +84,23 @@ __global__ void __maxnreg__(PersistShape<G>::max_regs(SLIM))
         }
         const DevMech& M = *Mp;
         if (SHARED) {
-            process_cell<G, WsC, false, NB, MS>(g, M, WsC{smem + (size_t)gib * ws_per_cell}, a, (int)cell);
+            const WsC w{smem + (size_t)gib * ws_per_cell};
+            // 256 threads per cell, one CTA per SM: the form of launches that mix
+            // mechanisms. Each of the known sizes has its own code in this kernel
+            // (fixed offsets, bounds and tiles, as in the tuned variants): 2,250
+            // cells of 10, 53 and 100 species 131.7 -> 123.6 ms. With several
+            // CTAs per SM their instructions would compete for the caches.
+            if constexpr (G == 256 && SLIM == 0 && MS == 0) {
+                if (M.m == 54) {
+                    process_cell<G, WsC, false, NB, 54>(g, M, w, a, (int)cell);
+                    continue;
+                }
+                if (M.m == 101) {
+                    process_cell<G, WsC, false, NB, 101>(g, M, w, a, (int)cell);
+                    continue;
+                }
+            }
+            process_cell<G, WsC, false, NB, MS>(g, M, w, a, (int)cell);
         } else if (G == 1) {
             process_cell<G, WsS, false, NB, MS>(g, M, WsS{a.ws + slot, n_slots}, a, (int)cell);
         } else {
