@@ -64,9 +64,16 @@ __global__ void __launch_bounds__(32) rates_kernel(const DevMech M, const double
 // One state per CTA of G threads (a warp for small systems; four warps share the
 // reactions, gathers and rows of a larger one: with one warp and 47 KB per state
 // an SM had four warps in flight, 577 us for 4,096 states of 53 species).
-template <int G>
-__global__ void __launch_bounds__(G, 512 / G) jacobian_kernel(const DevMech M, const double* y, double* dfdx, double* J) {
+// MS: the matrix size fixed at compile time, or 0.
+template <int G, int MS>
+__global__ void __launch_bounds__(G, 512 / G)
+    jacobian_kernel(const DevMech Mp, const double* y, double* dfdx, double* J) {
     extern __shared__ double smem[];
+    DevMech M = Mp;
+    if constexpr (MS > 0) {
+        M.m = MS;
+        M.nS = MS - 1;
+    }
     Grp<G> g;
     const WsLayout L = make_layout(M.nS, M.nR, M.n_slots, M.n_tb);
     const int n = M.nS + 2;
@@ -338,14 +345,15 @@ int launch_jacobian(const DevMech& m, int n, const double* y, double* dfdx, doub
     if (n <= 0) return 0;
     const size_t smem = (size_t)ws_layout(m).size * sizeof(double);
     const int G = m.m <= 32 ? 32 : 128;
-    const void* fn = G == 32 ? reinterpret_cast<const void*>(&jacobian_kernel<32>)
-                             : reinterpret_cast<const void*>(&jacobian_kernel<128>);
+    void (*fn)(const DevMech, const double*, double*, double*) =
+        m.m == 11    ? jacobian_kernel<32, 11>
+        : m.m <= 32  ? jacobian_kernel<32, 0>
+        : m.m == 54  ? jacobian_kernel<128, 54>
+        : m.m == 101 ? jacobian_kernel<128, 101>
+                     : jacobian_kernel<128, 0>;
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    if (G == 32)
-        jacobian_kernel<32><<<n, 32, smem, reinterpret_cast<cudaStream_t>(stream)>>>(m, y, dfdx, J);
-    else
-        jacobian_kernel<128><<<n, 128, smem, reinterpret_cast<cudaStream_t>(stream)>>>(m, y, dfdx, J);
+    fn<<<n, G, smem, reinterpret_cast<cudaStream_t>(stream)>>>(m, y, dfdx, J);
     return (int)cudaGetLastError();
 }
 
