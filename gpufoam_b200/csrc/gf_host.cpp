@@ -238,11 +238,12 @@ int ensure_ws(gf_solver* s, size_t bytes) {
 // this on a sample of cells). Measured on the B200, 64 threads per cell (two
 // warps, any m) against the rule:
 //  * m <= 32: a warp per cell, four cells per CTA; a second warp has no rows or
-//    reactions to work on. 65,536 cells of 10 species 148 -> 63 ms;
+//    reactions to work on. 65,536 cells of 10 species 148 -> 63 ms (46 ms since);
 //  * m <= 64: 128 threads and 128 registers; four cells per SM by registers,
 //    the other three warps shorten the reaction loops and gathers, and the rest
-//    of the SM's memory is L1 for the tables. 16,384 cells of 53 species
-//    224 -> 153 ms (96 threads: 139 ms there, but 5 % behind on 64k cells);
+//    of the SM's memory is L1 for the tables. 6,007 cells of 53 species,
+//    Rosenbrock23: 104 -> 73 ms (96 / 64 threads with the kernel compiled for m:
+//    1 % and 6 % slower over 400 .. 65,536 cells);
 //  * m <= 128: 256 threads; shared memory holds one cell per SM, and only its own
 //    threads hide its latency. 701 cells of 100 species 55 -> 31 ms;
 //  * larger ones, and workspaces in HBM: 64 threads.

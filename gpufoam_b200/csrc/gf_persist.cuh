@@ -54,12 +54,13 @@ __device__ __forceinline__ void reject_cell(const Grp<G>& g, const LaunchArgs& a
 }
 
 // Registers per thread the kernel is compiled for: SLIM = 1, at most 128
-// (512 resident threads per SM); otherwise up to 255, except for 64 threads
-// per cell, capped at 200 so that five 64-thread CTAs fit an SM's registers
+// (512 resident threads per SM); SLIM = 2 (a warp per cell, more cells than are
+// resident otherwise), at most 168: twelve warps per SM instead of eight;
+// otherwise up to 255, except for 64 threads per cell, capped at 200 so that five 64-thread CTAs fit an SM's registers
 // (their workspaces fit its shared memory: 45 KB each at 53 species).
 template <int G>
 struct PersistShape {
-    static constexpr int max_regs(int slim) { return slim ? 128 : (G == 64 ? 200 : 255); }
+    static constexpr int max_regs(int slim) { return slim == 2 ? 168 : (slim ? 128 : (G == 64 ? 200 : 255)); }
 };
 
 // NB: columns per LU panel of the blocked form (groups of less than 32 threads, m > 128); MS > 0: the matrix size m of every mechanism of
@@ -158,6 +159,8 @@ const void* persistent_fn_g4(bool shared, int slim);
 const void* persistent_fn_g8(bool shared, int slim);
 const void* persistent_fn_g16(bool shared, int slim);
 const void* persistent_fn_g32(bool shared, int slim);
+// a warp per cell with at most 168 registers, workspace in shared memory; ms: 11 or 0
+const void* persistent_dense_fn_g32(int ms);
 const void* persistent_fn_g64(bool shared, int slim);
 const void* persistent_fn_g96(bool shared, int slim);
 const void* persistent_fn_g128(bool shared, int slim);
