@@ -606,7 +606,8 @@ int gf_mech_create(const gf_mech_desc* d, gf_mech** out) {
         for (size_t i = 0; i < parts.size(); ++i) part_pos[i] = (int)i;
         dst_t.push_back(build_stream(parts, part_pos, n_slots, G));
         jst_t.push_back(build_stream(je, je_pos, n_slots, G));
-        cst_t.push_back(build_stream(cg, dn_pos, 2 * kSideInline * nRa, G));
+        // the sweep runs with 64 threads
+        cst_t.push_back(G == 64 ? build_stream(cg, dn_pos, 2 * kSideInline * nRa, G) : StreamTables{});
     }
     std::vector<double> effT(eff.size());
     for (int t = 0; t < n_tb; ++t)
