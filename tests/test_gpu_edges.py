@@ -1,0 +1,175 @@
+"""The kernels at the sizes where their paths change, on a B200.
+
+* the factorisation by register panels and matrix tiles (32 or more threads,
+  m <= 128) and the blocked solves, at the edges of panels, tiles, lanes and of
+  the range, against the one-thread blocked form (itself pinned to the reference's
+  factors by test_gpu_lu_forms.py): bit for bit, ties and a zero column included;
+* calculate() / tc() with a lane per cell (8,192 cells and more) against the
+  oracle and against the warp-per-cell form, ragged last tiles included;
+* reactions that the compact record does not hold (non-integer exponents,
+  exponent 3, four species on a side, a third-body row past 4,094);
+* rates clipped by the reaction temperature limits, which the Jacobian does not clip;
+* the default launch form of every range of its rule;
+* Qdot on ragged cell counts and padded rows.
+
+Tolerances are those of the tests of the same quantities (tests/parity.py).
+"""
+import copy
+
+import numpy as np
+import pytest
+
+from gpufoam_b200 import evaluator as E
+from gpufoam_b200 import mechanism as M
+from oracle.oracle import Oracle, ode_inputs
+from tests.parity import (assert_jacobian_close, assert_rates_close, assert_states_close, jacobian_scale, rate_scale,
+                          step_count_agreement)
+from tests.test_gpu_fields import species_scale
+from tests.test_oracle import fixture_mech, load
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch
+    from gpufoam_b200 import build
+    build.build()
+    assert torch.cuda.is_available()
+    return torch
+
+
+def lu_cases(m):
+    rng = np.random.default_rng(m)
+    A = rng.standard_normal((4, m, m))
+    A[1] *= 10.0 ** rng.uniform(-8, 8, (m, 1))                 # rows of very different size
+    A[2] = rng.integers(-2, 3, (m, m)) + 3.0 * np.eye(m)       # exact ties of the pivot rule
+    A[3, :, m // 2] = 0.0                                      # the zero pivot's replacement
+    return A, rng.standard_normal((4, 2, m))
+
+
+@pytest.mark.parametrize("m", [1, 2, 7, 8, 9, 15, 16, 17, 24, 31, 32, 33, 40, 48, 56, 63, 64, 65, 72, 96, 127, 128, 129, 160])
+@pytest.mark.parametrize("exact", [True, False])
+def test_lu_edges(torch, m, exact):
+    A, b = lu_cases(m)
+    LU1, piv1, x1 = (t.cpu().numpy() for t in E.lu_factor_solve(A, b, 1, exact))
+    for G in (32, 64, 96, 128, 256):
+        LU, piv, x = (t.cpu().numpy() for t in E.lu_factor_solve(A, b, G, exact))
+        assert np.array_equal(piv, piv1), (m, G)
+        assert np.array_equal(LU, LU1), (m, G)
+        ok = [0, 2] if m > 1 else [0]
+        scale = np.abs(x1[ok]).max(axis=2, keepdims=True)
+        cond = np.array([np.linalg.cond(A[k]) for k in ok])[:, None, None]
+        assert (np.abs(x - x1)[ok] <= 1e-14 * m * np.maximum(cond, 1.0) * scale).all(), (m, G)
+
+
+LANE_MECHS = {
+    "gri": lambda: fixture_mech(load("grisize")),
+    "coverage": lambda: fixture_mech(load("coverage")),   # fractional exponents, irreversible, Lindemann
+    "yao": lambda: fixture_mech(load("foam_yao")),        # exponent 3, four species on a side
+}
+
+
+@pytest.mark.parametrize("name", list(LANE_MECHS))
+@pytest.mark.parametrize("n", [8192, 8192 + 37])
+def test_lane_per_cell_rates(torch, name, n):
+    raw = LANE_MECHS[name]()
+    mech = E.Mechanism(raw)
+    y = M.make_cells(raw, n, seed=5)
+    rho = np.random.default_rng(6).uniform(0.05, 2.0, n)
+    RR, tc = (t.cpu().numpy() for t in E.cell_rates(mech, rho, y))
+    pick = np.r_[0:40, n - 70:n]
+    o = Oracle(raw, "port")
+    ref_RR, ref_tc = o.cell_fields(rho[pick], y[pick])
+    sc = species_scale(raw, o.rate_parts(rho[pick], y[pick]))
+    assert (np.abs(RR[pick] - ref_RR) <= 1e-12 * sc + 1e-300).all()
+    assert np.allclose(tc[pick], ref_tc, rtol=1e-12, atol=0)
+    RRw, tcw = (t.cpu().numpy() for t in E.cell_rates(mech, rho[pick], y[pick]))   # a warp per cell
+    assert (np.abs(RR[pick] - RRw) <= 2e-12 * sc + 1e-300).all()
+    assert np.allclose(tc[pick], tcw, rtol=2e-12, atol=0)
+
+
+def test_third_body_rows_past_the_record(torch):
+    """4,200 third-body reactions: the rows past 4,094 are not in the compact record."""
+    raw = M.coverage(0)
+    tb = [r for r in raw.reactions if r.rate_type == M.RATE_THIRD_BODY]
+    raw = copy.deepcopy(raw)
+    raw.reactions = raw.reactions + [copy.deepcopy(tb[i % len(tb)]) for i in range(4200)]
+    rng = np.random.default_rng(7)
+    for r in raw.reactions[-200:]:
+        r.efficiencies = rng.uniform(0.5, 12.0, raw.n_species)
+    mech = E.Mechanism(raw)
+    n = 8192
+    y = M.make_cells(raw, n, seed=8)
+    rho = rng.uniform(0.05, 2.0, n)
+    RR, tc = (t.cpu().numpy() for t in E.cell_rates(mech, rho, y))
+    o = Oracle(raw, "port")
+    ref_RR, ref_tc = o.cell_fields(rho[-8:], y[-8:])
+    sc = species_scale(raw, o.rate_parts(rho[-8:], y[-8:]))
+    assert (np.abs(RR[-8:] - ref_RR) <= 1e-12 * sc + 1e-300).all()
+    assert np.allclose(tc[-8:], ref_tc, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("limits", [(0.0, 1500.0), (1600.0, 3000.0)])
+def test_clipped_rates(torch, limits):
+    raw = M.make_mechanism(12, 14, 3, 2, seed=0, n_lindemann=2, n_irreversible=3, n_fractional=2, rxn_Tlow=limits[0],
+                           rxn_Thigh=limits[1])
+    mech = E.Mechanism(raw)
+    y = M.make_cells(raw, 24, seed=9, T_range=(1200.0, 2200.0))
+    o = Oracle(raw, "port")
+    assert_rates_close(E.rates(mech, y).cpu().numpy(), o.derivatives(y), rate_scale(raw, y))
+    dfdx, J = E.jacobian(mech, y)
+    ref_f, ref_J = o.jacobian(y)
+    assert_rates_close(dfdx.cpu().numpy(), ref_f, rate_scale(raw, y))
+    assert_jacobian_close(J.cpu().numpy(), ref_J, jacobian_scale(raw, y))
+    ref = o.cells(ode_inputs(34), y, 1e-6, 1e-7)
+    s = E.Solver([mech], E.OdeInputs("Rosenbrock34", absTol=1e-8, relTol=1e-4))
+    dtc = torch.full((24,), 1e-7, dtype=torch.float64, device="cuda")
+    out = s.solve(torch.as_tensor(y, device="cuda"), 1e-6, dtc)
+    assert np.array_equal(out["status"].cpu().numpy(), ref[3])
+    assert_states_close(out["Ynew"].cpu().numpy(), ref[0], raw.n_species, 1e-4)
+    assert step_count_agreement(out["counters"].cpu().numpy(), ref[2]) >= 0.99
+
+
+DEFAULTS = [(M.h2_size, 32, 1), (M.coverage, 32, 0), (M.gri_size, 128, 1), (M.large, 256, 0)]
+
+
+@pytest.mark.parametrize("factory, threads, specialize", DEFAULTS)
+def test_default_launch(torch, factory, threads, specialize):
+    raw = factory(0)
+    s = E.Solver([E.Mechanism(raw)], E.OdeInputs("Rosenbrock34", absTol=1e-8, relTol=1e-4))
+    cfg = s.get_launch()
+    assert cfg["kind"] == 1 and cfg["threads_per_cell"] == threads and cfg["specialize"] == specialize
+    n = 37
+    cells = M.make_cells(raw, n, seed=10)
+    dT = 1e-5 if raw.n_species <= 12 else 1e-6
+    ref = Oracle(raw, "port").cells(ode_inputs(34), cells, dT, 1e-7)
+    dtc = torch.full((n,), 1e-7, dtype=torch.float64, device="cuda")
+    out = s.solve(torch.as_tensor(cells, device="cuda"), dT, dtc)
+    st = out["status"].cpu().numpy()
+    assert np.array_equal(st, ref[3])
+    ok = st == 0
+    assert_states_close(out["Ynew"].cpu().numpy()[ok], ref[0][ok], raw.n_species, 1e-4)
+    assert step_count_agreement(out["counters"].cpu().numpy(), ref[2]) >= 0.99
+
+
+def test_jacobian_of_100_species(torch):
+    raw = M.large(0)
+    y = M.make_cells(raw, 2, seed=11)
+    dfdx, J = E.jacobian(E.Mechanism(raw), y)
+    ref_f, ref_J = Oracle(raw, "port").jacobian(y)
+    assert_rates_close(dfdx.cpu().numpy(), ref_f, rate_scale(raw, y))
+    assert_jacobian_close(J.cpu().numpy(), ref_J, jacobian_scale(raw, y))
+
+
+@pytest.mark.parametrize("n, pad", [(1, 0), (31, 3), (32, 0), (33, 1), (129, 0), (4099, 2)])
+@pytest.mark.parametrize("factory", [M.h2_size, M.gri_size, M.large])
+def test_qdot_ragged(torch, factory, n, pad):
+    raw = factory(0)
+    mech = E.Mechanism(raw)
+    RR = np.random.default_rng(n).standard_normal((n, raw.n_species + pad))
+    q = np.zeros(n)
+    hf = -E.qdot(mech, np.eye(raw.n_species)).cpu().numpy()   # one species at a time: 0 - hf_i
+    for i in range(raw.n_species):
+        q = q - hf[i] * RR[:, i]
+    assert np.array_equal(E.qdot(mech, RR).cpu().numpy(), q)
