@@ -148,10 +148,14 @@ typedef struct gf_launch_config {
     int cells_per_block;     /* groups per CTA (persistent, threads_per_cell <= 32;
                                 CTAs have at most 128 threads)                   */
     int blocks_per_sm;       /* 0 = as many as fit                               */
-    int register_budget;     /* persistent only: 0 = up to 255 registers per thread,
-                                1 = at most 128 (more resident cell groups)      */
+    int register_budget;     /* persistent only: 0 = up to 255 registers per thread
+                                (32 threads per cell: 168 when more cells come than
+                                are resident with 255), 1 = at most 128 (more
+                                resident cell groups)                            */
     int lu_panel;            /* persistent, 32/64/96/128 threads per cell: columns per LU
-                                panel, 4, 8 or 16 (0 = 8; see gf_solver_set_launch) */
+                                panel of the blocked factorisation (matrices larger
+                                than 128), 4, 8 or 16 (0 = 8; see
+                                gf_solver_set_launch)                            */
     int specialize;          /* persistent, 32/64/96/128 threads per cell: 1 = the kernel
                                 compiled for the matrix size of the solver's
                                 mechanisms (10, 53 or 100 species; all the same)  */
@@ -197,6 +201,9 @@ void gf_solver_destroy(gf_solver* solver);
  * 128 threads and 0 otherwise; without specialize, lu_panel 4/16 needs
  * scratch_in_shared; specialize needs a solver whose mechanisms share 10, 53 or
  * 100 species, with lu_panel 8 (or 0), or 4 for 53 species. */
+/* Without a call to it: persistent, by the largest matrix of the solver's
+ * mechanisms 32, 128 or 256 threads per cell (to 32, 64 and 128 unknowns; 64
+ * beyond, or with the workspace in HBM), specialised where compiled. */
 int gf_solver_set_launch(gf_solver* solver, const gf_launch_config* cfg);
 int gf_solver_get_launch(const gf_solver* solver, gf_launch_config* cfg);
 /* The per-cell workspace of the solve kernels (doubles: in shared memory or
