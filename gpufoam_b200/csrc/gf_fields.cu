@@ -165,8 +165,9 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
 // shared memory, species by species over the lanes (stride 33: the transposes in
 // and out are free of bank conflicts too). Per species the order of the
 // reference's sum inside a warp's reactions, then the warps in order. Bound by
-// instructions issued: some 220 per reaction and 32 cells, where a warp per cell
-// took 415 per 32 reactions of one cell and the gather besides.
+// instructions: some 500 per reaction and 32 cells, at twelve warps per SM, where
+// a warp per cell took 415 per 32 reactions of one cell and the gather besides.
+// 60,000 cells of 53 species: 1028 -> 813 us.
 constexpr int kLaneStride = 33;
 
 // A value per species of one lane's cell.
