@@ -883,11 +883,11 @@ __device__ __forceinline__ void jacobian(const Grp<G>& g, const DevMech& M, cons
     stream_gather<4>(g, M.jst[stream_index(G)], w, L.stage, w, L.J);
     g.sync();
     // phase 3: a thread per row and, where the group has more threads than
-    // rows, per part of its columns
+    // rows, per part of its columns (a part may be empty: it still leaves its sum)
     const int rows = (nS + 31) & ~31, parts = min(2, max(1, G / rows));
     const int part = G > 32 ? g.lane / rows : 0;
-    const int c0 = part < parts ? part * nS / parts : nS, c1 = part < parts ? (part + 1) * nS / parts : nS;
-    for (int s = G > 32 ? g.lane - part * rows : g.lane; s < nS && c0 < c1; s += parts > 1 ? rows : G) {
+    const int c0 = part * nS / parts, c1 = (part + 1) * nS / parts;
+    for (int s = G > 32 ? g.lane - part * rows : g.lane; s < nS && part < parts; s += parts > 1 ? rows : G) {
         const double Ws = ldg(M.W + s);
         const double dfs = w[L.dfdx + s];
         const int row = L.J + s * ld;

@@ -173,3 +173,25 @@ def test_qdot_ragged(torch, factory, n, pad):
     for i in range(raw.n_species):
         q = q - hf[i] * RR[:, i]
     assert np.array_equal(E.qdot(mech, RR).cpu().numpy(), q)
+
+
+@pytest.mark.parametrize("solver", [12, 23, 34])
+def test_one_species(torch, solver):
+    """One species, A -> 1.05 A (no net zero to hide behind): a group of 64 or more threads
+    splits the Jacobian row's single column into an empty part and the rest."""
+    a = np.array([[3.5, 1e-3, -2e-7, 1e-11, 0.0, -3e4, 4.0]])
+    raw = M.RawMechanism("one-species", ["A"], np.array([1.0]), np.array([200.0]), np.array([5000.0]),
+                         np.array([1000.0]), a, a, [M.RawReaction(M.RATE_ARRHENIUS, True, [(0, 1.0, 1.0)],
+                                                                  [(0, 1.05, 1.0)], 1e6, 0.5, 9e3)])
+    n = 16
+    cells = M.make_cells(raw, n, seed=12, T_range=(1200.0, 2200.0))
+    ref = Oracle(raw, "port").cells(ode_inputs(solver), cells, 1e-6, 1e-8)
+    s = E.Solver([E.Mechanism(raw)], E.OdeInputs(f"Rosenbrock{solver}", absTol=1e-8, relTol=1e-4))
+    for G in (8, 32, 64, 96, 128, 256):
+        s.set_launch(kind=1, threads_per_cell=G, scratch_in_shared=1)
+        dtc = torch.full((n,), 1e-8, dtype=torch.float64, device="cuda")
+        out = s.solve(torch.as_tensor(cells, device="cuda"), 1e-6, dtc)
+        assert np.array_equal(out["status"].cpu().numpy(), ref[3]), G
+        assert np.array_equal(out["counters"].cpu().numpy(), ref[2]), G
+        # the same steps: rounding only, amplified at most by the steps' number and a stiffness of order one
+        assert np.allclose(out["Ynew"].cpu().numpy(), ref[0], rtol=1e-10, atol=0), G
