@@ -793,9 +793,10 @@ int launch_record(const DevMech& M, const LaunchArgs& a, void* stream) {
     const int smem = make_layout(M.nS, M.nR, M.n_slots, M.n_tb).size * (int)sizeof(double);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
     const RecordFn fn = record_fn(M.m);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
+    if (e != cudaSuccess) return (int)e;
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, smem);
     if (e != cudaSuccess) return (int)e;
     if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
     launch_epilogue_reset(a.queue, stream);
@@ -820,7 +821,7 @@ int adjoint_blocks_per_sm(const DevMech& M) {
     const int smem = adjoint_smem_bytes(M);
     if (smem > 227 * 1024) return 0;
     const AdjointFn fn = adjoint_fn(M.m);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem) != cudaSuccess) return 0;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 64, smem) != cudaSuccess) return 0;
     return per_sm;

@@ -104,8 +104,7 @@ int launch_gather_states(int n, int nS, const double* const* Y, const double* T,
     FieldPtrs P{};
     for (int i = 0; i < nS; ++i) P.p[i] = Y[i];
     const size_t smem = (size_t)kTileCells * ((nS + 2) | 1) * sizeof(double);
-    const cudaError_t e = cudaFuncSetAttribute(gather_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&gather_states_kernel), smem);
     if (e != cudaSuccess) return (int)e;
     gather_states_kernel<<<(unsigned)tile_grid(n), kTileThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         P, T, p, n, nS, y, ld);
@@ -117,8 +116,7 @@ int launch_scatter_rates(int n, int nS, const double* RR, int ld, double* const*
     FieldOutPtrs P{};
     for (int i = 0; i < nS; ++i) P.p[i] = out[i];
     const size_t smem = (size_t)kTileCells * (nS | 1) * sizeof(double);
-    const cudaError_t e = cudaFuncSetAttribute(scatter_rates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&scatter_rates_kernel), smem);
     if (e != cudaSuccess) return (int)e;
     scatter_rates_kernel<<<(unsigned)tile_grid(n), kTileThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         RR, ld, n, nS, P);

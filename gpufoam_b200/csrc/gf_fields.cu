@@ -310,7 +310,7 @@ int launch_cell_fields(const DevMech& M, const FieldArgs& a, void* stream) {
         if (bytes(warps) <= 227 * 1024) {
             const size_t smem = bytes(warps);
             const void* fn = reinterpret_cast<const void*>(&cell_lanes_kernel);
-            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaError_t e = allow_dynamic_smem(fn, smem);
             if (e != cudaSuccess) return (int)e;
             int per_sm = 0;
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cell_lanes_kernel, 32 * warps, smem);
@@ -330,8 +330,7 @@ int launch_cell_fields(const DevMech& M, const FieldArgs& a, void* stream) {
     while (cells > 1 && per_cell * cells > (size_t)max_smem) --cells;
     if (per_cell * cells > (size_t)max_smem) return (int)cudaErrorInvalidValue;
     const size_t smem = per_cell * cells;
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&cell_fields_kernel),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&cell_fields_kernel), smem);
     if (e != cudaSuccess) return (int)e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cell_fields_kernel, 32 * cells, smem);
@@ -349,8 +348,7 @@ int launch_qdot(const DevMech& M, int n, const double* RR, int ld_rr, double* qd
     int warps = 4;
     while (warps > 1 && per_warp * warps > 100 * 1024) --warps;
     const size_t smem = per_warp * warps;
-    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&qdot_kernel),
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&qdot_kernel), smem);
     if (e != cudaSuccess) return (int)e;
     const long long grid = std::min<long long>((n + 32LL * warps - 1) / (32LL * warps), 8LL * device_sm_count());
     qdot_kernel<<<(unsigned)grid, 32 * warps, smem, reinterpret_cast<cudaStream_t>(stream)>>>(M, n, RR, ld_rr, qdot);

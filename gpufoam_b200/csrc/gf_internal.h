@@ -2,6 +2,8 @@
 // kernels (gf_kernels.cu). Not part of the public C ABI.
 #pragma once
 
+#include <cuda_runtime_api.h>
+
 #include <cstdint>
 #include <vector>
 
@@ -249,5 +251,12 @@ int specialized_size(const DevMech* mechs, int n_mechs);
 // Whether the library compiles the persistent kernel of this launch form.
 bool persistent_form_compiled(const gf_launch_config& cfg, int ms);
 int device_sm_count();
+// Before a launch of fn with `smem` bytes of dynamic shared memory. The limit on
+// them is an attribute of the function, not of the launch, and a launch above it
+// is refused: so it is always raised to the same value, the most that a block can
+// have beside fn's static part, and no host thread can lower it between another
+// one's call and its launch. The first 40 KB need no attribute (the default limit
+// is 48 KB with the static part, here at most 512 bytes), nor a driver call.
+cudaError_t allow_dynamic_smem(const void* fn, size_t smem);
 
 }  // namespace gf

@@ -162,7 +162,7 @@ template <int G, bool EXACT>
 static int launch_lu_form_g(int n_mats, int m, double* A, int* piv, double* b, int n_rhs, cudaStream_t s) {
     const size_t smem = ((size_t)m * (m | 1) + 5 * (size_t)m) * sizeof(double);
     const void* fn = reinterpret_cast<const void*>(&lu_form_kernel<G, EXACT>);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_dynamic_smem(fn, smem);
     if (e != cudaSuccess) return (int)e;
     lu_form_kernel<G, EXACT><<<n_mats, G < 32 ? 32 : G, smem, s>>>(m, A, piv, b, n_rhs);
     return (int)cudaGetLastError();
@@ -201,6 +201,16 @@ int device_sm_count() {
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     return n;
+}
+
+cudaError_t allow_dynamic_smem(const void* fn, size_t smem) {
+    if (smem <= 40 * 1024) return cudaSuccess;
+    cudaFuncAttributes fa{};
+    const cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    const size_t limit = 227 * 1024 - fa.sharedSizeBytes;
+    if (smem > limit) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
 }
 
 // The matrix size the tuned kernels are compiled for when every mechanism of a
@@ -268,7 +278,7 @@ static int slots_of(const void* fn, const gf_launch_config& cfg, int smem_bytes_
         smem = (size_t)cpb * smem_bytes_per_cell;
         if (smem > 227 * 1024) return -2;
     }
-    if (shared) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (allow_dynamic_smem(fn, smem) != cudaSuccess) return -3;
     // shared-memory carveout: just enough for the CTAs that are resident
     // (blocks_per_sm, or as many as registers, threads and shared memory allow
     // at the largest carveout), so that the rest of the SM's 256 KB serves as
@@ -355,8 +365,8 @@ int launch_cells(const DevMech* mechs, int n_mechs, const gf_launch_config& cfg,
 int launch_rates(const DevMech& m, int n, const double* y, double* dydx, void* stream) {
     if (n <= 0) return 0;
     const size_t smem = (size_t)ws_layout(m).size * sizeof(double);
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(&rates_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&rates_kernel), smem);
+    if (e != cudaSuccess) return (int)e;
     rates_kernel<<<n, 32, smem, reinterpret_cast<cudaStream_t>(stream)>>>(m, y, dydx);
     return (int)cudaGetLastError();
 }
@@ -372,7 +382,7 @@ int launch_jacobian(const DevMech& m, int n, const double* y, double* dfdx, doub
         : m.m == 54  ? jacobian_kernel<128, 54>
         : m.m == 101 ? jacobian_kernel<128, 101>
                      : jacobian_kernel<128, 0>;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (e != cudaSuccess) return (int)e;
     fn<<<n, G, smem, reinterpret_cast<cudaStream_t>(stream)>>>(m, y, dfdx, J);
     return (int)cudaGetLastError();
@@ -381,8 +391,8 @@ int launch_jacobian(const DevMech& m, int n, const double* y, double* dfdx, doub
 int launch_lu(int n_mats, int m, double* A, int* piv, double* /*vv*/, void* stream) {
     if (n_mats <= 0) return 0;
     const size_t smem = ((size_t)m * (m | 1) + 2 * m) * sizeof(double);
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(&lu_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&lu_kernel), smem);
+    if (e != cudaSuccess) return (int)e;
     lu_kernel<<<n_mats, 32, smem, reinterpret_cast<cudaStream_t>(stream)>>>(m, A, piv);
     return (int)cudaGetLastError();
 }
@@ -390,8 +400,8 @@ int launch_lu(int n_mats, int m, double* A, int* piv, double* /*vv*/, void* stre
 int launch_lusolve(int n_mats, int m, const double* LU, const int* piv, double* b, void* stream) {
     if (n_mats <= 0) return 0;
     const size_t smem = ((size_t)m * (m | 1) + 2 * m) * sizeof(double);
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(&lusolve_kernel),
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&lusolve_kernel), smem);
+    if (e != cudaSuccess) return (int)e;
     lusolve_kernel<<<n_mats, 32, smem, reinterpret_cast<cudaStream_t>(stream)>>>(m, LU, piv, b);
     return (int)cudaGetLastError();
 }

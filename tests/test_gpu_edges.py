@@ -15,6 +15,9 @@
 Tolerances are those of the tests of the same quantities (tests/parity.py).
 """
 import copy
+import ctypes as C
+import os
+import subprocess
 
 import numpy as np
 import pytest
@@ -195,3 +198,51 @@ def test_one_species(torch, solver):
         assert np.array_equal(out["counters"].cpu().numpy(), ref[2]), G
         # the same steps: rounding only, amplified at most by the steps' number and a stiffness of order one
         assert np.allclose(out["Ynew"].cpu().numpy(), ref[0], rtol=1e-10, atol=0), G
+
+
+HAMMER = r"""
+#include <atomic>
+#include <thread>
+#include "gpufoam_b200.h"
+// two host threads, each launching for its own number of species; the number of refused launches
+extern "C" int hammer(const double* const* fields, double* const* out, const double* T, double* y, int n, int loops,
+                      const int* sizes, const gf_mech* const* mechs, double* q) {
+    std::atomic<int> refused{0};
+    auto work = [&](int k) {
+        for (int i = 0; i < loops; ++i) {
+            refused += gf_gather_states(n, sizes[k], fields, T, T, y, sizes[k] + 2, nullptr) != GF_OK;
+            refused += gf_scatter_rates(n, sizes[k], y, sizes[k], out, nullptr) != GF_OK;
+            refused += gf_qdot(mechs[k], n, y, 100, q, nullptr) != GF_OK;
+        }
+    };
+    std::thread a(work, 0), b(work, 1);
+    a.join();
+    b.join();
+    return refused;
+}
+"""
+
+
+def test_host_threads_with_different_sizes(torch, tmp_path):
+    """The shared memory that one host thread's launches ask for is not taken away by those of
+    another with fewer species (64 cells a launch: the threads meet between setting and launching)."""
+    from gpufoam_b200 import _native as N
+    src, lib = tmp_path / "hammer.cpp", tmp_path / "libhammer.so"
+    src.write_text(HAMMER)
+    pkg = os.path.dirname(N.LIB_PATH)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-pthread", "-I",
+                    os.path.join(os.path.dirname(pkg), "include"), "-o", str(lib), str(src), "-L", pkg,
+                    "-lgpufoam_b200", f"-Wl,-rpath,{pkg}"], check=True, capture_output=True)
+    n, sizes = 64, (300, 200)
+    cols = torch.zeros((300, n), dtype=torch.float64, device="cuda")
+    out = torch.zeros((300, n), dtype=torch.float64, device="cuda")
+    y = torch.zeros((n, 302), dtype=torch.float64, device="cuda")
+    q = torch.zeros(n, dtype=torch.float64, device="cuda")
+    mechs = [E.Mechanism(M.large(0)), E.Mechanism(M.gri_size(0))]
+    ptrs = lambda t: (C.c_void_p * 300)(*[t[i].data_ptr() for i in range(300)])  # noqa: E731
+    torch.cuda.synchronize()
+    refused = C.CDLL(str(lib)).hammer(ptrs(cols), ptrs(out), C.c_void_p(cols.data_ptr()), C.c_void_p(y.data_ptr()),
+                                      n, 4000, (C.c_int * 2)(*sizes), (C.c_void_p * 2)(*[m.handle.value for m in mechs]),
+                                      C.c_void_p(q.data_ptr()))
+    torch.cuda.synchronize()
+    assert refused == 0
