@@ -28,25 +28,32 @@ constexpr int kFieldCellsMax = 4;  // cells (warps) per CTA of the warp-per-cell
 constexpr int kLaneCells = 8192;   // cells from which the lane-per-cell form is the faster one
 
 struct FieldLayout {
-    WsLayout L;  // only c, Mtb and stage are used
-    int out;     // dN/dt of every species
+    WsLayout L;  // only c, Mtb, stage and part are used
+    int out;     // dN/dt of every species (one reaction)
     int size;
 };
 
+// Mechanisms with thousands of reactions fill a block's shared memory with their
+// staging slots, so nothing lies beside them but c, out and the third-body sums:
+//  * the 1 for the absent species of a reaction side is out[0], which takes its
+//    dN/dt only after the rates;
+//  * the 0 for the gather's missing records (behind the last slot) is c[0] and the
+//    parts of dN/dt lie on the rest of c, out and the sums: all free by then. There are at
+//    most max(nS, 32) parts for a warp, or 2 m for few species.
 __host__ __device__ inline FieldLayout field_layout(const DevMech& M) {
     FieldLayout F{};
     int o = 0;
-    F.L.c = o;
-    o += M.nS + 1;  // and a 1 for the absent species of a reaction side
-    F.L.Mtb = o;
-    o += M.n_tb > 0 ? M.n_tb : 1;
     F.L.stage = o;
-    o += M.n_slots + 1;  // and a 0 for the gather's missing records
-    F.L.part = o;
-    o += 2 * M.m;
+    o += M.n_slots;
+    F.L.c = o;
+    F.L.part = o + 1;
+    o += M.nS;
     F.out = o;
     o += M.nS;
-    F.size = o;
+    F.L.Mtb = o;
+    o += M.n_tb > 0 ? M.n_tb : 1;
+    const int parts = M.nS >= 32 ? M.nS : (2 * M.m < 32 ? 2 * M.m : 32);
+    F.size = o > F.L.part + parts ? o : F.L.part + parts;
     return F;
 }
 
@@ -88,7 +95,6 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
     const int warp = threadIdx.x >> 5;
     WsC w{smem + (size_t)warp * F.size};
     const int nS = M.nS;
-    if (g.lane == 0) w[F.L.stage + M.n_slots] = 0.0;
     for (long long cell = (long long)blockIdx.x * per_cta + warp; cell < a.n_cells;
          cell += (long long)gridDim.x * per_cta) {
         const double* y = a.y + cell * a.ld_y;
@@ -99,7 +105,7 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
             w[F.L.c + i] = ci;
             csum += ci;
         }
-        if (g.lane == 0) w[F.L.c + nS] = 1.0;
+        if (g.lane == 0) w[F.out] = 1.0;  // c[nS]
         g.sync();
         if (M.n_tb > 0) {
             third_body_all(g, M, w, F.L.c, F.L.Mtb);
@@ -111,7 +117,7 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
             // reactionRR / specieReactionRR: one reaction, lane 0
             double* rr = a.RR ? a.RR + cell * a.ld_rr : nullptr;
             if (rr)
-                for (int i = g.lane; i < nS; i += 32) w[F.out + i] = 0.0;
+                for (int i = 1 + g.lane; i < nS; i += 32) w[F.out + i] = 0.0;
             g.sync();
             if (g.lane == 0) {
                 const int q = a.reaction_q;
@@ -122,6 +128,7 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
                 const double om = kf * fast_C(M, w, F.L.c, R, q, 0) - kr * fast_C(M, w, F.L.c, R, q, 1);
                 if (a.omega) a.omega[cell] = om;
                 if (rr) {
+                    w[F.out] = 0.0;
                     // gpuReaction::dNdtByV (gpuReaction.H:490-508): lhs, then rhs
                     const int b0 = ldg(M.sp_off + q);
                     for (int e = 0; e < R.nl(); ++e) {
@@ -144,6 +151,8 @@ __global__ void __launch_bounds__(32 * kFieldCellsMax) cell_fields_kernel(const 
         stage_fields(g, M, w, F.L, tcache, a.tc != nullptr, &sW, &sW2);
         g.sync();
         if (a.RR) {
+            if (g.lane == 0) w[F.L.stage + M.n_slots] = 0.0;  // c[0]
+            g.sync();
             stream_gather(g, M.dst[stream_index(32)], w, F.L.stage, w, F.L.part);
             g.sync();
             const int* part = M.dst_part[stream_index(32)];

@@ -246,3 +246,72 @@ def test_host_threads_with_different_sizes(torch, tmp_path):
                                       C.c_void_p(q.data_ptr()))
     torch.cuda.synchronize()
     assert refused == 0
+
+
+def filled(raw, doubles):
+    """raw with its reactions repeated until a cell of calculate() takes `doubles` of shared memory:
+    the staging slots, twice the species, the third-body sums."""
+    raw = copy.deepcopy(raw)
+    cost = lambda r: (2 + len(r.lhs) + len(r.rhs) + (r.rate_type == M.RATE_THIRD_BODY)  # noqa: E731
+                      + (r.rate_type != M.RATE_ARRHENIUS))
+    base = list(raw.reactions)
+    left = doubles - 2 * raw.n_species - sum(cost(r) for r in base)
+    small, large = (next(r for r in base if cost(r) == k) for k in (5, 6))
+    k = 0
+    while left > 60:
+        raw.reactions.append(copy.deepcopy(base[k % len(base)]))
+        left -= cost(base[k % len(base)])
+        k += 1
+    n6 = left % 5
+    for r in [large] * n6 + [small] * ((left - 6 * n6) // 5):
+        raw.reactions.append(copy.deepcopy(r))
+    assert 2 * raw.n_species + sum(cost(r) for r in raw.reactions) == doubles
+    return raw
+
+
+@pytest.mark.parametrize("factory", [M.h2_size, M.coverage, M.gri_size])
+@pytest.mark.parametrize("less", [0, 1, 2])
+def test_rates_that_just_fit(torch, factory, less):
+    """As many reactions as a block's 227 KB of shared memory hold: a warp per cell takes them, and the
+    places that a cell uses twice do not meet. Also every single-reaction rate of a few reactions."""
+    raw = filled(factory(0), 227 * 1024 // 8 - less)
+    mech = E.Mechanism(raw)
+    n = 5
+    y = M.make_cells(raw, n, seed=14)
+    rho = np.random.default_rng(15).uniform(0.05, 2.0, n)
+    o = Oracle(raw, "port")
+    ref_RR, ref_tc = o.cell_fields(rho, y)
+    parts = o.rate_parts(rho, y)
+    RR, tc = (t.cpu().numpy() for t in E.cell_rates(mech, rho, y))
+    assert (np.abs(RR - ref_RR) <= 1e-12 * species_scale(raw, parts) + 1e-300).all()
+    assert np.allclose(tc, ref_tc, rtol=1e-12, atol=0)
+    for r in (0, 7, raw.n_reactions - 1):
+        om, RR1 = (t.cpu().numpy() for t in E.reaction_rates(mech, r, rho, y))
+        ref_om, ref_RR1 = o.reaction_fields(r, rho, y)
+        gross = np.abs(parts[:, r]).sum(axis=1)
+        assert (np.abs(om - ref_om) <= 1e-12 * gross + 1e-300).all(), r
+        sc = np.zeros((n, raw.n_species))
+        for i, st, _ in raw.reactions[r].lhs + raw.reactions[r].rhs:
+            sc[:, i] += abs(st) * gross * raw.W[i]
+        assert (np.abs(RR1 - ref_RR1) <= 1e-12 * sc + 1e-300).all(), r
+
+
+@pytest.mark.parametrize("name", list(LANE_MECHS))
+def test_single_reaction_rates(torch, name):
+    """reactionRR / specieReactionRR of every reaction against the port, general reactions included."""
+    raw = LANE_MECHS[name]()
+    mech = E.Mechanism(raw)
+    n = 9
+    y = M.make_cells(raw, n, seed=16)
+    rho = np.random.default_rng(17).uniform(0.05, 2.0, n)
+    o = Oracle(raw, "port")
+    parts = o.rate_parts(rho, y)
+    for r, rx in enumerate(raw.reactions):
+        om, RR = (t.cpu().numpy() for t in E.reaction_rates(mech, r, rho, y))
+        ref_om, ref_RR = o.reaction_fields(r, rho, y)
+        gross = np.abs(parts[:, r]).sum(axis=1)
+        assert (np.abs(om - ref_om) <= 1e-12 * gross + 1e-300).all(), r
+        sc = np.zeros((n, raw.n_species))
+        for i, st, _ in rx.lhs + rx.rhs:
+            sc[:, i] += abs(st) * gross * raw.W[i]
+        assert (np.abs(RR - ref_RR) <= 1e-12 * sc + 1e-300).all(), r
