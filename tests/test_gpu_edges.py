@@ -315,3 +315,39 @@ def test_single_reaction_rates(torch, name):
         for i, st, _ in rx.lhs + rx.rhs:
             sc[:, i] += abs(st) * gross * raw.W[i]
         assert (np.abs(RR - ref_RR) <= 1e-12 * sc + 1e-300).all(), r
+
+
+def widened(raw, n_species):
+    """raw with copies of its species (before the last, inert one); every other reaction takes the copies."""
+    raw = copy.deepcopy(raw)
+    b, k = raw.n_species, n_species - raw.n_species
+    assert 0 <= k < b
+    ix = np.r_[0:b - 1, np.arange(k), b - 1]
+    raw.species = [raw.species[i] + ("" if j < b - 1 or j == n_species - 1 else "_copy") for j, i in enumerate(ix)]
+    for f in ("W", "Tlow", "Thigh", "Tcommon", "high_raw", "low_raw"):
+        setattr(raw, f, getattr(raw, f)[ix])
+    for j, r in enumerate(raw.reactions):
+        if r.efficiencies is not None:
+            r.efficiencies = r.efficiencies[ix]
+        move = lambda i: n_species - 1 if i == b - 1 else (b - 1 + i if j % 2 and i < k else i)  # noqa: E731
+        r.lhs = [(move(i), st, e) for i, st, e in r.lhs]
+        r.rhs = [(move(i), st, e) for i, st, e in r.rhs]
+    return raw
+
+
+@pytest.mark.parametrize("n_species", [144, 145, 300])
+def test_rates_of_many_species(torch, n_species):
+    """calculate() and tc() on 8,192 + 5 cells where the lane-per-cell form has two warps (144 species)
+    and where a warp per cell takes over, to the largest number of species."""
+    raw = widened(M.make_mechanism(min(n_species, 151), 300, 60, 40, seed=1), n_species)
+    mech = E.Mechanism(raw)
+    n = 8192 + 5
+    y = M.make_cells(raw, n, seed=18)
+    rho = np.random.default_rng(19).uniform(0.05, 2.0, n)
+    RR, tc = (t.cpu().numpy() for t in E.cell_rates(mech, rho, y))
+    pick = np.r_[0:33, n - 9:n]
+    o = Oracle(raw, "port")
+    ref_RR, ref_tc = o.cell_fields(rho[pick], y[pick])
+    sc = species_scale(raw, o.rate_parts(rho[pick], y[pick]))
+    assert (np.abs(RR[pick] - ref_RR) <= 1e-12 * sc + 1e-300).all()
+    assert np.allclose(tc[pick], ref_tc, rtol=1e-12, atol=0)
