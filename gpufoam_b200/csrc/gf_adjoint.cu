@@ -52,8 +52,9 @@ enum { MS_RHO = 0, MS_CPM, MS_DCPM, MS_AV, MS_RHOB, MS_CPMB, MS_DCPMB, MS_AVB, M
 // y2, y3, fs, f2 and f3 live in the forward workspace (shared memory), after
 // its make_layout part (fwd_size doubles in all); every other array is in the
 // per-CTA adjoint region in global memory, offsets from 0.
-__host__ __device__ inline AdjLayout make_adj_layout(const WsLayout& L, int nS, int nR, int n_tb, int* fwd_size) {
-    const int m = nS + 1;
+__host__ __device__ inline AdjLayout make_adj_layout(const WsLayout& L, int nS, int nR, int n_tb, int* fwd_size,
+                                                    int pad) {
+    const int m = nS + 1, v = pad ? pad : m;
     AdjLayout A;
     A.y2 = L.size;
     A.y3 = L.size + m;
@@ -62,24 +63,24 @@ __host__ __device__ inline AdjLayout make_adj_layout(const WsLayout& L, int nS, 
     A.f3 = L.size + 4 * m;
     *fwd_size = L.size + 5 * m;
     int o = 0;
-    A.rb = o; o += 4 * m;
-    A.kb = o; o += 4 * m;
-    A.yb = o; o += m;
-    A.fb0 = o; o += m;
-    A.fb2 = o; o += m;
-    A.fb3 = o; o += m;
+    A.rb = o; o += 4 * v;
+    A.kb = o; o += 4 * v;
+    A.yb = o; o += v;
+    A.fb0 = o; o += v;
+    A.fb2 = o; o += v;
+    A.fb3 = o; o += v;
+    A.dfc = o; o += v;                // dfdx of the converted Jacobian
+    A.cb = o; o += v;
+    A.ms = o; o += MS_N;
+    A.vb = o; o += 4 * v;            // Cp, Ha, rhoM/W, v adjoints
+    A.dn = o; o += v;                // dN/dt adjoints
+    A.ab = o; o += v;                // T-row scratch
+    A.dd = o; o += v;                // ddN adjoints of the rows
     A.Jb = o; o += m * L.ld;
     A.raw = o; o += m * L.ld;
     A.Jc = o; o += m * L.ld;          // the converted Jacobian at y0 (before the shift)
-    A.dfc = o; o += m;                // its dfdx
-    A.cb = o; o += nS;
     A.Mb = o; o += (n_tb > 0 ? n_tb : 1);
     A.gq = o; o += 2 * kSideInline * (nR > 0 ? nR : 1) + 1;  // and a 0 for the gather's missing records
-    A.ms = o; o += MS_N;
-    A.vb = o; o += 4 * nS;           // Cp, Ha, rhoM/W, v adjoints
-    A.dn = o; o += nS;               // dN/dt adjoints
-    A.ab = o; o += m;                // T-row scratch
-    A.dd = o; o += m;                // ddN adjoints of the rows
     A.size = o;
     return A;
 }
@@ -692,7 +693,7 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
     for (int e = g.lane; e < m * m; e += G) {
         const int a = e / m, b = e % m;
         double acc = 0.0;
-        for (int st = 0; st < C.s; ++st) acc += wa[A.rb + st * m + a] * w[L.k1 + st * m + b];
+        for (int st = 0; st < C.s; ++st) acc += wa[A.rb + st * m + a] * w[L.k1 + st * L.ks + b];
         wa[A.Jb + a * ld + b] = acc;
     }
     g.sync();
@@ -703,19 +704,16 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
     }
 }
 
-// MS > 0: the matrix size fixed at compile time, as in process_cell.
+// MS: the matrix sizes that it is compiled for (fix_size).
 template <int MS>
 __global__ void __launch_bounds__(64) adjoint_kernel(const DevMech Mp, const AdjArgs a) {
     extern __shared__ double smem[];
     DevMech M = Mp;
-    if constexpr (MS > 0) {
-        M.m = MS;
-        M.nS = MS - 1;
-    }
+    if (!fix_size<MS>(M)) return;
     Grp<64> g;
-    const WsLayout L = make_layout(M.nS, M.nR, M.n_slots, M.n_tb, true);
+    const WsLayout L = make_layout(M.nS, M.nR, M.n_slots, M.n_tb, true, size_pad(MS));
     int fwd = 0;
-    const AdjLayout A = make_adj_layout(L, M.nS, M.nR, M.n_tb, &fwd);
+    const AdjLayout A = make_adj_layout(L, M.nS, M.nR, M.n_tb, &fwd, size_pad(MS));
     WsC w{smem};
     WsC wa{a.ws + (size_t)blockIdx.x * a.ws_per_cell};
     const RosCoeffs C = ros_coeffs(a.ode.solver);
@@ -772,27 +770,49 @@ __global__ void __launch_bounds__(128, 4) record_kernel(const DevMech M, const L
         if (g.lane == 0) cell = (long long)atomicAdd(a.queue, 1ull);
         cell = g.bcast_ll(cell, 0);
         if (cell >= a.n_cells) break;
-        process_cell<128, WsC, true, 8, MS>(g, M, WsC{smem}, a, (int)cell);
+        if (!process_cell<128, WsC, true, 8, MS, size_pad(MS)>(g, M, WsC{smem}, a, (int)cell)) return;
     }
 }
 
 __global__ void adj_reset(unsigned long long* q) { q[0] = 0; }
 
-// The kernels compiled for the 53-species and the 10-species mechanisms, else
-// the general ones (with the transposed solves in blocks: gradient of 600 cells
-// of 53 species 95.4 -> 74.0 ms, of 2,048 cells of 10 species 24.7 -> 17.1 ms).
+// Kernels for m <= 32, for 33 .. 64 and for any size. In the first two a vector of
+// the workspaces has room for the range's largest size, so that all but the
+// matrices and what follows them lie at offsets known at compile time. Recording
+// and sweep of 1,024 cells of 20 species 6.65 + 17.9 -> 4.66 + 16.2 ms against
+// code for any size, of 600 cells of 60 species 8.0 + 20.0 -> 5.8 + 18.6.
 using RecordFn = void (*)(const DevMech, const LaunchArgs);
 using AdjointFn = void (*)(const DevMech, const AdjArgs);
-static RecordFn record_fn(int m) { return m == 54 ? record_kernel<54> : (m == 11 ? record_kernel<11> : record_kernel<0>); }
-static AdjointFn adjoint_fn(int m) {
-    return m == 54 ? adjoint_kernel<54> : (m == 11 ? adjoint_kernel<11> : adjoint_kernel<0>);
+static int record_smem_bytes(const DevMech& M, int pad) {
+    return make_layout(M.nS, M.nR, M.n_slots, M.n_tb, false, pad).size * (int)sizeof(double);
+}
+static AdjLayout adjoint_layout(const DevMech& M, int pad, int* fwd) {
+    return make_adj_layout(make_layout(M.nS, M.nR, M.n_slots, M.n_tb, true, pad), M.nS, M.nR, M.n_tb, fwd, pad);
+}
+static int adjoint_smem_bytes(const DevMech& M, int pad) {
+    int fwd = 0;
+    adjoint_layout(M, pad, &fwd);
+    return fwd * (int)sizeof(double);
+}
+// The size class of a mechanism whose padded workspace takes `bytes` of shared
+// memory, or 0: the kernel for any size, whose workspace is not padded.
+static int adj_class(const DevMech& M, int (*bytes)(const DevMech&, int)) {
+    const int pad = size_range(M.m) <= 64 ? size_range(M.m) : 0;
+    return bytes(M, pad) <= 226 * 1024 ? -pad : 0;
+}
+static RecordFn record_fn(int ms) {
+    return ms == -32 ? record_kernel<-32> : (ms == -64 ? record_kernel<-64> : record_kernel<0>);
+}
+static AdjointFn adjoint_fn(int ms) {
+    return ms == -32 ? adjoint_kernel<-32> : (ms == -64 ? adjoint_kernel<-64> : adjoint_kernel<0>);
 }
 
 int launch_record(const DevMech& M, const LaunchArgs& a, void* stream) {
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const int smem = make_layout(M.nS, M.nR, M.n_slots, M.n_tb).size * (int)sizeof(double);
+    const int ms = adj_class(M, record_smem_bytes);
+    const int smem = record_smem_bytes(M, -ms);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
-    const RecordFn fn = record_fn(M.m);
+    const RecordFn fn = record_fn(ms);
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (e != cudaSuccess) return (int)e;
     int per_sm = 0;
@@ -805,22 +825,15 @@ int launch_record(const DevMech& M, const LaunchArgs& a, void* stream) {
 }
 
 int adjoint_ws_doubles(const DevMech& M) {
-    const WsLayout L = make_layout(M.nS, M.nR, M.n_slots, M.n_tb, true);
     int fwd = 0;
-    return make_adj_layout(L, M.nS, M.nR, M.n_tb, &fwd).size;
-}
-
-static int adjoint_smem_bytes(const DevMech& M) {
-    const WsLayout L = make_layout(M.nS, M.nR, M.n_slots, M.n_tb, true);
-    int fwd = 0;
-    make_adj_layout(L, M.nS, M.nR, M.n_tb, &fwd);
-    return fwd * (int)sizeof(double);
+    return adjoint_layout(M, -adj_class(M, adjoint_smem_bytes), &fwd).size;
 }
 
 int adjoint_blocks_per_sm(const DevMech& M) {
-    const int smem = adjoint_smem_bytes(M);
+    const int ms = adj_class(M, adjoint_smem_bytes);
+    const int smem = adjoint_smem_bytes(M, -ms);
     if (smem > 227 * 1024) return 0;
-    const AdjointFn fn = adjoint_fn(M.m);
+    const AdjointFn fn = adjoint_fn(ms);
     if (allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem) != cudaSuccess) return 0;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 64, smem) != cudaSuccess) return 0;
@@ -852,7 +865,8 @@ int launch_adjoint_cells(const DevMech& M, int n_cells, const double* traj, int 
     a.queue = queue;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     adj_reset<<<1, 1, 0, s>>>(queue);
-    if (n_cells > 0) adjoint_fn(M.m)<<<n_blocks, 64, adjoint_smem_bytes(M), s>>>(M, a);
+    const int ms = adj_class(M, adjoint_smem_bytes);
+    if (n_cells > 0) adjoint_fn(ms)<<<n_blocks, 64, adjoint_smem_bytes(M, -ms), s>>>(M, a);
     return (int)cudaGetLastError();
 }
 

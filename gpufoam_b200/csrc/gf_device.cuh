@@ -588,40 +588,46 @@ __device__ __forceinline__ double fast_products(const DevMech& M, const W& w, in
 // written while the Jacobian is built), and have one pivot region: the solves
 // follow either the pivots or their permutation (solve_layout places the other
 // in k1, free until the first stage). The adjoint's sweep (sweep = true) needs
-// both after the stages and gets separate regions.
-__host__ __device__ inline WsLayout make_layout(int nS, int nR, int n_slots, int n_tb, bool sweep = false) {
+// both after the stages and gets separate regions. pad: the doubles given to a
+// vector (m or more), or 0: as many as it needs.
+__host__ __device__ inline WsLayout make_layout(int nS, int nR, int n_slots, int n_tb, bool sweep = false,
+                                                int pad = 0) {
     WsLayout L;
-    const int m = nS + 1;
+    const int m = nS + 1, v = pad ? pad : m;
     L.ld = m | 1;
+    L.ks = v;
     int o = 0;
-    L.J = o;
-    o += m * L.ld;
-    L.y0 = o; o += m;
-    L.yt = o; o += m;
-    L.dydx0 = o; o += m;
-    L.dydx = o; o += m;
-    L.dfdx = o; o += m;
-    L.k1 = o; o += m;
-    L.k2 = o; o += m;
-    L.k3 = o; o += m;
-    L.k4 = o; o += m;
-    L.vv = o; o += m;
-    L.piv = o; o += m;
+    L.J = 0;
+    if (!pad) o += m * L.ld;
+    L.y0 = o; o += v;
+    L.yt = o; o += v;
+    L.dydx0 = o; o += v;
+    L.dydx = o; o += v;
+    L.dfdx = o; o += v;
+    L.k1 = o; o += v;
+    L.k2 = o; o += v;
+    L.k3 = o; o += v;
+    L.k4 = o; o += v;
+    L.vv = o; o += v;
+    L.piv = o; o += v;
     if (sweep) {
-        L.perm = o; o += m;
+        L.perm = o; o += v;
     } else {
         L.perm = L.piv;
     }
-    L.c = o; o += nS + 1;  // and a 1 for the absent species of a reaction side
-    L.Ha = o; o += nS;
+    L.c = o; o += v;  // nS, and a 1 for the absent species of a reaction side
+    L.Ha = o; o += pad ? v : nS;
     if (sweep) {
-        L.Cp = o; o += nS;
-        L.rhoMbyW = o; o += nS;
-        L.vj = o; o += nS;
+        L.Cp = o; o += pad ? v : nS;
+        L.rhoMbyW = o; o += pad ? v : nS;
+        L.vj = o; o += pad ? v : nS;
     } else {
         L.Cp = L.k2;
         L.vj = L.k3;
         L.rhoMbyW = L.k4;
+    }
+    if (pad) {  // behind the vectors, whose places are then known
+        L.J = o; o += m * L.ld;
     }
     L.stage = o; o += n_slots + 1;  // and a 0 for the gathers' missing records
     L.part = L.k3;                  // k3, k4: no stage has written them when f is assembled
@@ -1569,8 +1575,8 @@ __host__ __device__ constexpr bool solve_uses_perm(int m) {
 // solves do not read (written by the factorisation or by lu_perm, consumed
 // before the first stage) goes to k1.
 template <int G>
-__host__ __device__ inline WsLayout solve_layout(int nS, int nR, int n_slots, int n_tb) {
-    WsLayout L = make_layout(nS, nR, n_slots, n_tb);
+__host__ __device__ inline WsLayout solve_layout(int nS, int nR, int n_slots, int n_tb, int pad = 0) {
+    WsLayout L = make_layout(nS, nR, n_slots, n_tb, false, pad);
     if (solve_uses_perm<G>(nS + 1))
         L.piv = L.k1;
     else
@@ -1941,7 +1947,7 @@ __device__ __forceinline__ double ros_attempt(const Grp<G>& g, const DevMech& M,
             const int pt = !SAVE ? yt_off : (st == 1 ? save_y2 : (st == 2 ? save_y3 : yt_off));
             for (int i = g.lane; i < m; i += G) {
                 double v = w[y0_off + i];
-                for (int j = 0; j < st; ++j) v += ros_a(C, st, j) * w[L.k1 + j * m + i];
+                for (int j = 0; j < st; ++j) v += ros_a(C, st, j) * w[L.k1 + j * L.ks + i];
                 w[pt + i] = v;
             }
             at = pt;
@@ -1962,14 +1968,14 @@ __device__ __forceinline__ double ros_attempt(const Grp<G>& g, const DevMech& M,
                 continue;
             }
         }
-        const int ki = L.k1 + st * m;
+        const int ki = L.k1 + st * L.ks;
         const int src = st == 0 ? L.dydx0 : L.dydx;
         const double dd = dx * ros_d(C, st);
         for (int i = g.lane; i < m; i += G) {
             double v = w[src + i] + dd * w[L.dfdx + i];
             if (st > 0) {
                 double cs = ros_c(C, st, 0) * w[L.k1 + i];
-                for (int j = 1; j < st; ++j) cs += ros_c(C, st, j) * w[L.k1 + j * m + i];
+                for (int j = 1; j < st; ++j) cs += ros_c(C, st, j) * w[L.k1 + j * L.ks + i];
                 v += cs / dx;
             }
             w[ki + i] = v;
@@ -2082,10 +2088,10 @@ __device__ __forceinline__ unsigned long long dbl_key(double v) {
 // singleCellSolver::operator() (singleCellSolver.H:27-51) with the
 // computeYNew / computeRR epilogue (gpuKernelEvaluator.cu:84-96) fused:
 // RR, the min of deltaTChemNew before clamping, and the clamp.
-template <int G, class W, bool REC = false, int NB = 8>
+template <int G, class W, bool REC = false, int NB = 8, int PAD = 0>
 __device__ __forceinline__ void process_cell_body(const Grp<G>& g, const DevMech& M, const W& w, const LaunchArgs& a,
                                                   int cell) {
-    const WsLayout L = solve_layout<G>(M.nS, M.nR, M.n_slots, M.n_tb);
+    const WsLayout L = solve_layout<G>(M.nS, M.nR, M.n_slots, M.n_tb, PAD);
     const int nS = M.nS, m = M.m;
     const double* yin = a.Y0 + (size_t)cell * a.ld_y;
     int y_off = L.y0, yt_off = L.yt;
@@ -2150,21 +2156,50 @@ __device__ __forceinline__ void process_cell_body(const Grp<G>& g, const DevMech
     g.sync();
 }
 
-// process_cell_body with the LU panel width NB and, for MS > 0, the matrix
-// size m = MS (nS = MS - 1) fixed at compile time: the caller launches such a
-// kernel only for mechanisms of that size, and the compiler then resolves the
-// workspace offsets, loop bounds and tile predicates that depend on it.
-template <int G, class W, bool REC = false, int NB = 8, int MS = 0>
-__device__ __forceinline__ void process_cell(const Grp<G>& g, const DevMech& M, const W& w, const LaunchArgs& a,
+// The matrix sizes that a kernel is compiled for. MS > 0: the size MS, the only one
+// that its caller launches it for; MS < 0: the range of sizes up to -MS (and above
+// half of it, from 64 on); 0: any size.
+//
+// fix_size: whether M has a size of the kernel's, with M.m and M.nS as far as the
+// compiler can know them: all of a size, or its range, which decides the rows per
+// lane, the tiles and many loops and drops the code of the other sizes. The caller
+// leaves the mechanism alone where this says no.
+template <int MS>
+__device__ __forceinline__ bool fix_size(DevMech& M) {
+    if (MS > 0) {
+        M.m = MS;
+        M.nS = MS - 1;
+    } else if (MS < 0) {
+        constexpr int above = MS < -32 ? -MS / 2 : 1;
+        int m = M.m;
+        if (m <= above || m > -MS) return false;
+        // what the test has just shown, on a copy that the compiler knows nothing
+        // else about: it loses the range of the test itself on the way to the loops
+        asm("" : "+r"(m));
+        __builtin_assume(m <= -MS);
+        __builtin_assume(m > above);
+        M.m = m;
+        M.nS = m - 1;
+    }
+    return true;
+}
+// the largest size of m's range, 0 beyond the ranges
+__host__ __device__ constexpr int size_range(int m) { return m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 0)); }
+__host__ __device__ constexpr int size_pad(int MS) { return MS < 0 ? -MS : 0; }
+
+// process_cell_body with the LU panel width NB and the kernel's matrix sizes MS.
+// False: not a mechanism of the kernel's sizes, nothing done.
+template <int G, class W, bool REC = false, int NB = 8, int MS = 0, int PAD = 0>
+__device__ __forceinline__ bool process_cell(const Grp<G>& g, const DevMech& M, const W& w, const LaunchArgs& a,
                                              int cell) {
     if constexpr (MS == 0) {
-        process_cell_body<G, W, REC, NB>(g, M, w, a, cell);
+        process_cell_body<G, W, REC, NB, PAD>(g, M, w, a, cell);
     } else {
         DevMech Ms = M;
-        Ms.m = MS;
-        Ms.nS = MS - 1;
-        process_cell_body<G, W, REC, NB>(g, Ms, w, a, cell);
+        if (!fix_size<MS>(Ms)) return false;
+        process_cell_body<G, W, REC, NB, PAD>(g, Ms, w, a, cell);
     }
+    return true;
 }
 
 }  // namespace gf

@@ -158,6 +158,7 @@ struct OdeParams {
 struct WsLayout {
     int ld;          // Jacobian / LU row stride (odd, bank-conflict free columns)
     int J, y0, yt, dydx0, dydx, dfdx, k1, k2, k3, k4, c, Cp, Ha, rhoMbyW, vj, vv, piv, perm, stage, Mtb;
+    int ks;          // from one stage vector k1 .. k4 to the next
     int part;        // partial sums of dN/dt, 2 m doubles that are free while f is assembled
     int size;        // total doubles
 };

@@ -63,17 +63,16 @@ __global__ void __launch_bounds__(32) rates_kernel(const DevMech M, const double
 
 // One state per CTA of G threads (a warp for small systems; four warps share the
 // reactions, gathers and rows of a larger one: with one warp and 47 KB per state
-// an SM had four warps in flight: 350 us for 4,096 states of 53 species, 196 now).
-// MS: the matrix size fixed at compile time, or 0.
+// an SM had four warps in flight: 350 us for 4,096 states of 53 species, 207 now).
+// MS: the range of matrix sizes that it is compiled for (fix_size): 4,096 states of
+// 40 species 199 -> 172 us against code for any size, of 53 231 -> 225, of 31
+// species no difference.
 template <int G, int MS>
 __global__ void __launch_bounds__(G, 512 / G)
     jacobian_kernel(const DevMech Mp, const double* y, double* dfdx, double* J) {
     extern __shared__ double smem[];
     DevMech M = Mp;
-    if constexpr (MS > 0) {
-        M.m = MS;
-        M.nS = MS - 1;
-    }
+    if (!fix_size<MS>(M)) return;
     Grp<G> g;
     const WsLayout L = make_layout(M.nS, M.nR, M.n_slots, M.n_tb);
     const int n = M.nS + 2;
@@ -335,8 +334,22 @@ int launch_cells(const DevMech* mechs, int n_mechs, const gf_launch_config& cfg,
     const bool shared = cfg.scratch_in_shared != 0;
     int blocks = 0, threads = 0;
     const int ms = specialized_size(mechs, n_mechs);
-    const int ws_bytes = ws_doubles_per_cell * (int)sizeof(double);
     const void* fn = persistent_fn(cfg, ms);
+    if (G == 256 && shared && cfg.register_budget == 0) {
+        // by ranges of sizes, where the padded workspaces still fit
+        int ws = 0;
+        bool ranged = true;
+        for (int i = 0; i < P.n; ++i) {
+            const DevMech& M = mechs[i];
+            ranged = ranged && size_range(M.m) != 0;
+            ws = std::max(ws, make_layout(M.nS, M.nR, M.n_slots, M.n_tb, false, size_range(M.m)).size);
+        }
+        if (ranged && (size_t)ws * sizeof(double) <= 226 * 1024) {
+            fn = persistent_ranged_fn_g256();
+            ws_doubles_per_cell = ws;
+        }
+    }
+    const int ws_bytes = ws_doubles_per_cell * (int)sizeof(double);
     int slots = slots_of(fn, cfg, ws_bytes, &blocks, &threads);
     // A warp per cell, up to 255 registers, and more cells than run at once: the
     // kernel with 168 registers, if it holds more of them (small workspaces).
@@ -377,10 +390,9 @@ int launch_jacobian(const DevMech& m, int n, const double* y, double* dfdx, doub
     const size_t smem = (size_t)ws_layout(m).size * sizeof(double);
     const int G = m.m <= 32 ? 32 : 128;
     void (*fn)(const DevMech, const double*, double*, double*) =
-        m.m == 11    ? jacobian_kernel<32, 11>
-        : m.m <= 32  ? jacobian_kernel<32, 0>
-        : m.m == 54  ? jacobian_kernel<128, 54>
-        : m.m == 101 ? jacobian_kernel<128, 101>
+        m.m <= 32    ? jacobian_kernel<32, -32>
+        : m.m <= 64  ? jacobian_kernel<128, -64>
+        : m.m <= 128 ? jacobian_kernel<128, -128>
                      : jacobian_kernel<128, 0>;
     const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (e != cudaSuccess) return (int)e;

@@ -63,8 +63,9 @@ struct PersistShape {
     static constexpr int max_regs(int slim) { return slim == 2 ? 168 : (slim ? 128 : (G == 64 ? 200 : 255)); }
 };
 
-// NB: columns per LU panel of the blocked form (groups of less than 32 threads, m > 128); MS > 0: the matrix size m of every mechanism of
-// the launch, fixed at compile time (process_cell).
+// NB: columns per LU panel of the blocked form (groups of less than 32 threads,
+// m > 128); MS: the matrix sizes that it is compiled for (process_cell); negative:
+// every range of sizes to 128 has its own code and layout (persistent_ranged_fn_g256).
 template <int G, bool SHARED, int SLIM, int NB = 8, int MS = 0>
 __global__ void __maxnreg__(PersistShape<G>::max_regs(SLIM))
     persistent_kernel(const MechSet P, const LaunchArgs a, int ws_per_cell, long long n_slots) {
@@ -86,20 +87,12 @@ __global__ void __maxnreg__(PersistShape<G>::max_regs(SLIM))
         const DevMech& M = *Mp;
         if (SHARED) {
             const WsC w{smem + (size_t)gib * ws_per_cell};
-            // 256 threads per cell, one CTA per SM: the form of launches that mix
-            // mechanisms. Each of the known sizes has its own code in this kernel
-            // (fixed offsets, bounds and tiles, as in the tuned variants): 2,250
-            // cells of 10, 53 and 100 species 131.7 -> 123.6 ms. With several
-            // CTAs per SM their instructions would compete for the caches.
-            if constexpr (G == 256 && SLIM == 0 && MS == 0) {
-                if (M.m == 54) {
-                    process_cell<G, WsC, false, NB, 54>(g, M, w, a, (int)cell);
-                    continue;
-                }
-                if (M.m == 101) {
-                    process_cell<G, WsC, false, NB, 101>(g, M, w, a, (int)cell);
-                    continue;
-                }
+            if constexpr (MS < 0) {
+                if (!(process_cell<G, WsC, false, NB, -32, 32>(g, M, w, a, (int)cell) ||
+                      process_cell<G, WsC, false, NB, -64, 64>(g, M, w, a, (int)cell) ||
+                      process_cell<G, WsC, false, NB, -128, 128>(g, M, w, a, (int)cell)))
+                    reject_cell(g, a, cell);
+                continue;
             }
             process_cell<G, WsC, false, NB, MS>(g, M, w, a, (int)cell);
         } else if (G == 1) {
@@ -165,6 +158,14 @@ const void* persistent_fn_g64(bool shared, int slim);
 const void* persistent_fn_g96(bool shared, int slim);
 const void* persistent_fn_g128(bool shared, int slim);
 const void* persistent_fn_g256(bool shared, int slim);
+// The 256-thread form, workspace in shared memory, for matrix sizes to 128: the
+// form of launches that mix mechanisms and of those with one cell per SM. Each
+// range of sizes (fix_size) has its own code, with its own rows per lane and
+// tiles, and a vector of the workspace has room for the range's largest size, so
+// that the vectors lie at places known at compile time. Against one code for any
+// size, 701 cells of 70, 75, 90 and 120 species: 26.5, 20.3, 62.4 and 61.3 ->
+// 22.3, 16.9, 52.1 and 50.3 ms, 148 cells of 70: 7.7 -> 6.5 ms. With several CTAs per SM the ranges' instructions would compete for the caches.
+const void* persistent_ranged_fn_g256();
 // defined in gf_persist_g<G>_tuned.cu
 const void* persistent_tuned_fn_g32(bool shared, int slim, int nb, int ms);
 const void* persistent_tuned_fn_g64(bool shared, int slim, int nb, int ms);

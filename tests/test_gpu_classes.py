@@ -1,0 +1,94 @@
+"""Kernels compiled for a range of matrix sizes m = species + 1 (to 32, 33 .. 64,
+65 .. 128, any) at the edges of the ranges, on a B200: solves that mix mechanisms
+of every range in one launch, the Jacobian, and the gradient, whose transposed
+solves have two, four or ten rows per lane. Oracle and tolerances are those of the
+tests of the same quantities (tests/parity.py, tests/test_adjoint.py)."""
+import numpy as np
+import pytest
+
+from gpufoam_b200 import evaluator as E
+from gpufoam_b200 import mechanism as M
+from oracle.complex_step import ComplexStepMap
+from oracle.oracle import Oracle, ode_inputs
+from gpufoam_b200 import adjoint as AD
+from tests.parity import (assert_jacobian_close, assert_rates_close, assert_states_close, jacobian_scale, rate_scale,
+                          step_count_agreement)
+from tests.test_adjoint import Case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch
+    from gpufoam_b200 import build
+    build.build()
+    assert torch.cuda.is_available()
+    return torch
+
+
+def mechanism(n_species):
+    """A mechanism of n_species with about two reactions per species, of every reversible rate type."""
+    n = min(n_species, 14) if n_species < 20 else 2 * n_species
+    return M.make_mechanism(n_species, n, max(2, n // 8), max(2, n // 10), seed=n_species)
+
+
+@pytest.mark.parametrize("sizes", [(15, 31, 32, 63), (64, 100, 127), (128, 12, 40)])
+@pytest.mark.parametrize("threads", [32, 64, 256])
+def test_mixed_sizes(torch, sizes, threads):
+    raws = [mechanism(s) for s in sizes]
+    nS = max(r.n_species for r in raws)
+    per, ld = 9, nS + 2
+    Y = np.zeros((per * len(raws), ld))
+    mid = np.zeros(per * len(raws), dtype=np.int32)
+    for k, raw in enumerate(raws):
+        Y[k * per:(k + 1) * per, :raw.n_eqns] = M.make_cells(raw, per, seed=30 + k)
+        mid[k * per:(k + 1) * per] = k
+    order = np.random.default_rng(31).permutation(len(Y))
+    s = E.Solver([E.Mechanism(r) for r in raws], E.OdeInputs("Rosenbrock34", absTol=1e-8, relTol=1e-4))
+    s.set_launch(kind=1, threads_per_cell=threads, scratch_in_shared=1)
+    dtc = torch.full((len(Y),), 1e-7, dtype=torch.float64, device="cuda")
+    out = s.solve(torch.as_tensor(Y[order], device="cuda"), 1e-6, dtc,
+                  mech_id=torch.as_tensor(mid[order], device="cuda"))
+    got = {k: np.empty_like(out[k].cpu().numpy()) for k in ("Ynew", "status", "counters")}
+    for k in got:
+        got[k][order] = out[k].cpu().numpy()
+    for k, raw in enumerate(raws):
+        rows = slice(k * per, (k + 1) * per)
+        ref = Oracle(raw, "port").cells(ode_inputs(34), np.ascontiguousarray(Y[rows, :raw.n_eqns]), 1e-6, 1e-7)
+        assert np.array_equal(got["status"][rows], ref[3]), raw.n_species
+        ok = ref[3] == 0
+        assert_states_close(got["Ynew"][rows, :raw.n_eqns][ok], ref[0][ok], raw.n_species, 1e-4, f"{raw.n_species} species")
+        assert step_count_agreement(got["counters"][rows], ref[2]) >= 0.99, raw.n_species
+
+
+@pytest.mark.parametrize("n_species", [12, 31, 32, 63, 64, 127, 128])
+def test_jacobian_sizes(torch, n_species):
+    raw = mechanism(n_species)
+    y = M.make_cells(raw, 3, seed=32)
+    dfdx, J = E.jacobian(E.Mechanism(raw), y)
+    ref_f, ref_J = Oracle(raw, "port").jacobian(y)
+    assert_rates_close(dfdx.cpu().numpy(), ref_f, rate_scale(raw, y))
+    assert_jacobian_close(J.cpu().numpy(), ref_J, jacobian_scale(raw, y))
+
+
+@pytest.mark.parametrize("n_species, solver", [(15, 34), (31, 23), (32, 34), (63, 34), (64, 23), (100, 34), (127, 12),
+                                               (128, 34), (135, 23)])
+def test_gradient_sizes(torch, n_species, solver):
+    """The gradient along a random direction of all states and one of all rate parameters against the
+    tangent-linear map in complex arithmetic, and the recorded integration against the oracle's replay."""
+    raw = mechanism(n_species)
+    case = Case(raw, 2, 2e-7 if solver == 12 else 1e-6, solver, seed=40 + n_species)
+    for c in range(case.n):
+        np.testing.assert_allclose(case.orc.replay(case.inp, case.cells[c], case.steps[c]), case.Y1[c], rtol=1e-10,
+                                   atol=1e-14)
+    d = case.rng.standard_normal(case.cells.shape) * (np.abs(case.cells) + 1e-6)
+    d[:, raw.n_species + 1] = 0.0
+    cs, th0 = ComplexStepMap(raw, solver), AD.parameters_of(raw)
+    tl = sum(float(np.dot(case.w[c], cs.directional(case.cells[c], case.steps[c], th0, dy=d[c]))) for c in range(2))
+    ad = float(np.sum(case.Y0bar * d))
+    assert abs(ad - tl) <= 1e-5 * abs(tl), ("states", ad, tl)
+    dth = case.rng.standard_normal(th0.shape) * np.maximum(np.abs(th0), 1.0)
+    tl = sum(float(np.dot(case.w[c], cs.directional(case.cells[c], case.steps[c], th0, dtheta=dth))) for c in range(2))
+    ad = float(np.sum(case.thb * dth))
+    assert abs(ad - tl) <= 1e-5 * abs(tl), ("parameters", ad, tl)
