@@ -759,18 +759,18 @@ __global__ void __launch_bounds__(64) adjoint_kernel(const DevMech Mp, const Adj
 }
 
 // The recording solve (gf_solve_record): the persistent form with one cell
-// per 128-thread CTA, workspace in shared memory, at most 128 registers, and
+// per CTA of 128 threads, workspace in shared memory, at most 128 registers, and
 // each accepted step recorded for the sweep.
-template <int MS>
-__global__ void __launch_bounds__(128, 4) record_kernel(const DevMech M, const LaunchArgs a) {
+template <int MS, int G = 128>
+__global__ void __launch_bounds__(G, 512 / G) record_kernel(const DevMech M, const LaunchArgs a) {
     extern __shared__ double smem[];
-    Grp<128> g;
+    Grp<G> g;
     for (;;) {
         long long cell = 0;
         if (g.lane == 0) cell = (long long)atomicAdd(a.queue, 1ull);
         cell = g.bcast_ll(cell, 0);
         if (cell >= a.n_cells) break;
-        if (!process_cell<128, WsC, true, 8, MS, size_pad(MS)>(g, M, WsC{smem}, a, (int)cell)) return;
+        if (!process_cell<G, WsC, true, 8, MS, size_pad(MS)>(g, M, WsC{smem}, a, (int)cell)) return;
     }
 }
 
@@ -812,15 +812,17 @@ int launch_record(const DevMech& M, const LaunchArgs& a, void* stream) {
     const int ms = adj_class(M, record_smem_bytes);
     const int smem = record_smem_bytes(M, -ms);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
-    const RecordFn fn = record_fn(ms);
+    // beside the largest workspaces the reductions of 64 threads fit, not those of 128
+    const int G = smem + kGroupStaticBytes > 227 * 1024 ? 64 : 128;
+    const RecordFn fn = G == 64 ? record_kernel<0, 64> : record_fn(ms);
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (e != cudaSuccess) return (int)e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, G, smem);
     if (e != cudaSuccess) return (int)e;
     if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
     launch_epilogue_reset(a.queue, stream);
-    if (a.n_cells > 0) fn<<<per_sm * device_sm_count(), 128, smem, s>>>(M, a);
+    if (a.n_cells > 0) fn<<<per_sm * device_sm_count(), G, smem, s>>>(M, a);
     return (int)cudaGetLastError();
 }
 

@@ -69,7 +69,7 @@ enum { PH_MIX = 0, PH_NMPOW, PH_OMEGA, PH_GATHER_RHS, PH_JPARAMS, PH_JROWS, PH_T
 // used in turn, so that a reduction needs one barrier (a warp writes a buffer
 // again only after the barrier of the reduction in between, which every warp
 // reaches after reading it).
-constexpr int kRedMax = 4;  // values reduced together
+constexpr int kRedMax = 3;  // values reduced together
 template <int NW>
 __device__ __forceinline__ double* grp_red_buf() {
     __shared__ double buf[2 * NW * kRedMax];

@@ -257,7 +257,8 @@ int device_sm_count();
 // is refused: so it is always raised to the same value, the most that a block can
 // have beside fn's static part, and no host thread can lower it between another
 // one's call and its launch. The first 40 KB need no attribute (the default limit
-// is 48 KB with the static part, here at most 512 bytes), nor a driver call.
+// is 48 KB with the static part, here at most 384 bytes), nor a driver call.
 cudaError_t allow_dynamic_smem(const void* fn, size_t smem);
+constexpr int kGroupStaticBytes = 384;  // the most that a group's reductions take (256 threads)
 
 }  // namespace gf

@@ -311,12 +311,23 @@ static int slots_of(const void* fn, const gf_launch_config& cfg, int smem_bytes_
     return blocks * cpb;
 }
 
-int persistent_slots(const gf_launch_config& cfg, int ms, int smem_bytes_per_cell, int* blocks_out,
+// The form that a launch takes where the set one's reductions do not fit a block's
+// shared memory beside the workspace: those of 64 threads do.
+static gf_launch_config form_that_fits(gf_launch_config cfg, int smem_bytes_per_cell) {
+    if (cfg.scratch_in_shared && cfg.threads_per_cell > 64 && smem_bytes_per_cell + kGroupStaticBytes > 227 * 1024) {
+        cfg.threads_per_cell = 64;
+        cfg.register_budget = cfg.lu_panel = cfg.specialize = 0;
+    }
+    return cfg;
+}
+
+int persistent_slots(const gf_launch_config& set, int ms, int smem_bytes_per_cell, int* blocks_out,
                      int* threads_out) {
+    const gf_launch_config cfg = form_that_fits(set, smem_bytes_per_cell);
     return slots_of(persistent_fn(cfg, ms), cfg, smem_bytes_per_cell, blocks_out, threads_out);
 }
 
-int launch_cells(const DevMech* mechs, int n_mechs, const gf_launch_config& cfg, const LaunchArgs& a,
+int launch_cells(const DevMech* mechs, int n_mechs, const gf_launch_config& set, const LaunchArgs& a,
                  int ws_doubles_per_cell, int n_slots_total, void* stream) {
     MechSet P;
     P.n = std::min(n_mechs, kMaxMechs);
@@ -324,12 +335,13 @@ int launch_cells(const DevMech* mechs, int n_mechs, const gf_launch_config& cfg,
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     reset_kernel<<<1, 1, 0, s>>>(a.queue);
     if (a.n_cells <= 0) return (int)cudaGetLastError();
-    if (cfg.kind == 0) {
+    if (set.kind == 0) {
         const int threads = 128;
         const long long blocks = (a.n_cells + threads - 1) / threads;
         plain_kernel<<<(unsigned)blocks, threads, 0, s>>>(P, a);
         return (int)cudaGetLastError();
     }
+    const gf_launch_config cfg = form_that_fits(set, ws_doubles_per_cell * (int)sizeof(double));
     const int G = cfg.threads_per_cell;
     const bool shared = cfg.scratch_in_shared != 0;
     int blocks = 0, threads = 0;
@@ -388,9 +400,11 @@ int launch_jacobian(const DevMech& m, int n, const double* y, double* dfdx, doub
                     void* stream) {
     if (n <= 0) return 0;
     const size_t smem = (size_t)ws_layout(m).size * sizeof(double);
-    const int G = m.m <= 32 ? 32 : 128;
+    // four warps, where their reductions fit beside the workspace
+    const int G = m.m <= 32 || smem + kGroupStaticBytes > 227 * 1024 ? 32 : 128;
     void (*fn)(const DevMech, const double*, double*, double*) =
         m.m <= 32    ? jacobian_kernel<32, -32>
+        : G == 32    ? jacobian_kernel<32, 0>
         : m.m <= 64  ? jacobian_kernel<128, -64>
         : m.m <= 128 ? jacobian_kernel<128, -128>
                      : jacobian_kernel<128, 0>;

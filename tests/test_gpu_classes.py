@@ -6,14 +6,15 @@ tests of the same quantities (tests/parity.py, tests/test_adjoint.py)."""
 import numpy as np
 import pytest
 
+from gpufoam_b200 import adjoint as AD
 from gpufoam_b200 import evaluator as E
 from gpufoam_b200 import mechanism as M
 from oracle.complex_step import ComplexStepMap
 from oracle.oracle import Oracle, ode_inputs
-from gpufoam_b200 import adjoint as AD
 from tests.parity import (assert_jacobian_close, assert_rates_close, assert_states_close, jacobian_scale, rate_scale,
                           step_count_agreement)
 from tests.test_adjoint import Case
+from tests.test_gpu_edges import filled
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +93,43 @@ def test_gradient_sizes(torch, n_species, solver):
     tl = sum(float(np.dot(case.w[c], cs.directional(case.cells[c], case.steps[c], th0, dtheta=dth))) for c in range(2))
     ad = float(np.sum(case.thb * dth))
     assert abs(ad - tl) <= 1e-5 * abs(tl), ("parameters", ad, tl)
+
+
+def filled_workspace(factory, doubles):
+    """A mechanism whose solve workspace is `doubles` long (and the mechanism's own check of that)."""
+    raw = factory(0)
+    nS, m = raw.n_species, raw.n_species + 1
+    raw = filled(raw, doubles - (m * (m | 1) + 11 * m + nS + 1 + nS + 1) + 2 * nS)
+    mech = E.Mechanism(raw)
+    solver = E.Solver([mech], E.OdeInputs("Rosenbrock34", absTol=1e-8, relTol=1e-4))
+    assert solver.workspace_doubles() == doubles
+    return raw, mech, solver
+
+
+def test_workspaces_that_just_fit(torch):
+    """Workspaces that fill a block's 227 KB but for the 64 bytes that a group's reductions take at
+    least: every number of threads takes them, as do the recorded solve and the Jacobian."""
+    raw, mech, solver = filled_workspace(M.gri_size, (227 * 1024 - 64) // 8 - 6)
+    n, dT = 3, 1e-8
+    cells = M.make_cells(raw, n, seed=50)
+    ref = Oracle(raw, "port").cells(ode_inputs(34), cells, dT, 1e-9)
+    assert (ref[3] == 0).all()
+    forms = [None] + [dict(threads_per_cell=G, register_budget=r) for G in (32, 64, 96, 128, 256) for r in (0, 1)]
+    for f in forms:
+        if f is not None:
+            solver.set_launch(kind=1, scratch_in_shared=1, **f)
+        dtc = torch.full((n,), 1e-9, dtype=torch.float64, device="cuda")
+        out = solver.solve(torch.as_tensor(cells, device="cuda"), dT, dtc)
+        assert np.array_equal(out["status"].cpu().numpy(), ref[3]), f
+        assert_states_close(out["Ynew"].cpu().numpy(), ref[0], raw.n_species, 1e-4, str(f))
+    adj = AD.AdjointSolver(raw, E.OdeInputs("Rosenbrock34", absTol=1e-8, relTol=1e-4), traj_cap=64)
+    Y1, status, _ = adj.forward(torch.as_tensor(cells, device="cuda"), dT,
+                                torch.full((n,), 1e-9, dtype=torch.float64, device="cuda"))
+    assert (status.cpu().numpy() == 0).all()
+    assert_states_close(Y1.cpu().numpy(), ref[0], raw.n_species, 1e-4, "recorded")
+    # the Jacobian needs no reductions beside the workspace: one warp takes eight doubles more
+    raw, mech, _ = filled_workspace(M.gri_size, 227 * 1024 // 8 - 6)
+    dfdx, J = E.jacobian(mech, cells)
+    ref_f, ref_J = Oracle(raw, "port").jacobian(cells)
+    assert_rates_close(dfdx.cpu().numpy(), ref_f, rate_scale(raw, cells))
+    assert_jacobian_close(J.cpu().numpy(), ref_J, jacobian_scale(raw, cells))
