@@ -327,6 +327,46 @@ int persistent_slots(const gf_launch_config& set, int ms, int smem_bytes_per_cel
     return slots_of(persistent_fn(cfg, ms), cfg, smem_bytes_per_cell, blocks_out, threads_out);
 }
 
+// The kernel of G threads for a range of sizes: its largest, or kAllRanges.
+static const void* ranged_fn(int G, int range, bool dense) {
+    switch (G) {
+    case 32: return persistent_ranged_fn_g32(range, dense);
+    case 64: return persistent_ranged_fn_g64(range);
+    case 128: return persistent_ranged_fn_g128(range);
+    case 256: return range == kAllRanges ? persistent_ranged_fn_g256() : nullptr;
+    default: return nullptr;
+    }
+}
+
+// The range of sizes (ranged_fn) whose kernel takes this launch, or 0: where one
+// is compiled, the workspace is in shared memory and as many of the padded
+// workspaces as of the plain ones are resident on an SM. *ws: the workspace then.
+static int ranged_launch(const DevMech* mechs, int n_mechs, const gf_launch_config& cfg, int* ws) {
+    const int G = cfg.threads_per_cell;
+    if (!cfg.scratch_in_shared || cfg.register_budget || cfg.specialize) return 0;
+    int padded = 0, range = size_range(mechs[0].m);
+    for (int i = 0; i < n_mechs; ++i) {
+        const DevMech& M = mechs[i];
+        const int r = size_range(M.m);
+        if (r == 0) return 0;
+        if (r != range) range = kAllRanges;
+        padded = std::max(padded, make_layout(M.nS, M.nR, M.n_slots, M.n_tb, false, r).size);
+    }
+    if (G == 256) range = kAllRanges;
+    if (!ranged_fn(G, range, false)) return 0;
+    // CTAs per SM by shared memory (1 KB of each is the system's) and by registers
+    const int cells = G > 32 ? 1 : (cfg.cells_per_block > 0 ? std::min(cfg.cells_per_block, 4) : 4);
+    const int regs = G == 32 ? 168 : (G == 64 ? 200 : 255);
+    auto resident = [&](int doubles) {
+        const int bytes = cells * doubles * (int)sizeof(double);
+        if (bytes + kGroupStaticBytes > 227 * 1024) return 0;
+        return std::min(228 * 1024 / (bytes + kGroupStaticBytes + 1024), 65536 / (regs * cells * G));
+    };
+    if (resident(padded) == 0 || resident(padded) < resident(*ws)) return 0;
+    *ws = padded;
+    return range;
+}
+
 int launch_cells(const DevMech* mechs, int n_mechs, const gf_launch_config& set, const LaunchArgs& a,
                  int ws_doubles_per_cell, int n_slots_total, void* stream) {
     MechSet P;
@@ -347,29 +387,17 @@ int launch_cells(const DevMech* mechs, int n_mechs, const gf_launch_config& set,
     int blocks = 0, threads = 0;
     const int ms = specialized_size(mechs, n_mechs);
     const void* fn = persistent_fn(cfg, ms);
-    if (G == 256 && shared && cfg.register_budget == 0) {
-        // by ranges of sizes, where the padded workspaces still fit
-        int ws = 0;
-        bool ranged = true;
-        for (int i = 0; i < P.n; ++i) {
-            const DevMech& M = mechs[i];
-            ranged = ranged && size_range(M.m) != 0;
-            ws = std::max(ws, make_layout(M.nS, M.nR, M.n_slots, M.n_tb, false, size_range(M.m)).size);
-        }
-        if (ranged && (size_t)ws * sizeof(double) <= 226 * 1024) {
-            fn = persistent_ranged_fn_g256();
-            ws_doubles_per_cell = ws;
-        }
-    }
+    const int range = ranged_launch(mechs, P.n, cfg, &ws_doubles_per_cell);
+    if (range) fn = ranged_fn(G, range, false);
     const int ws_bytes = ws_doubles_per_cell * (int)sizeof(double);
     int slots = slots_of(fn, cfg, ws_bytes, &blocks, &threads);
     // A warp per cell, up to 255 registers, and more cells than run at once: the
     // kernel with 168 registers, if it holds more of them (small workspaces).
     // 65,536 cells of 10 species 54.1 -> 46.5 ms; 1,024, which are resident
     // either way, would take 3.31 instead of 3.15 ms.
-    if (G == 32 && shared && cfg.register_budget == 0 && (cfg.lu_panel == 0 || cfg.lu_panel == 8) && slots > 0 &&
-        a.n_cells > slots && (!cfg.specialize || ms == 11)) {
-        const void* dense = persistent_dense_fn_g32(cfg.specialize ? ms : 0);
+    if (G == 32 && shared && cfg.register_budget == 0 && (range || cfg.lu_panel == 0 || cfg.lu_panel == 8) &&
+        slots > 0 && a.n_cells > slots && (!cfg.specialize || ms == 11)) {
+        const void* dense = range ? ranged_fn(G, range, true) : persistent_dense_fn_g32(cfg.specialize ? ms : 0);
         int b = 0, t = 0;
         const int k = slots_of(dense, cfg, ws_bytes, &b, &t);
         if (k > slots) {
@@ -454,6 +482,9 @@ extern "C" int gf_debug_phase_cycles(unsigned long long* out, int reset) {
     phase_cycles_g64t(out, reset);
     phase_cycles_g96t(out, reset);
     phase_cycles_g128t(out, reset);
+    phase_cycles_g32r(out, reset);
+    phase_cycles_g64r(out, reset);
+    phase_cycles_g128r(out, reset);
     return phase_cycles_g256(out, reset);
 }
 namespace gf {

@@ -64,8 +64,10 @@ struct PersistShape {
 };
 
 // NB: columns per LU panel of the blocked form (groups of less than 32 threads,
-// m > 128); MS: the matrix sizes that it is compiled for (process_cell); negative:
-// every range of sizes to 128 has its own code and layout (persistent_ranged_fn_g256).
+// m > 128); MS: the matrix sizes that it is compiled for (process_cell); with a
+// range of sizes the workspace is padded to its largest (persistent_ranged_fn).
+// kAllRanges: every range of sizes to 128, each with its own code and layout.
+constexpr int kAllRanges = -1;
 template <int G, bool SHARED, int SLIM, int NB = 8, int MS = 0>
 __global__ void __maxnreg__(PersistShape<G>::max_regs(SLIM))
     persistent_kernel(const MechSet P, const LaunchArgs a, int ws_per_cell, long long n_slots) {
@@ -87,14 +89,15 @@ __global__ void __maxnreg__(PersistShape<G>::max_regs(SLIM))
         const DevMech& M = *Mp;
         if (SHARED) {
             const WsC w{smem + (size_t)gib * ws_per_cell};
-            if constexpr (MS < 0) {
+            if constexpr (MS == kAllRanges) {
                 if (!(process_cell<G, WsC, false, NB, -32, 32>(g, M, w, a, (int)cell) ||
                       process_cell<G, WsC, false, NB, -64, 64>(g, M, w, a, (int)cell) ||
                       process_cell<G, WsC, false, NB, -128, 128>(g, M, w, a, (int)cell)))
                     reject_cell(g, a, cell);
-                continue;
+            } else {
+                if (!process_cell<G, WsC, false, NB, MS, size_pad(MS)>(g, M, w, a, (int)cell))
+                    reject_cell(g, a, cell);
             }
-            process_cell<G, WsC, false, NB, MS>(g, M, w, a, (int)cell);
         } else if (G == 1) {
             process_cell<G, WsS, false, NB, MS>(g, M, WsS{a.ws + slot, n_slots}, a, (int)cell);
         } else {
@@ -164,8 +167,19 @@ const void* persistent_fn_g256(bool shared, int slim);
 // tiles, and a vector of the workspace has room for the range's largest size, so
 // that the vectors lie at places known at compile time. Against one code for any
 // size, 701 cells of 70, 75, 90 and 120 species: 26.5, 20.3, 62.4 and 61.3 ->
-// 22.3, 16.9, 52.1 and 50.3 ms, 148 cells of 70: 7.7 -> 6.5 ms. With several CTAs per SM the ranges' instructions would compete for the caches.
+// 22.3, 16.9, 52.1 and 50.3 ms, 148 cells of 70: 7.7 -> 6.5 ms. With several CTAs
+// per SM the ranges' instructions would compete for the caches.
 const void* persistent_ranged_fn_g256();
+// The same for the other forms that the default rule takes (default_launch), a kernel
+// per range (32, 64 or 128, the largest size) for launches whose mechanisms share
+// one; nullptr for a pair that is not compiled. gf_persist_g<G>_ranged.cu
+// 8,192 cells against one code for any size: a warp per cell, 20 and 31 species
+// 16.7 -> 12.2 and 27.5 -> 18.3 ms (65,536 of 10 species 38.1 -> 22.3; compiled for
+// m = 11 19.1); 64 threads, 44, 52 and 60 species 59.4, 36.6 and 135 -> 50.1, 30.1 and
+// 106; 128 threads, 66, 75 and 90 species 148, 119 and 275 -> 128, 99 and 230.
+const void* persistent_ranged_fn_g32(int range, bool dense);
+const void* persistent_ranged_fn_g64(int range);
+const void* persistent_ranged_fn_g128(int range);
 // defined in gf_persist_g<G>_tuned.cu
 const void* persistent_tuned_fn_g32(bool shared, int slim, int nb, int ms);
 const void* persistent_tuned_fn_g64(bool shared, int slim, int nb, int ms);
@@ -190,6 +204,10 @@ int phase_cycles_g32t(unsigned long long* out, int reset);
 int phase_cycles_g64t(unsigned long long* out, int reset);
 int phase_cycles_g96t(unsigned long long* out, int reset);
 int phase_cycles_g128t(unsigned long long* out, int reset);
+// the ranged kernels' units (gf_persist_g<G>_ranged.cu)
+int phase_cycles_g32r(unsigned long long* out, int reset);
+int phase_cycles_g64r(unsigned long long* out, int reset);
+int phase_cycles_g128r(unsigned long long* out, int reset);
 #endif
 
 }  // namespace gf

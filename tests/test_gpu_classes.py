@@ -63,6 +63,35 @@ def test_mixed_sizes(torch, sizes, threads):
         assert step_count_agreement(got["counters"][rows], ref[2]) >= 0.99, raw.n_species
 
 
+@pytest.mark.parametrize("sizes", [(12,), (15, 31), (32,), (40, 63), (64,), (100, 127), (128,)])
+def test_one_range(torch, sizes):
+    """Launches whose mechanisms are all of one range, with the forms that have a kernel for it; more cells
+    than are resident, so that a warp per cell takes the kernel with fewer registers."""
+    raws = [mechanism(s) for s in sizes]
+    nS = max(r.n_species for r in raws)
+    n, few, ld = (20000 if nS <= 31 else 300), 24, nS + 2
+    solver = E.Solver([E.Mechanism(r) for r in raws], E.OdeInputs("Rosenbrock23", absTol=1e-8, relTol=1e-4))
+    Y, mid = np.zeros((n, ld)), (np.arange(n) % len(raws)).astype(np.int32)
+    ref = []
+    for k, raw in enumerate(raws):
+        cells = M.make_cells(raw, few, seed=33 + k)
+        Y[mid == k, :raw.n_eqns] = cells[np.arange((mid == k).sum()) % few]
+        ref.append(Oracle(raw, "port").cells(ode_inputs(23), cells, 1e-6, 1e-7))
+    for form in (dict(threads_per_cell=32), dict(threads_per_cell=32, cells_per_block=1, lu_panel=4),
+                 dict(threads_per_cell=64), dict(threads_per_cell=128), dict(threads_per_cell=256)):
+        solver.set_launch(kind=1, scratch_in_shared=1, **form)
+        dtc = torch.full((n,), 1e-7, dtype=torch.float64, device="cuda")
+        out = {k: v.cpu().numpy() for k, v in solver.solve(torch.as_tensor(Y, device="cuda"), 1e-6, dtc,
+               mech_id=torch.as_tensor(mid, device="cuda")).items() if k in ("Ynew", "status", "counters")}
+        for k, raw in enumerate(raws):
+            at = np.arange((mid == k).sum()) % few
+            got = {name: v[mid == k] for name, v in out.items()}
+            assert np.array_equal(got["status"], ref[k][3][at]), form
+            ok = got["status"] == 0
+            assert_states_close(got["Ynew"][ok, :raw.n_eqns], ref[k][0][at][ok], raw.n_species, 1e-4, str(form))
+            assert step_count_agreement(got["counters"], ref[k][2][at]) >= 0.99, form
+
+
 @pytest.mark.parametrize("n_species", [12, 31, 32, 63, 64, 127, 128])
 def test_jacobian_sizes(torch, n_species):
     raw = mechanism(n_species)
