@@ -232,40 +232,50 @@ int ensure_ws(gf_solver* s, size_t bytes) {
     return GF_OK;
 }
 
-// The launch form of a solver that none was set for, by the largest matrix
-// size m of its mechanisms: persistent, the workspace in shared memory where it
-// fits, and the kernel compiled for m where there is one (the autotuner refines
-// this on a sample of cells). Measured on the B200, 64 threads per cell (two
-// warps, any m) against the rule:
-//  * m <= 32: a warp per cell, four cells per CTA; a second warp has no rows or
-//    reactions to work on. 65,536 cells of 10 species 148 -> 63 ms (46 ms since);
-//  * m <= 64: 128 threads and 128 registers; four cells per SM by registers,
-//    the other three warps shorten the reaction loops and gathers, and the rest
-//    of the SM's memory is L1 for the tables. 6,007 cells of 53 species,
-//    Rosenbrock23: 104 -> 73 ms (96 / 64 threads with the kernel compiled for m:
-//    1 % and 6 % slower over 400 .. 65,536 cells);
-//  * m <= 128: 256 threads; shared memory holds one cell per SM, and only its own
-//    threads hide its latency. 701 cells of 100 species 55 -> 31 ms;
-//  * larger ones, and workspaces in HBM: 64 threads.
+// The launch form of a solver that none was set for: persistent, by the number of
+// workspaces that an SM's shared memory holds (the autotuner refines this on a
+// sample of cells). The fewer cells an SM has, the more threads of its own each one
+// needs to hide its latency. Measured on the B200, many cells, against the next best
+// of 32, 64, 128 and 256 threads; the kernels are those for a range of sizes:
+//  * eight and m <= 32: a warp per cell, four cells per CTA; a second warp has no
+//    rows and few reactions to work on. 8,192 cells of 31 species and 153 reactions
+//    18.3 ms, with 64 threads 27.2;
+//  * four: 64 threads. 8,192 cells of 31 species and 500 reactions 70.8 ms, a warp
+//    each 75.0 or more; 44 species 50.1, 128 threads 71.8; 60 species 106 and 136;
+//  * two or three: 128 threads. 66 species 128 ms, 64 threads 133; 90 species 230, 64
+//    threads 311, 256 threads 375 (more than 128 registers a thread: one cell per SM);
+//  * one: 256 threads. 2,000 cells of 126 species 177 ms, 128 threads 264; of 130
+//    species 503 and 584; of 28 species with 2,200 reactions 183 and 347;
+//  * workspaces in HBM: 64 threads.
+// A kernel compiled for m (10, 53 and 100 species) is taken where there is one for the
+// form; that of 53 species, where three cells or more fit, with 128 threads and 128
+// registers: 8,192 cells of 325 reactions 67.9 ms, with 64 threads 72.3; of 800
+// reactions 145 and 161, with the range's kernel of 128 threads 181.
 gf_launch_config default_launch(const gf_solver* s) {
     int m = 0;
     for (const gf::DevMech& d : s->dmechs) m = std::max(m, d.m);
-    const bool shared = (size_t)s->max_ws_doubles * sizeof(double) <= 227 * 1024;
+    const size_t ws = (size_t)s->max_ws_doubles * sizeof(double);
     // kind, threads, shared, cells / CTA, CTAs / SM, registers, panel, specialize
-    gf_launch_config c{1, 64, shared ? 1 : 0, 1, 0, 0, 0, 0};
-    if (shared && m <= 32) {
-        c.threads_per_cell = 32;
-        c.cells_per_block = 0;
-    } else if (shared && m <= 64) {
-        c.threads_per_cell = 128;
-        c.register_budget = 1;
-    } else if (shared && m <= 128) {
-        c.threads_per_cell = 256;
+    gf_launch_config c{1, 64, 0, 1, 0, 0, 0, 0};
+    const int ms = gf::specialized_size(s->dmechs.data(), (int)s->dmechs.size());
+    if (ws <= 227 * 1024) {
+        c.scratch_in_shared = 1;
+        // 228 KB per SM; a CTA's reductions and the system's 1 KB beside its workspace
+        const int cells = (int)(228 * 1024 / (ws + gf::kGroupStaticBytes + 1024));
+        if (cells >= 8 && m <= 32) {
+            c.threads_per_cell = 32;
+            c.cells_per_block = 0;
+        } else if (cells < 4) {
+            c.threads_per_cell = cells >= 2 ? 128 : 256;
+        }
+        gf_launch_config sp = c;
+        sp.threads_per_cell = 128;
+        sp.register_budget = sp.specialize = 1;
+        if (cells >= 3 && m > 32 && gf::persistent_form_compiled(sp, ms)) return sp;
     }
     gf_launch_config sp = c;
     sp.specialize = 1;
-    if (gf::persistent_form_compiled(sp, gf::specialized_size(s->dmechs.data(), (int)s->dmechs.size()))) c = sp;
-    return c;
+    return gf::persistent_form_compiled(sp, ms) ? sp : c;
 }
 
 int ensure_staging(gf_solver* s, int n) {

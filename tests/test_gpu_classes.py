@@ -124,6 +124,28 @@ def test_gradient_sizes(torch, n_species, solver):
     assert abs(ad - tl) <= 1e-5 * abs(tl), ("parameters", ad, tl)
 
 
+@pytest.mark.parametrize("n_species, n_reactions, threads, shared", [
+    (31, 75, 32, 1), (31, 500, 64, 1), (25, 1300, 128, 1), (40, 98, 64, 1), (64, 156, 64, 1), (80, 194, 128, 1),
+    (100, 245, 128, 1), (127, 310, 256, 1), (135, 329, 256, 1), (160, 390, 64, 0)])
+def test_default_form(torch, n_species, n_reactions, threads, shared):
+    """The default launch form by the number of workspaces that an SM's shared memory holds: eight, four, two, one,
+    none."""
+    raw = mechanism(n_species)
+    raw.reactions = [raw.reactions[k % raw.n_reactions] for k in range(n_reactions)]
+    s = E.Solver([E.Mechanism(raw)], E.OdeInputs("Rosenbrock34", absTol=1e-8, relTol=1e-4))
+    cfg = s.get_launch()
+    assert (cfg["threads_per_cell"], cfg["scratch_in_shared"], cfg["specialize"]) == (threads, shared, 0)
+    n = 6
+    cells = M.make_cells(raw, n, seed=60)
+    ref = Oracle(raw, "port").cells(ode_inputs(34), cells, 1e-7, 1e-8)
+    dtc = torch.full((n,), 1e-8, dtype=torch.float64, device="cuda")
+    out = s.solve(torch.as_tensor(cells, device="cuda"), 1e-7, dtc)
+    assert np.array_equal(out["status"].cpu().numpy(), ref[3])
+    ok = ref[3] == 0
+    assert_states_close(out["Ynew"].cpu().numpy()[ok], ref[0][ok], n_species, 1e-4)
+    assert step_count_agreement(out["counters"].cpu().numpy(), ref[2]) >= 0.99
+
+
 def filled_workspace(factory, doubles):
     """A mechanism whose solve workspace is `doubles` long (and the mechanism's own check of that)."""
     raw = factory(0)
