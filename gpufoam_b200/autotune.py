@@ -8,9 +8,10 @@ offers on a sample of the caller's cells and keeps the fastest:
     inside a warp) or 64, 96, 128, 256 (one cell per CTA), the per-cell workspace in
     shared memory (when it fits) or in HBM, and two register budgets;
   * for 32, 64, 96 and 128 threads per cell, the tile and specialisation variants:
-    LU panels of 4 or 16 columns instead of 8, and the kernel compiled for the
-    mechanism's matrix size (10-, 53- and 100-species mechanisms), which fixes
-    the workspace offsets, loop bounds and the unrolled tiles' predicates.
+    LU panels of 4 or 16 columns instead of 8 (128 species and more), and the
+    kernel compiled for the mechanism's matrix size (10-, 53- and 100-species
+    mechanisms), which fixes the workspace offsets, loop bounds and the unrolled
+    tiles' predicates.
 
 Results are cached per (device, library build, mechanism shape, solver) in
 memory and in a JSON file (GPUFOAM_AUTOTUNE_CACHE, default
@@ -63,10 +64,11 @@ def _key(mechs, ode: E.OdeInputs) -> str:
     return h.hexdigest()[:16]
 
 
-def candidates(max_ws_doubles: int) -> List[dict]:
+def candidates(max_ws_doubles: int, lu_panels: bool = True) -> List[dict]:
     """Launch forms worth timing for a workspace of max_ws_doubles per cell:
     the plain kernel, and persistent forms with the workspace in shared memory
-    when a CTA's groups fit (else in HBM), both register budgets."""
+    when a CTA's groups fit (else in HBM), both register budgets. lu_panels:
+    also LU panels of 4 and 16 columns, which change nothing to 128 unknowns."""
     ws = max_ws_doubles * 8
     out = [dict(kind=0, threads_per_cell=1, scratch_in_shared=0, cells_per_block=0, blocks_per_sm=0,
                 register_budget=0, lu_panel=0, specialize=0)]
@@ -81,10 +83,9 @@ def candidates(max_ws_doubles: int) -> List[dict]:
                 # the tuned variants (gf_solver_set_launch refuses those that do
                 # not apply to the solver's mechanisms; tune() skips them)
                 regs = 1 if G in (96, 128) else 0
-                for nb in (0, 4):
-                    out.append(dict(kind=1, threads_per_cell=G, scratch_in_shared=shared, cells_per_block=0,
-                                    blocks_per_sm=0, register_budget=regs, lu_panel=nb, specialize=1))
-                if shared:
+                out.append(dict(kind=1, threads_per_cell=G, scratch_in_shared=shared, cells_per_block=0,
+                                blocks_per_sm=0, register_budget=regs, lu_panel=0, specialize=1))
+                if shared and lu_panels:
                     for nb in (4, 16):
                         out.append(dict(kind=1, threads_per_cell=G, scratch_in_shared=1, cells_per_block=0,
                                         blocks_per_sm=0, register_budget=regs, lu_panel=nb, specialize=0))
@@ -143,7 +144,7 @@ def tune(solver: E.Solver, Y_sample, deltaT: float, dtc0: float = 1e-7, deltaT_c
     d0 = torch.full((Y0.shape[0],), dtc0, dtype=torch.float64, device="cuda")
     ws = solver.workspace_doubles()
     table = []
-    cands = configs or candidates(ws)
+    cands = configs or candidates(ws, any(m.n_species >= 128 for m in solver.mechs))
     # the usual winners first, so that slow forms are cut off early
     cands = sorted(cands, key=lambda c: (c["kind"] == 0, abs(c["threads_per_cell"] - 96), -c["scratch_in_shared"]))
     best_ms = float("inf")

@@ -116,10 +116,10 @@ const void* persistent_variant(bool shared, int slim) {
 }
 
 // The tuned variants of the 32-, 64-, 96- and 128-thread forms (gf_persist_g<G>_tuned.cu):
-// LU panels of 4 or 16 columns (workspace in shared memory), and the matrix
-// size fixed at compile time for the 10-, 53- and 100-species mechanisms
-// (m = 11, 54, 101; workspace in shared memory or HBM; for m = 54 also with
-// 4-column panels). Each with the register budget the form is usually run with
+// LU panels of 4 or 16 columns (workspace in shared memory; they matter for m > 128
+// only, lu_factor), and the matrix size fixed at compile time for the 10-, 53- and
+// 100-species mechanisms (m = 11, 54, 101; workspace in shared memory or HBM; 4-column
+// panels are accepted for m = 54, and are the same kernel). Each with the register budget the form is usually run with
 // (SLIM for 96 and 128 threads); nullptr for a variant that is not compiled.
 constexpr int kTunedSlim(int G) { return (G == 128 || G == 96) ? 1 : 0; }
 template <int G, int S, int NB, int MS>
@@ -137,11 +137,7 @@ const void* persistent_tuned_variant(bool shared, int slim, int nb, int ms) {
         if (nb == 16) return tuned_kernel<G, S, 16, 0>(true);
         return nullptr;
     }
-    if (ms == 54) {
-        if (nb == 4) return tuned_kernel<G, S, 4, 54>(shared);
-        if (nb == 8) return tuned_kernel<G, S, 8, 54>(shared);
-        return nullptr;
-    }
+    if (ms == 54 && (nb == 8 || nb == 4)) return tuned_kernel<G, S, 8, 54>(shared);
     if (nb != 8) return nullptr;
     if (ms == 11) return tuned_kernel<G, S, 8, 11>(shared);
     if (ms == 101) return tuned_kernel<G, S, 8, 101>(shared);
