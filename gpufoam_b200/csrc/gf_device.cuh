@@ -1,9 +1,10 @@
-// Device code of the per-cell chemistry path (sm_100a, FP64 on CUDA cores).
+// Device code of the per-cell chemistry path (sm_100a, FP64 on CUDA cores, the
+// factorisation's trailing updates on the FP64 matrix units).
 //
 // One templated code path serves every launch form: a "group" of G threads
-// (G = 1, 2, 4, 8, 16, 32, aligned inside a warp) integrates one cell. G = 1 is
-// the reference's one-thread-per-cell model; G = 32 is a warp per cell with the
-// cell's Jacobian/LU held in shared memory. Loops over species, reactions,
+// (G = 1, 2, 4, 8, 16, 32, aligned inside a warp, or 64, 96, 128, 256, a whole CTA)
+// integrates one cell. G = 1 is the reference's one-thread-per-cell model; from
+// G = 32 on the cell's Jacobian/LU is usually held in shared memory. Loops over species, reactions,
 // rows and columns are strided over the group's lanes; everything that decides
 // control flow (error norm, step size, status) is group-uniform.
 //
@@ -59,7 +60,7 @@ static inline int phase_cycles_local(unsigned long long* out, int reset) {
 #define GF_PH_BEGIN(g)
 #define GF_PH_END(g, k)
 #endif
-enum { PH_MIX = 0, PH_NMPOW, PH_OMEGA, PH_GATHER_RHS, PH_JPARAMS, PH_JROWS, PH_TROW, PH_SHIFT, PH_LU, PH_SOLVE,
+enum { PH_MIX = 0, PH_OMEGA, PH_GATHER_RHS, PH_JPARAMS, PH_JROWS, PH_TROW, PH_SHIFT, PH_LU, PH_SOLVE,
        PH_ADJ_RXN, PH_ATTEMPT, PH_ADJ_RECOMPUTE, PH_ADJ_TSOLVE, PH_ADJ_VJP, PH_ADJ_JTERM, PH_LU_PANEL, PH_LU_U12,
        PH_LU_TRAIL, PH_LU_PERM };
 
@@ -583,9 +584,10 @@ __device__ __forceinline__ double fast_products(const DevMech& M, const W& w, in
 
 // ------------------------------------------------------------- layout
 
-// Per-cell workspace layout. The solve kernels (sweep = false) keep Cp, v and
-// rhoM/W, which only the Jacobian reads, in k2..k4 (the stage vectors, not yet
-// written while the Jacobian is built), and have one pivot region: the solves
+// Per-cell workspace layout. The solve kernels (sweep = false) keep Cp, which only
+// the Jacobian reads, in k2 and the parts of dN/dt in k3 and k4 (stage vectors, not
+// yet written while f or the Jacobian is formed; v and rhoM/W are kept by the sweep
+// alone, which has room for both), and have one pivot region: the solves
 // follow either the pivots or their permutation (solve_layout places the other
 // in k1, free until the first stage). The adjoint's sweep (sweep = true) needs
 // both after the stages and gets separate regions. pad: the doubles given to a
@@ -728,8 +730,8 @@ __host__ __device__ constexpr int stream_index(int G) { return G == 96 ? 9 : log
 // wd[dst + pos] = sum of coef * ws[src + slot] over each entry's records, in
 // order. The group's loads (48 coalesced bytes and the position) are
 // independent of the sums, so they pipeline (U groups at a time); one thread
-// owns each output entry (no barriers inside). Bound by instructions: 20 per four records, where
-// 16-byte records that each carried a position took 12 per record.
+// owns each output entry (no barriers inside). Bound by instructions,
+// of which 16-byte records that each carried a position took more.
 template <int U = 2, int G, class WS, class WD>
 __device__ __forceinline__ void stream_gather(const Grp<G>& g, const Stream& st, const WS& ws, int src, const WD& wd,
                                               int dst) {
@@ -1102,8 +1104,10 @@ __device__ __forceinline__ void lu_panel(const Grp<G>& g, const W& w, int A, int
 // c += a b for one 8 x 8 tile of doubles held by a warp (a: 8 x 4, b: 4 x 8;
 // lane l holds a[l/4][l%4], b[l%4][l/4], c[l/4][2 (l%4) + 0, 1]). The unit
 // accumulates its four products as a chain of FMAs in ascending k (measured on
-// the B200: 262,144 results of random tiles bit for bit), so a tile update is
-// the same as the scalar loop's.
+// the B200: 262,144 results of random tiles bit for bit; the instruction's
+// definition does not promise the order), so a tile update is the same as the
+// scalar loop's. test_lu_edges (tests/test_gpu_edges.py) holds every form's factors
+// to the scalar form's bit for bit, and would show a chip that adds otherwise.
 __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
                  : "+d"(c0), "+d"(c1)
@@ -1282,8 +1286,8 @@ __device__ __forceinline__ void lu_panel_reg(const W& w, int A, int ld, int piv,
 // updates with two roundings). sc: the row scalings; rd: out, 1 / U[i][i].
 //
 // Why: the factorisation was 30k of the 108k warp instructions of an attempt
-// (m = 54, 128 threads): rank-4 updates spent eleven instructions on four FMAs,
-// and the exchanges another pass. A tile takes 16 instructions for 512 FMAs.
+// (m = 54, 128 threads): rank-4 updates spend most of theirs on addresses and
+// loads, and the exchanges were another pass.
 // A form with the whole matrix in registers and one barrier per column was
 // slower (rank-1 updates: 62k instructions).
 template <int G, int RP, bool EXACT, class W>
@@ -1299,7 +1303,7 @@ __device__ __forceinline__ void lu_decompose_mma(const Grp<G>& g, const W& w, in
         const int k1 = min(k0 + kPanel, m);
         {
             GF_PH_BEGIN(g)
-            // the last panels have one row per lane: 70 instead of 110 instructions a step
+            // the last panels have one row per lane: fewer instructions a step
             if (wid == 0) {
                 if (RP == 1 || m - k0 <= 32)
                     lu_panel_reg<1, EXACT>(w, A, ld, piv, sc, rd, perm, m, k0, k1 - k0);

@@ -25,7 +25,11 @@ namespace gf {
 namespace {
 
 constexpr int kFieldCellsMax = 4;  // cells (warps) per CTA of the warp-per-cell form
-constexpr int kLaneCells = 8192;   // cells from which the lane-per-cell form is the faster one
+// Cells from which the lane-per-cell form is taken: from there its 256 CTAs of 32 cells
+// keep the SMs busy. 8,191 cells with a warp each / 8,192 with a lane each: 10 species
+// 33 / 32 us, 53 159 / 156, 75 273 / 218, 100 656 / 417, 126 883 / 787; 20 and 31 species
+// 38 / 45 and 55 / 77, and level with the warps near 12,000.
+constexpr int kLaneCells = 8192;
 
 struct FieldLayout {
     WsLayout L;  // only c, Mtb, stage and part are used

@@ -131,7 +131,7 @@ struct DevMech {
     const int* r_of_q;         // [nR] mechanism index of the reaction in compute position q
     const RxnHead* rxh;        // [nR]
     const RxnFast* rxf;        // [nR]
-    const double* lnk;         // [2][7][nR]: the coefficients of ln K (b = 0 low, 1 high), see reaction_lnK
+    const double* lnk;         // [2][7][nR]: the coefficients of ln K (b = 0 low, 1 high), see load_lnK
     double Tc_all;             // Tcommon of every reaction, or NaN where they differ
     const RxnSpecie* rxs;      // [nR][2 * kSideInline]: lhs, then rhs (wider sides: sidx/siexp/sexp)
     const int* sidx;

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(32) rates_kernel(const DevMech M, const double
 }
 
 // One state per CTA of G threads (a warp for small systems; four warps share the
-// reactions, gathers and rows of a larger one: with one warp and 47 KB per state
+// reactions, gathers and rows of a larger one: with one warp and 45 KB per state
 // an SM had four warps in flight: 350 us for 4,096 states of 53 species, 207 now).
 // MS: the range of matrix sizes that it is compiled for (fix_size): 4,096 states of
 // 40 species 199 -> 172 us against code for any size, of 53 231 -> 225, of 31

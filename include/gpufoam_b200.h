@@ -197,13 +197,14 @@ int gf_solver_create(const gf_mech* const* mechs, int n_mechs, const gf_ode_inpu
                      double Treact, gf_solver** out);
 void gf_solver_destroy(gf_solver* solver);
 /* GF_ERR_UNSUPPORTED for a form the library does not compile: lu_panel 4/16 or
- * specialize need 32, 64 or 128 threads per cell with register_budget 1 for
- * 128 threads and 0 otherwise; without specialize, lu_panel 4/16 needs
+ * specialize need 32, 64, 96 or 128 threads per cell with register_budget 1 for
+ * 96 and 128 threads and 0 otherwise; without specialize, lu_panel 4/16 needs
  * scratch_in_shared; specialize needs a solver whose mechanisms share 10, 53 or
  * 100 species, with lu_panel 8 (or 0), or 4 for 53 species. */
-/* Without a call to it: persistent, by the largest matrix of the solver's
- * mechanisms 32, 128 or 256 threads per cell (to 32, 64 and 128 unknowns; 64
- * beyond, or with the workspace in HBM), specialised where compiled. */
+/* Without a call to it: persistent, by the number of the largest mechanism's
+ * workspaces that an SM's shared memory holds: one, 256 threads per cell; two or
+ * three, 128; more, 64, or 32 for eight and up to 32 unknowns; 64 with the workspace
+ * in HBM. Specialised where compiled (53 species: 128 threads from three on). */
 int gf_solver_set_launch(gf_solver* solver, const gf_launch_config* cfg);
 int gf_solver_get_launch(const gf_solver* solver, gf_launch_config* cfg);
 /* The per-cell workspace of the solve kernels (doubles: in shared memory or
@@ -392,7 +393,7 @@ int gf_lu_backsubstitute(int n_mats, int m, const double* LU, const int* pivots,
 /* LUDecompose + LUBacksubstitute (ludecompose.H:9-130) as the solve kernels
  * run them, with threads_per_matrix (1, 4, 8, 16, 32, 64, 96, 128 or 256) threads
  * per matrix: after the implicit row scaling, the register-panel factorisation
- * for 32 or more threads and m <= 64, the blocked one otherwise; solves by
+ * for 32 or more threads and m <= 128, the blocked one otherwise; solves by
  * reciprocal pivots for 16 or more threads. exact != 0 rounds every
  * elimination update a - l u twice (no FMA contraction), as the reference's
  * CPU build computes its Crout sums, so the factors can be compared bit for
