@@ -758,11 +758,12 @@ __global__ void __launch_bounds__(64) adjoint_kernel(const DevMech Mp, const Adj
     }
 }
 
-// The recording solve (gf_solve_record): the persistent form with one cell
-// per CTA of 128 threads, workspace in shared memory, at most 128 registers, and
-// each accepted step recorded for the sweep.
+// The recording solve (gf_solve_record): the persistent form with one cell per CTA
+// of 128 threads (64, a warp: record_fn), workspace in shared memory, registers for
+// four CTAs per SM (five, twelve), and each accepted step recorded for the sweep.
 template <int MS, int G = 128>
-__global__ void __launch_bounds__(G, 512 / G) record_kernel(const DevMech M, const LaunchArgs a) {
+__global__ void __launch_bounds__(G, G == 128 ? 4 : (G == 64 ? 5 : 12))
+    record_kernel(const DevMech M, const LaunchArgs a) {
     extern __shared__ double smem[];
     Grp<G> g;
     for (;;) {
@@ -800,7 +801,24 @@ static int adj_class(const DevMech& M, int (*bytes)(const DevMech&, int)) {
     const int pad = size_range(M.m) <= 64 ? size_range(M.m) : 0;
     return bytes(M, pad) <= 226 * 1024 ? -pad : 0;
 }
-static RecordFn record_fn(int ms) {
+// The recording kernel and its threads per cell, as the solve's default form has them
+// (default_launch): a warp for small systems, 64 threads to 64 unknowns, and 128
+// where an SM's shared memory holds fewer than eight and four cells. Recording of
+// 2,048 cells of 20, 31, 40 and 60 species, 128 threads and any size 11.0, 13.7, 18.4
+// and 49.5 -> 4.8, 6.7, 10.1 and 33.3 ms; of 10 species, compiled for them, 2.64 -> 1.95.
+static RecordFn record_fn(int ms, int smem, int* threads) {
+    const int cells = 228 * 1024 / (smem + kGroupStaticBytes + 1024);
+    if (ms == -32 && cells >= 8) {
+        *threads = 32;
+        return record_kernel<-32, 32>;
+    }
+    if (ms == -64 && cells >= 4) {
+        *threads = 64;
+        return record_kernel<-64, 64>;
+    }
+    // beside the largest workspaces the reductions of 64 threads fit, not those of 128
+    *threads = smem + kGroupStaticBytes > 227 * 1024 ? 64 : 128;
+    if (*threads == 64) return record_kernel<0, 64>;
     return ms == -32 ? record_kernel<-32> : (ms == -64 ? record_kernel<-64> : record_kernel<0>);
 }
 static AdjointFn adjoint_fn(int ms) {
@@ -812,9 +830,8 @@ int launch_record(const DevMech& M, const LaunchArgs& a, void* stream) {
     const int ms = adj_class(M, record_smem_bytes);
     const int smem = record_smem_bytes(M, -ms);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
-    // beside the largest workspaces the reductions of 64 threads fit, not those of 128
-    const int G = smem + kGroupStaticBytes > 227 * 1024 ? 64 : 128;
-    const RecordFn fn = G == 64 ? record_kernel<0, 64> : record_fn(ms);
+    int G = 0;
+    const RecordFn fn = record_fn(ms, smem, &G);
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (e != cudaSuccess) return (int)e;
     int per_sm = 0;

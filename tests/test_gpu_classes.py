@@ -124,6 +124,24 @@ def test_gradient_sizes(torch, n_species, solver):
     assert abs(ad - tl) <= 1e-5 * abs(tl), ("parameters", ad, tl)
 
 
+@pytest.mark.parametrize("n_species, n_reactions", [(15, 18), (25, 1300), (40, 98), (40, 1300)])
+def test_recorded_forms(torch, n_species, n_reactions):
+    """The recorded solve with a warp, 64 threads and, for long lists of reactions, 128 threads per cell."""
+    raw = mechanism(n_species)
+    raw.reactions = [raw.reactions[k % raw.n_reactions] for k in range(n_reactions)]
+    adj = AD.AdjointSolver(raw, E.OdeInputs("Rosenbrock34", absTol=1e-8, relTol=1e-4), traj_cap=256)
+    few, n = 12, 2400   # more cells than are resident
+    cells = M.make_cells(raw, few, seed=61)
+    ref = Oracle(raw, "port").cells(ode_inputs(34), cells, 1e-7, 1e-8)
+    at = np.arange(n) % few
+    Y1, status, _ = adj.forward(torch.as_tensor(cells[at], device="cuda"), 1e-7,
+                                torch.full((n,), 1e-8, dtype=torch.float64, device="cuda"))
+    assert np.array_equal(status.cpu().numpy(), ref[3][at])
+    ok = status.cpu().numpy() == 0
+    assert ok.any()
+    assert_states_close(Y1.cpu().numpy()[ok], ref[0][at][ok], n_species, 1e-4)
+
+
 @pytest.mark.parametrize("n_species, n_reactions, threads, shared", [
     (31, 75, 32, 1), (31, 500, 64, 1), (25, 1300, 128, 1), (40, 98, 64, 1), (64, 156, 64, 1), (80, 194, 128, 1),
     (100, 245, 128, 1), (127, 310, 256, 1), (135, 329, 256, 1), (160, 390, 64, 0)])
