@@ -536,7 +536,18 @@ __device__ void adj_jacobian_term(const Grp<G>& g, const DevMech& M, const W& w,
         CpMb += -Jb * w[L.J + nS * ld + i] / CpM;
         wa[A.vb + i] += -ab * dTdt;  // Cp_i
         dTdtb += -ab * w[L.Cp + i];
-        for (int j = 0; j < nS; ++j) wa[A.Jb + j * ld + i] += -ab * w[L.Ha + j];
+        // a column in memory, eight entries in flight: entry by entry, with a stride that
+        // the compiler does not know, each load would wait for the store before it
+        constexpr int U = 8;
+        int j = 0;
+        for (; j + U <= nS; j += U) {
+            double v[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) v[k] = wa[A.Jb + (j + k) * ld + i];
+#pragma unroll
+            for (int k = 0; k < U; ++k) wa[A.Jb + (j + k) * ld + i] = v[k] + -ab * w[L.Ha + j + k];
+        }
+        for (; j < nS; ++j) wa[A.Jb + j * ld + i] += -ab * w[L.Ha + j];
     }
     CpMb = g.sum(CpMb);
     dTdtb = g.sum(dTdtb);
@@ -690,11 +701,19 @@ __device__ void adj_step(const Grp<G>& g, const DevMech& M, const W& w, const Ws
         }
     }
     // Jbar = sum_i rbar_i k_i^T  (W = I/(gamma h) - J, k_i = W^-1 r_i)
-    for (int e = g.lane; e < m * m; e += G) {
-        const int a = e / m, b = e % m;
-        double acc = 0.0;
-        for (int st = 0; st < C.s; ++st) acc += wa[A.rb + st * m + a] * w[L.k1 + st * L.ks + b];
-        wa[A.Jb + a * ld + b] = acc;
+    // a thread per column, its k_i in registers (a division per entry otherwise)
+    for (int b = g.lane; b < m; b += G) {
+        double k[4];
+#pragma unroll
+        for (int st = 0; st < 4; ++st) k[st] = st < C.s ? w[L.k1 + st * L.ks + b] : 0.0;
+#pragma unroll 4
+        for (int a = 0; a < m; ++a) {
+            double acc = 0.0;
+#pragma unroll
+            for (int st = 0; st < 4; ++st)
+                if (st < C.s) acc += wa[A.rb + st * m + a] * k[st];
+            wa[A.Jb + a * ld + b] = acc;
+        }
     }
     g.sync();
     {
