@@ -86,12 +86,12 @@ def metric_name(workload, solver):
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of the
 # persistent kernel on the GRI-size mechanism, from one ncu capture of 4 096
-# cells in the launch form below (profiles/persistent_kernel_g128_gri4k.md):
-# 2 801 664 B read, 222 208 B written. Scaled by the cell count for the same
+# cells in the launch form below, which the autotuner picks on those batches
+# (profiles/persistent_kernel_g128_gri4k.md): 3 348 736 B read, 279 552 B written. Scaled by the cell count for the same
 # kernel on the larger GRI-size batches (the per-cell inputs and outputs are
 # moved once, the tables stay in L2).
-NCU_DRAM_BYTES_PER_CELL_GRI = (2801664 + 222208) / 4096
-NCU_PROFILED_FORM = dict(threads_per_cell=128, register_budget=1, lu_panel=4, specialize=1)
+NCU_DRAM_BYTES_PER_CELL_GRI = (3348736 + 279552) / 4096
+NCU_PROFILED_FORM = dict(threads_per_cell=96, register_budget=1, lu_panel=0, specialize=1)
 
 
 def parse():
